@@ -21,6 +21,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <dlfcn.h>
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -44,6 +45,7 @@ enum : int {
     kCntNodes = 3,                 // + level
     kCntUnique = 3 + kMaxDepth,    // + level
     kCntSlots = 3 + 2 * kMaxDepth + 1,
+    kCntDirectBlocks = 62,         // occupied blocks of the direct-mapped brick table
     kCntOverflow = 63,             // fragments the grouping spilled past their partition's slab
 };
 
@@ -61,7 +63,7 @@ struct CallHeader {
     uint32_t leaf_sorted;               // 1: the distinct leaf masks were sorted by one CTA in shared memory
     uint32_t pad1;
 };
-static_assert(kCntSlots <= kCntOverflow, "count slots");
+static_assert(kCntSlots <= kCntDirectBlocks, "count slots");
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -91,6 +93,7 @@ inline cudaError_t dev_malloc(void** p, size_t bytes, AllocStats* st) {
 class DevicePool {
 public:
     AllocStats* stats = nullptr;
+    std::function<void()> on_oom;  // gives back what the context can do without, before the retry
     ~DevicePool() {
         trim();
         for (cudaEvent_t e : spare_events_) cudaEventDestroy(e);
@@ -112,6 +115,7 @@ public:
         if (e == cudaErrorMemoryAllocation) {
             cudaGetLastError();
             trim();
+            if (on_oom) on_oom();
             e = dev_malloc(p, bytes, stats);
             if (e == cudaSuccess && stats) ++stats->retries_ok;
         }
@@ -215,6 +219,7 @@ struct Arena {
     void* base = nullptr;
     size_t cap = 0;
     AllocStats* stats = nullptr;
+    std::function<void()> on_oom;  // as DevicePool::on_oom
     // Grows to at least `bytes` (with 25% headroom; without it when that
     // does not fit).
     cudaError_t reserve(size_t bytes) {
@@ -226,6 +231,7 @@ struct Arena {
         cudaError_t e = dev_malloc(&base, want, stats);
         if (e != cudaSuccess) {
             cudaGetLastError();
+            if (on_oom) on_oom();
             e = dev_malloc(&base, align_up(bytes, 1u << 21), stats);
             if (e != cudaSuccess) { cudaGetLastError(); base = nullptr; return e; }
             if (stats) ++stats->retries_ok;
@@ -298,10 +304,11 @@ struct GraphKey {
     bool dedup;        // hash-set dedup (else radix sort + unique) for the leaves and levels
     void* table;       // the dedup table block
     int group;         // fragment grouping mode
+    void* direct;      // the direct-mapped brick table (null: not used)
     bool operator==(const GraphKey& o) const {
         return frag == o.frag && n == o.n && depth == o.depth && arena == o.arena && chunks == o.chunks &&
                chunk_depth == o.chunk_depth && chunk_path == o.chunk_path && dedup == o.dedup && table == o.table &&
-               group == o.group;
+               group == o.group && direct == o.direct;
     }
 };
 struct GraphEntry {
@@ -354,6 +361,11 @@ struct dagc_context_t {
     void* gtable = nullptr;  // fragment grouping scratch
     uint64_t table_cap = 0;  // slots (table_size_for of the largest item count so far)
     bool table_dirty = true;
+    // Direct-mapped brick table (direct.cu): direct_cap leaf masks, all zero
+    // between calls; cleared before the next use after a call that failed.
+    void* direct = nullptr;
+    uint64_t direct_cap = 0;
+    bool direct_dirty = true;
     uint64_t fallbacks = 0;  // calls rerun with the radix form
     uint32_t* trace_err = nullptr;  // tracer error word
     void* vox_scratch = nullptr;    // voxelizer counters and look-back status
@@ -806,11 +818,13 @@ struct CreateLayout {
     // Persistent per-chunk leaves (batched form): zeroed chunk state
     // (histograms, cursors, done counters, item counter), tile offsets, the
     // mask stage and per-item brick counts / offsets.
+    // Direct-mapped leaves: block counters (zeroed) and the occupied blocks.
+    size_t o_dcount = 0, o_dsv = 0, o_dlist = 0;
     uint32_t ck_bins = 0, ck_groups = 0;
     size_t o_ck_state = 0, ck_state_bytes = 0, o_ck_hist = 0, o_ck_cursor = 0, o_ck_done = 0, o_ck_work = 0;
     size_t o_ck_tile = 0, o_ck_mask = 0, o_ck_gb = 0, o_ck_gs = 0, o_ck_gd = 0;
     CreateLayout(uint64_t n, int depth, uint32_t k_batch, bool use_dedup, uint64_t unique_limit = kDedupMaxUnique,
-                 bool grouping = false, int chunk_depth = 0) {
+                 bool grouping = false, int chunk_depth = 0, bool direct_table = false, bool direct = false) {
         const int nl = depth - 2;
         cap.resize(nl);
         for (int l = 0; l < nl; ++l) { cap[l] = level_cap(l, n); capmax = std::max(capmax, cap[l]); }
@@ -820,11 +834,16 @@ struct CreateLayout {
         Layout L;
         o_hdr = L.take<CallHeader>(1);
         o_sv = L.take<uint64_t>(sv_total);
+        if (direct_table) {
+            o_dcount = L.take<uint32_t>(direct_blocks(depth));
+            o_dsv = L.take<uint64_t>(direct_plan_tiles(depth));
+        }
         zero_bytes = L.off;
+        if (direct_table) o_dlist = L.take<uint2>(direct_blocks(depth));
         o_ss0 = L.take<uint32_t>(sort_status_words(n));
         o_ss1 = L.take<uint32_t>(sort_status_words(n));
-        o_A = L.take<uint64_t>(n);
-        o_B = L.take<uint64_t>(n);
+        o_A = L.take<uint64_t>(direct ? 0 : n);
+        o_B = L.take<uint64_t>(direct ? 0 : n);
         if (grouping) {
             group_shape(n, &group_slab_total, &group_probe_max);
             o_slab = L.take<uint64_t>(group_slab_total);
@@ -889,6 +908,15 @@ struct CreateLayout {
     }
 };
 
+// Gives the brick table back (it is idle between a call's pipelines); a later
+// call allocates it again if there is room.
+void release_direct(dagc_context ctx) {
+    if (ctx->direct) cudaFree(ctx->direct);
+    ctx->direct = nullptr;
+    ctx->direct_cap = 0;
+    ctx->direct_dirty = true;
+}
+
 // Grows the context's dedup table to `slots` (zeroed); clears it after a call
 // that may have stopped between an insert and its map.
 int reserve_table(dagc_context ctx, uint64_t slots, cudaStream_t s) {
@@ -896,7 +924,14 @@ int reserve_table(dagc_context ctx, uint64_t slots, cudaStream_t s) {
         if (ctx->table) cudaFree(ctx->table);
         ctx->table = nullptr;
         ctx->table_cap = 0;
-        DAGC_CUDA(ctx, cudaMalloc(&ctx->table, slots * 16));  // per slot: key u64, aux u64
+        cudaError_t e = cudaMalloc(&ctx->table, slots * 16);  // per slot: key u64, aux u64
+        if (e == cudaErrorMemoryAllocation && ctx->direct) {
+            cudaGetLastError();
+            release_direct(ctx);
+            e = cudaMalloc(&ctx->table, slots * 16);
+        }
+        if (e != cudaSuccess) ctx->table = nullptr;
+        DAGC_CUDA(ctx, e);
         ctx->table_cap = slots;
         ctx->table_dirty = true;
     }
@@ -908,6 +943,46 @@ int reserve_table(dagc_context ctx, uint64_t slots, cudaStream_t s) {
     return DAGC_OK;
 }
 
+// Whether an unbatched call uses the direct-mapped brick table (direct.cu). It
+// has 8 bytes per brick of the volume whatever the fragments, so the line is
+// its size: up to depth 10 (134 MB, about the L2) always, at depth 11 (1 GB)
+// from 2^21 fragments on, where the call's own scratch (about 400 bytes per
+// fragment) is of that order.
+bool direct_table_applies(uint64_t n, int depth) {
+    return depth < kDirectMaxDepth || (depth == kDirectMaxDepth && n >= (1u << 21));
+}
+// Whether the fragments go straight into that table, or are grouped or sorted
+// first (at depth 11 the table then orders the grouped bricks). A fragment
+// costs one random access of the table, at 60-100 G/s while the L2 serves it
+// (leaf stages, us, before / with the table: triangle soup of 0.65M fragments,
+// depth 10, 115 / 32; 61M, 1500 / 1140; terrain of 7.9M, depth 10, 200 / 93;
+// sphere shell in 32^3, 52 / 16) but at 20-50 G/s over the 1 GB of depth 11
+// (terrain, 31M: 400 grouped, 617 straight in). Crowded bricks go through the
+// grouping's shared-memory tables faster: depth 9, 61M fragments, 29 per
+// brick, 700 grouped, 792 straight in.
+bool direct_mark_applies(uint64_t n, int depth) {
+    return depth < kDirectMaxDepth && (n <= (1u << 25) || n <= 4 * direct_entries(depth));
+}
+
+// Grows the context's brick table to `entries`, zeroed; clears it after
+// a failed call. False (and no error) when the device has no room for it: the
+// call then takes the other paths.
+bool reserve_direct(dagc_context ctx, uint64_t entries, cudaStream_t s) {
+    if (entries > ctx->direct_cap) {
+        void* p = nullptr;
+        release_direct(ctx);
+        if (cudaMalloc(&p, entries * 8) != cudaSuccess) { cudaGetLastError(); return false; }
+        ctx->direct = p;
+        ctx->direct_cap = entries;
+        ctx->direct_dirty = true;
+    }
+    if (ctx->direct_dirty) {
+        if (cudaMemsetAsync(ctx->direct, 0, ctx->direct_cap * 8, s) != cudaSuccess) { cudaGetLastError(); return false; }
+        ctx->direct_dirty = false;
+    }
+    return true;
+}
+
 int load_tune_file(dagc_context ctx, const char* path);
 
 // Internal status: the hash-set dedup could not hold this input; the caller
@@ -915,7 +990,7 @@ int load_tune_file(dagc_context ctx, const char* path);
 constexpr int kStatusFallback = -1000;
 
 int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int depth, cudaStream_t s,
-                    CreatePools& out, const BatchSpec* batch, bool use_dedup) {
+                    CreatePools& out, const BatchSpec* batch, bool use_dedup, bool allow_direct = true) {
     t_pdl = ctx->pdl;
     const int group_mode = ctx->group_mode;
     const int nl = depth - 2;
@@ -923,8 +998,11 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
     // Batched calls take the persistent per-chunk leaf build (chunks.cu) when
     // the chunk's bins fit its limits; otherwise the composite-key path.
     const bool chunk_path = batch && ctx->batch_path == 1 && chunk_bin_bits(batch->chunk_depth) <= kChunkMaxBinBits;
+    const bool direct_table = allow_direct && !batch && use_dedup && group_mode == 1 && direct_table_applies(n, depth);
+    const bool direct = direct_table && direct_mark_applies(n, depth);
     const CreateLayout Lo(n, depth, batch ? batch->k : 0u, use_dedup, ctx->dedup_unique_limit,
-                          group_mode != 0 && use_dedup && !chunk_path, chunk_path ? batch->chunk_depth : 0);
+                          group_mode != 0 && use_dedup && !chunk_path && !direct, chunk_path ? batch->chunk_depth : 0,
+                          direct_table, direct);
     const std::vector<uint64_t>& cap = Lo.cap;
     const uint64_t capmax = Lo.capmax, p0cap = Lo.p0cap, sv_total = Lo.sv_total;
     const size_t zero_bytes = Lo.zero_bytes;
@@ -935,6 +1013,8 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
         const int st = reserve_table(ctx, Lo.table_slots, s);
         if (st) return st;
     }
+    if (direct_table && !reserve_direct(ctx, direct_entries(depth), s))
+        return create_pipeline(ctx, d_frag, n, depth, s, out, batch, use_dedup, false);
     char* b = static_cast<char*>(ctx->arena.base);
     auto P64 = [&](size_t o) { return reinterpret_cast<uint64_t*>(b + o); };
     auto P32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(b + o); };
@@ -1018,7 +1098,35 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
             DAGC_LAUNCHED(ctx);
             t.stop();
         }
-        if (!chunk_path && group_mode != 0 && use_dedup && ctx->gtable) {
+        DirectArgs da{};
+        if (direct_table) {
+            DirectArgs& a = da;
+            a.frags = d_frag;
+            a.n = n;
+            a.code_bits = bits;
+            a.table = static_cast<uint64_t*>(ctx->direct);
+            a.blocks = (uint32_t)direct_blocks(depth);
+            a.block_count = P32(Lo.o_dcount);
+            a.list = reinterpret_cast<uint2*>(b + Lo.o_dlist);
+            a.d_blocks = cs.count(kCntDirectBlocks);
+            a.status = P64(Lo.o_dsv);
+            a.tile_counter = cs.counter();
+            a.parents = P64(Lo.o_P);
+            a.leaves = P64(Lo.o_LM);
+            a.out_capacity = p0cap;
+            a.d_out_n = cs.count(kCntBricks);
+            a.err = err;
+        }
+        if (direct) {
+            // 1. Every fragment's bit into the brick table, and the table's
+            //    nonzero entries out in order.
+            StageTimer t(ctx, DAGC_STAGE_LEAF_BUILD, s);
+            ctx->launches += launch_direct_mark(da, s);
+            ctx->launches += launch_direct_compact(da, s);
+            DAGC_LAUNCHED(ctx);
+            t.stop();
+        }
+        if (!chunk_path && !direct && group_mode != 0 && use_dedup && ctx->gtable) {
             GroupArgs g{};
             g.frags = d_frag;
             g.n = n;
@@ -1049,6 +1157,11 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
             g.parents = P64(Lo.o_P);
             g.leaves = P64(Lo.o_LM);
             g.err = err;
+            if (direct_table) {
+                g.table = da.table;
+                g.block_count = da.block_count;
+                da.gate = cs.h->path;
+            }
             {
                 StageTimer t1(ctx, DAGC_STAGE_GROUP_SKETCH, s);
                 launch_group_probe(g, s);
@@ -1066,13 +1179,18 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
             }
             DAGC_LAUNCHED(ctx);
             StageTimer tg(ctx, DAGC_STAGE_GROUP, s);
-            // The bricks (B of them instead of N fragments), sorted with their indices.
-            st = run_sort(ctx, cs, sb, P64(Lo.o_A), P64(Lo.o_P), P64(Lo.o_B), P32(Lo.o_M0), P32(Lo.o_M1),
-                          P32(Lo.o_LM), true, g.cap, cs.count(kCntBricks), 0, sort_hi - 6, 0, s, -1, -1, nullptr,
-                          cs.h->path, 1u);
-            if (st) return st;
-            launch_group_gather(g, s);
-            ++ctx->launches;
+            if (direct_table) {
+                // The bricks in order through the direct-mapped table.
+                ctx->launches += launch_direct_compact(da, s);
+            } else {
+                // The bricks (B of them instead of N fragments), sorted with their indices.
+                st = run_sort(ctx, cs, sb, P64(Lo.o_A), P64(Lo.o_P), P64(Lo.o_B), P32(Lo.o_M0), P32(Lo.o_M1),
+                              P32(Lo.o_LM), true, g.cap, cs.count(kCntBricks), 0, sort_hi - 6, 0, s, -1, -1, nullptr,
+                              cs.h->path, 1u);
+                if (st) return st;
+                launch_group_gather(g, s);
+                ++ctx->launches;
+            }
             DAGC_LAUNCHED(ctx);
             tg.stop();
             gate = cs.h->path;
@@ -1081,13 +1199,13 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
         // 1b. Fragment sort on the brick key bits [6, 3*depth): only the order of
         //     code >> 6 matters downstream (the leaf mask ORs the low 6 bits).
         const SegmentSpec seg{batch ? P64(Lo.o_seg_off) : nullptr, batch ? batch->k : 0u, seg_shift};
-        if (!chunk_path)
+        if (!chunk_path && !direct)
             st = run_sort(ctx, cs, sb, d_frag, P64(Lo.o_A), P64(Lo.o_B), nullptr, nullptr, nullptr, false, n, nullptr, 6,
                           sort_hi, validate, s, DAGC_STAGE_FRAGMENT_HIST, DAGC_STAGE_FRAGMENT_PASS, &seg, gate, 0u);
         if (st) return st;
 
         // 2. Fused unique + leaf build.
-        if (!chunk_path) {
+        if (!chunk_path && !direct) {
             StageTimer t(ctx, DAGC_STAGE_LEAF_BUILD, s);
             LeafBuildArgs a{};
             a.sorted = P64(Lo.o_A);
@@ -1306,9 +1424,10 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
     };
     int st = run_enqueue(ctx, GraphKey{d_frag, n, depth, ctx->arena.base, batch ? batch->k : 0u,
                                        batch ? batch->chunk_depth : 0, chunk_path, use_dedup,
-                                       use_dedup ? ctx->table : nullptr, use_dedup ? group_mode : 0},
+                                       use_dedup ? ctx->table : nullptr, use_dedup ? group_mode : 0,
+                                       direct_table ? ctx->direct : nullptr},
                          s, enqueue);
-    if (st) { ctx->table_dirty = true; return st; }
+    if (st) { ctx->table_dirty = true; ctx->direct_dirty = true; return st; }
     CallHeader* hdr = reinterpret_cast<CallHeader*>(b + Lo.o_hdr);
     // 5. One read-back of every count and the error word.
     static_assert(sizeof(CallHeader) >= 8 * 65, "header");
@@ -1328,12 +1447,13 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
         // Grouping: the probe reads a sixteenth of the fragments; the scatter
         // reads 8 bytes per fragment and writes its slab entry (4 bytes in the
         // narrow form, else 8), which the aggregation reads; the brick sort
-        // and the gather move ~60 bytes per brick.
+        // and the gather move ~60 bytes per brick, the brick table's
+        // compaction 32 and its block counters.
         const uint64_t entry = sort_hi <= 37 ? 4 : 8;
         set_pending_bytes(ctx, DAGC_STAGE_GROUP_SKETCH, n / 2);
         set_pending_bytes(ctx, DAGC_STAGE_GROUP_SCATTER, (8 + entry) * n);
         set_pending_bytes(ctx, DAGC_STAGE_GROUP_AGGREGATE, entry * n + 20 * p0);
-        set_pending_bytes(ctx, DAGC_STAGE_GROUP, 60 * p0);
+        set_pending_bytes(ctx, DAGC_STAGE_GROUP, direct_table ? 32 * p0 + 4 * direct_blocks(depth) : 60 * p0);
         // Chunk leaves: COUNT reads the fragments, SCATTER reads and writes
         // them, LEAVES reads them and writes 16 bytes per brick, the pack
         // moves those bricks once more.
@@ -1346,7 +1466,7 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
         }
         set_pending_bytes(ctx, DAGC_STAGE_LEVELS, lb);
         // The kernels of the path the device did not take returned at once.
-        if (group_mode != 0 && use_dedup && ctx->gtable) {
+        if (!direct && group_mode != 0 && use_dedup && ctx->gtable) {
             uint32_t path = 0;
             DAGC_CUDA(ctx, cudaMemcpy(&path, &hdr->path[0], 4, cudaMemcpyDeviceToHost));
             if (path == 1) {
@@ -1361,7 +1481,7 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
         }
         settle_profile(ctx);
     }
-    if (e32) ctx->table_dirty = true;  // a level may have stopped before clearing its slots
+    if (e32) ctx->table_dirty = ctx->direct_dirty = true;  // a kernel may have stopped before clearing its slots
     if ((e32 & kErrFallback) && !(e32 & (kErrBadInput | kErrTimeout))) return kStatusFallback;
     std::string msg;
     st = device_error_status(e32, msg);
@@ -1984,6 +2104,7 @@ int dagc_context_create(int device, dagc_context* out) {
     c->device = device;
     c->pool.stats = &c->alloc_stats;
     c->arena.stats = &c->alloc_stats;
+    c->pool.on_oom = c->arena.on_oom = [p = c.get()] { release_direct(p); };
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
     sort_configure();
     kernels_configure();
@@ -2041,6 +2162,7 @@ int dagc_context_create(int device, dagc_context* out) {
     c->grid_write = std::max(1, occupancy_kernel(kKernelFinalWrite)) * c->sms;
     dedup_configure(c->sms);
     group_configure(c->sms);
+    direct_configure(c->sms);
     chunk_configure(c->sms);
     *out = c.release();
     return DAGC_OK;
@@ -2059,6 +2181,7 @@ void dagc_context_destroy(dagc_context ctx) {
     ctx->arena.release();
     if (ctx->table) cudaFree(ctx->table);
     if (ctx->gtable) cudaFree(ctx->gtable);
+    release_direct(ctx);
     if (ctx->trace_err) cudaFree(ctx->trace_err);
     if (ctx->vox_scratch) cudaFree(ctx->vox_scratch);
     ctx->pool.trim();
@@ -2136,7 +2259,7 @@ int dagc_create_batched(dagc_context ctx, const uint64_t* d_fragments, const uin
 uint64_t dagc_create_footprint(uint64_t n, int depth) {
     if (depth < 2 || depth > kMaxDepth || n == 0) return 0;
     const CreateLayout L(n, depth, 0, true, kDedupMaxUnique, true);
-    return L.total + L.table_slots * 16 + kGroupScratchBytes;
+    return L.total + L.table_slots * 16 + kGroupScratchBytes + (direct_table_applies(n, depth) ? direct_entries(depth) * 8 : 0);
 }
 
 int dagc_dag_num_levels(dagc_dag d, int* num_levels) {
@@ -2370,6 +2493,7 @@ int dagc_free_all(dagc_context ctx) {
     if (ctx->table) cudaFree(ctx->table);
     if (ctx->gtable) cudaFree(ctx->gtable);
     ctx->table = nullptr;
+    release_direct(ctx);
     ctx->gtable = nullptr;
     ctx->table_cap = 0;
     ctx->table_dirty = true;
@@ -2548,6 +2672,7 @@ int dagc_memory_report(dagc_context ctx, char* buf, uint64_t capacity, uint64_t*
         if (ctx->arena.cap) m["scratch arena"] = {ctx->arena.cap, 1};
         if (ctx->table_cap) m["dedup table"] = {ctx->table_cap * 16, 1};
         if (ctx->gtable) m["grouping table"] = {kGroupScratchBytes, 1};
+        if (ctx->direct) m["brick table"] = {ctx->direct_cap * 8, 1};
         uint64_t total = 0;
         for (const auto& kv : m) total += kv.second.first;
         std::vector<std::pair<std::string, std::pair<uint64_t, uint64_t>>> list(m.begin(), m.end());

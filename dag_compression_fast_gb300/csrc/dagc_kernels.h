@@ -187,6 +187,9 @@ struct GroupArgs {
     uint64_t* overflow_count;  // zero on entry
     uint32_t* part_over;       // kGroupMaxParts flags, zero on entry: the partition spilled
     uint64_t* bricks; uint32_t* idx; uint64_t* masks; uint64_t cap;  // brick list (unsorted), masks[idx]
+    // Or, when non-null (unbatched input): the direct-mapped table of all
+    // bricks and its block counters (DirectArgs), which puts them in order.
+    uint64_t* table; uint32_t* block_count;
     uint64_t* d_count;         // bricks found
     const uint64_t* sorted_bricks; const uint32_t* sorted_idx;      // after the brick sort
     uint64_t* parents; uint64_t* leaves;
@@ -202,6 +205,34 @@ void launch_group_plan(const GroupArgs& a, cudaStream_t s);      // picks the pa
 void launch_group_scatter(const GroupArgs& a, cudaStream_t s);
 void launch_group_aggregate(const GroupArgs& a, cudaStream_t s);
 void launch_group_gather(const GroupArgs& a, cudaStream_t s);
+
+// Leaves by a direct-mapped table of the whole brick space (direct.cu).
+constexpr int kDirectBlockLog = 6;            // 64 bricks per block
+constexpr uint32_t kDirectScanBlocks = 4096;  // up to here (depth 8) the compaction sums the block counts itself
+constexpr uint32_t kDirectPlanTile = 4096;    // blocks per tile of the plan
+constexpr int kDirectMaxDepth = 11;           // a table of 8^9 entries: 1 GB
+DAGC_HD uint64_t direct_blocks(int depth) {
+    return ((1ull << (3 * (depth - 2))) + (1ull << kDirectBlockLog) - 1) >> kDirectBlockLog;
+}
+DAGC_HD uint64_t direct_entries(int depth) { return direct_blocks(depth) << kDirectBlockLog; }  // whole blocks
+DAGC_HD uint64_t direct_plan_tiles(int depth) { return direct_blocks(depth) / kDirectPlanTile + 1; }
+struct DirectArgs {
+    const uint64_t* frags; uint64_t n;
+    int code_bits;          // 3 * depth: codes are below 2^code_bits
+    uint64_t* table;        // a leaf mask per brick (direct_entries), zero on entry and exit
+    uint32_t blocks;
+    uint32_t* block_count;  // bricks per block, zero on entry
+    uint2* list; uint64_t* d_blocks;             // occupied blocks: (block, bricks before it), and how many
+    uint64_t* status; uint32_t* tile_counter;    // of the plan: zero on entry
+    uint64_t* parents; uint64_t* leaves; uint64_t out_capacity; uint64_t* d_out_n;
+    uint32_t* err;
+    const uint32_t* gate;   // non-null: the compaction does nothing unless *gate == 1 (grouping, GroupArgs::path)
+};
+void direct_configure(int sms);
+// The fragments into the table; the table's bricks out in order. Both return
+// the number of launches.
+int launch_direct_mark(const DirectArgs& a, cudaStream_t s);
+int launch_direct_compact(const DirectArgs& a, cudaStream_t s);
 
 // Batched form: every chunk's leaves in one persistent launch (chunks.cu).
 // A chunk's local bricks (local code >> 6) fall in 2^bin_bits bins of at most

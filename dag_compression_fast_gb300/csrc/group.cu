@@ -29,7 +29,10 @@
 //                    brick list (brick, index) and the masks;
 //   (then the brick list is sorted by brick with the radix sort, values =
 //    indices: B items instead of N)
-//   group_gather     parents and masks in sorted brick order.
+//   group_gather     parents and masks in sorted brick order;
+//   or, where the context keeps a direct-mapped table of the volume's bricks
+//   (direct.cu), the aggregation stores each brick's mask there and the
+//   table's compaction gives both in order, without the brick sort.
 //
 // The scatter reads the fragments in order and writes one slab entry per
 // fragment (4 bytes in the narrow form: the brick's 32-bit product without
@@ -560,6 +563,20 @@ __global__ void __launch_bounds__(kAggThreads) group_aggregate(GroupArgs a) {
             for (uint32_t j = 0; j < per; ++j) cnt += sm.key[s0 + j] != 0;
             uint32_t total;
             const uint32_t ex = block_exclusive_sum<uint32_t>(cnt, sm.scan, &total);
+            if (a.table) {
+                // Every brick is in one partition's one sub-range: a plain
+                // store into its entry of the direct-mapped table.
+                for (uint32_t j = 0; j < per; ++j) {
+                    const uint64_t t = (uint64_t)sm.key[s0 + j];
+                    if (t == 0) continue;
+                    const uint64_t brick = kNarrow ? compact_brick(p, lp, (uint32_t)t - 1) : t - 1;
+                    if (brick >> (a.validate_bits - 6)) continue;  // out of range: flagged by the scatter
+                    a.table[brick] = sm.mask[s0 + j];
+                    atomicAdd(a.block_count + (brick >> kDirectBlockLog), 1u);
+                }
+                __syncthreads();  // the table is cleared for the next sub-range
+                continue;
+            }
             if (threadIdx.x == 0)
                 sm.base = total ? atomicAdd((unsigned long long*)a.d_count, (unsigned long long)total) : 0ull;
             __syncthreads();

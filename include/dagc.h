@@ -205,7 +205,10 @@ int dagc_last_counts(dagc_context ctx, uint64_t* out, int cap);
  * that larger levels take the rerun. */
 #define DAGC_OPT_DEDUP_UNIQUE_LIMIT 5
 /* How fragments are grouped into bricks (SortKeys + SelectUnique +
- * ReduceByKey): 1 (default) choose on the device per call, from a sketch of
+ * ReduceByKey): 1 (default) up to depth 10 through a direct-mapped table of
+ * the volume's bricks (8 bytes each, kept by the context; not for calls of
+ * more than 2^25 fragments with more than 4 per brick of the volume); beyond,
+ * choose on the device per call, from a sketch of
  * the distinct bricks in a sample of the fragments: hash partitions and
  * per-partition tables when the fragments hold >= 8 per brick (and the
  * tables can hold the bricks), else the radix sort; 0 always the radix sort;
