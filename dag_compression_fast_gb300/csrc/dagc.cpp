@@ -60,8 +60,7 @@ struct CallHeader {
     uint32_t gover[kGroupMaxParts];     // its partitions that spilled past their slabs
     uint64_t gcursor[kGroupMaxParts];   // its partition starts, then ends
     uint32_t path[4];                   // [0] 1: fragments grouped by hash, 0: sorted; [1], [2] its shape
-    uint32_t leaf_sorted;               // 1: the distinct leaf masks were sorted by one CTA in shared memory
-    uint32_t pad1;
+    LeafOrder leaf;                     // ordering of the distinct leaf masks
 };
 static_assert(kCntSlots <= kCntDirectBlocks, "count slots");
 
@@ -813,7 +812,7 @@ struct CreateLayout {
     // Hash-set dedup (when `dedup`): per-item slots, the unique list, buckets.
     bool dedup = false;
     uint64_t item_cap = 0, uniq_cap = 0, bucket_area = 0, table_slots = 0;
-    size_t o_islot = 0, o_ukey = 0, o_ukey_alt = 0;
+    size_t o_islot = 0, o_ukey = 0, o_uslot = 0;
     size_t o_bcnt = 0, o_bent = 0;
     // Persistent per-chunk leaves (batched form): zeroed chunk state
     // (histograms, cursors, done counters, item counter), tile offsets, the
@@ -840,8 +839,9 @@ struct CreateLayout {
         }
         zero_bytes = L.off;
         if (direct_table) o_dlist = L.take<uint2>(direct_blocks(depth));
-        o_ss0 = L.take<uint32_t>(sort_status_words(n));
-        o_ss1 = L.take<uint32_t>(sort_status_words(n));
+        const bool sorts = !direct || !use_dedup;
+        o_ss0 = L.take<uint32_t>(sorts ? sort_status_words(n) : 0);
+        o_ss1 = L.take<uint32_t>(sorts ? sort_status_words(n) : 0);
         o_A = L.take<uint64_t>(direct ? 0 : n);
         o_B = L.take<uint64_t>(direct ? 0 : n);
         if (grouping) {
@@ -862,12 +862,10 @@ struct CreateLayout {
             item_cap = std::min<uint64_t>(p0cap, kDedupMaxItems);
             uniq_cap = std::min<uint64_t>(p0cap, std::min<uint64_t>(unique_limit, kDedupMaxUnique));
             bucket_area = dedup_bucket_area(uniq_cap);
-            table_slots = std::max(table_size_for(item_cap, true), table_size_for(item_cap, false));
+            table_slots = table_slots_upto(item_cap);
             o_islot = L.take<uint32_t>(item_cap);
             o_ukey = L.take<uint64_t>(uniq_cap);
-            // The other key buffer of the unique leaf masks' sort (the sorted
-            // keys go out to the leaf array).
-            o_ukey_alt = L.take<uint64_t>(uniq_cap);
+            o_uslot = L.take<uint32_t>(uniq_cap);
             o_bcnt = L.take<uint32_t>(kDedupMaxBuckets);
             o_bent = L.take<uint4>(bucket_area);
         }
@@ -1248,6 +1246,9 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
             d.table_cap = ctx->table_cap;
             d.item_slot = P32(Lo.o_islot);
             d.uniq_key = P64(Lo.o_ukey);
+            d.uniq_slot = P32(Lo.o_uslot);
+            d.leaf = &cs.h->leaf;
+            d.leaf_keys = leaf_keys_for(Lo.uniq_cap);
             d.uniq_cap = Lo.uniq_cap;
             d.bucket_count = P32(Lo.o_bcnt);
             d.bucket = reinterpret_cast<uint4*>(b + Lo.o_bent);
@@ -1264,22 +1265,12 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
         };
         if (use_dedup) {
             // Distinct masks into the table and the unique list; the list
-            // sorted (keys only) straight into the leaf array; each mask's
-            // slot gets the mask's rank as unique id; every brick its id.
+            // ordered into the leaf array, each mask's rank to its slot as
+            // unique id; every brick its id.
             const DedupArgs d = dedup_args(P64(Lo.o_LM), cs.count(kCntBricks), nullptr, nullptr, P64(Lo.o_PL), nullptr,
                                            nullptr, p0cap, cs.count(kCntLeaves), P32(Lo.o_M0));
             launch_dedup_insert(d, s);
-            ++ctx->launches;
-            DAGC_LAUNCHED(ctx);
-            // Up to kSmallSortMax distinct masks: one CTA sorts them in shared
-            // memory and the grid-wide sort's kernels return at once.
-            const uint64_t* d_u = reinterpret_cast<const uint64_t*>(&d.state->u);
-            launch_small_sort(P64(Lo.o_ukey), P64(Lo.o_PL), d_u, Lo.uniq_cap, &cs.h->leaf_sorted, s);
-            ++ctx->launches;
-            st = run_sort(ctx, cs, sb, P64(Lo.o_ukey), P64(Lo.o_PL), P64(Lo.o_ukey_alt), nullptr, nullptr, nullptr,
-                          false, Lo.uniq_cap, d_u, 0, 64, 0, s, -1, -1, nullptr, &cs.h->leaf_sorted, 0u);
-            if (st) return st;
-            launch_dedup_assign(d, P64(Lo.o_PL), s);
+            ctx->launches += launch_leaf_order(d, s);
             launch_dedup_map(d, s);
             ctx->launches += 2;
             DAGC_LAUNCHED(ctx);

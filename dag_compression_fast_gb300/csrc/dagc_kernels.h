@@ -111,12 +111,6 @@ int sort_shape_items(int shape, bool with_values);
 // Resident CTAs per SM of a shape at a digit width (occupancy query) for grid sizing.
 int occupancy_sort_shape(int shape, bool with_values, int radix_bits = kRadixBits);
 int occupancy_sort_histogram();
-// One-CTA sort of up to kSmallSortMax 64-bit keys (all 64 bits) held in
-// shared memory, keys_in -> keys_out, when the device count *d_n fits; sets
-// *done to 1 then (a grid-wide sort gated on *done == 0 then does nothing).
-constexpr uint32_t kSmallSortMax = 12288;
-void launch_small_sort(const uint64_t* keys_in, uint64_t* keys_out, const uint64_t* d_n, uint64_t n_bound,
-                       uint32_t* done, cudaStream_t s);
 // Whether a (shape, width) plan can sort bits [lo, hi): histogram room and
 // look-back status room.
 bool sort_plan_valid(int shape, bool with_values, int radix_bits, int lo_bit, int hi_bit);
@@ -302,24 +296,48 @@ DAGC_HD uint64_t dedup_bucket_area(uint64_t uniq_cap) {
 }
 // Table slots for n items. Leaf masks repeat (about one distinct mask per ten
 // bricks): 1.25 n slots, at most 0.8 full even when every mask is distinct,
-// small enough to stay largely in the L2. Node hashes are about half distinct
+// small enough to stay largely in the L2. Up to kLeafSparseMax of them the
+// table is in the L2 anyway and the insert's time is its longest probe chain, a
+// round trip per two slots: 4 n slots (25k distinct masks of 36k bricks: the
+// insert takes 12 us, 25 with 1.25 n). Node hashes are about half distinct
 // and each probe step is a dependent round trip: kNodeTableQuarters / 4 * n
 // slots keep the load low. At least 1024 slots, a multiple of 32.
 constexpr uint64_t kNodeTableQuarters = 8;
+constexpr uint64_t kLeafSparseMax = 1ull << 20;
 DAGC_HD uint64_t table_size_for(uint64_t n, bool leaf_masks) {
-    const uint64_t want = leaf_masks ? n + (n >> 2) : n * kNodeTableQuarters / 4;
+    const uint64_t want = !leaf_masks ? n * kNodeTableQuarters / 4 : n <= kLeafSparseMax ? 4 * n : n + (n >> 2);
     return want < 1024 ? 1024 : (want + 31) & ~31ull;
+}
+// Slots that hold any count of up to `items` items of either kind.
+DAGC_HD uint64_t table_slots_upto(uint64_t items) {
+    const uint64_t sparse = table_size_for(items < kLeafSparseMax ? items : kLeafSparseMax, true);
+    const uint64_t leaf = table_size_for(items, true), node = table_size_for(items, false);
+    const uint64_t most = leaf > node ? leaf : node;
+    return most > sparse ? most : sparse;
 }
 struct DedupState {
     unsigned long long u;  // distinct keys found (zero before the level)
     uint32_t nbuckets, pad0;
     uint32_t inserted, pad;  // 1: extract_level already inserted the level's hashes
 };
+// Ordering of the distinct leaf masks: up to kLeafRankMax of them are ranked
+// at once, more go through buckets between samples (half as many buckets up to
+// kLeafMidMax).
+constexpr uint32_t kLeafRankMax = 8192;
+constexpr uint32_t kLeafBuckets = 2048;
+constexpr uint64_t kLeafMidMax = 1ull << 18;
+struct LeafOrder {
+    uint32_t count[kLeafBuckets];  // keys per bucket, zero on entry
+    uint64_t splitter[kLeafBuckets];
+};
+// Most keys of one bucket (10 bytes of shared memory each) when the list may
+// hold uniq_cap: the mean is at most 256 up to kLeafMidMax, then uniq_cap / 2048.
+DAGC_HD uint32_t leaf_keys_for(uint64_t uniq_cap) { return uniq_cap <= kLeafMidMax ? 2048u : 8192u; }
 struct DedupArgs {
     const uint64_t* keys; const uint64_t* d_n;       // items: key per item
     const uint8_t* masks; const uint32_t* children;  // item payloads (null for leaves)
-    // Leaf masks (far from uniform): winners go to the unique list, which the
-    // caller sorts. Node hashes: winners go to the bucket of their top bits.
+    // Leaf masks (far from uniform): winners go to the unique list, ordered by
+    // launch_leaf_order. Node hashes: winners go to the bucket of their top bits.
     bool to_list;
     uint64_t item_cap;
     // Table of table_cap slots, 16 bytes each so that a
@@ -328,7 +346,8 @@ struct DedupArgs {
     // << 32 (table_aux = table_key + 1).
     uint64_t* table_key; uint64_t* table_aux; uint64_t table_cap;
     uint32_t* item_slot;
-    uint64_t* uniq_key; uint64_t uniq_cap;  // the unique list (leaf masks)
+    uint64_t* uniq_key; uint32_t* uniq_slot; uint64_t uniq_cap;  // the unique list (leaf masks) and its slots
+    LeafOrder* leaf; uint32_t leaf_keys;                         // its ordering; leaf_keys_for(uniq_cap)
     uint32_t* bucket_count;                                       // kDedupMaxBuckets
     // Bucket entries, one 16-byte store each: key (two words), slot, representative.
     uint4* bucket; uint64_t bucket_area;
@@ -342,10 +361,11 @@ void dedup_configure(int sms);
 // Node levels: insert (unless extract_level did), bucket sort, map; returns
 // the number of launches.
 int launch_dedup(const DedupArgs& a, cudaStream_t s);
-// Leaf masks: insert into the table and the unique list; after the caller's
-// sort of the list (keys only), assign the unique ids; then map.
+// Leaf masks: insert into the table and the unique list; order the list into
+// the leaf array and assign the unique ids (returns the number of launches);
+// then map.
 void launch_dedup_insert(const DedupArgs& a, cudaStream_t s);
-void launch_dedup_assign(const DedupArgs& a, const uint64_t* sorted, cudaStream_t s);
+int launch_leaf_order(const DedupArgs& a, cudaStream_t s);
 void launch_dedup_map(const DedupArgs& a, cudaStream_t s);
 
 constexpr uint64_t kFuseInsertMax = 1ull << 20;

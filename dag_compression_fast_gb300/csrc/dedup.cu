@@ -14,10 +14,13 @@
 //                  MurmurHash outputs, so their top bits are the bucket and
 //                  the bucket count follows from the item count; dedup_map of
 //                  the previous level zeroed the bucket counters);
-//   leaf masks     (far from uniform) the unique list is ordered by a 64-bit
-//                  keys-only radix sort (the caller's sort), then
-//   dedup_assign   finds each sorted key's slot (probing as the insert did)
-//                  and gives it its unique id (its rank);
+//   leaf_rank      (leaf masks, far from uniform) ranks the unique list, or
+//                  where it is long a sample of it, by counting smaller keys;
+//                  a list ranked whole is done: each key goes to its rank in
+//                  the leaf array and its rank to its slot (its unique id);
+//   leaf_scatter   else the keys (with their slots) go to the buckets between
+//                  every fourth (or second) sample;
+//   leaf_order     and each bucket's keys are ranked and written so;
 //   dedup_sort     (node hashes) each bucket is ranked in shared memory (rank
 //                  = number of smaller keys) and written at its global ranks,
 //                  with the representative's payload; the unique id goes to
@@ -26,9 +29,8 @@
 //                  its slot, duplicates are compared in full with their
 //                  representative (collision check). Every slot's key is
 //                  cleared once per distinct key: by dedup_sort (node hashes)
-//                  or here by the key's representative (leaf masks, after
-//                  every probe of dedup_assign); items sharing a slot
-//                  otherwise only read its aux word.
+//                  or here by the key's representative (leaf masks); items
+//                  sharing a slot otherwise only read its aux word.
 //
 // What the fixed sizes cannot hold (table, unique list, a bucket) sets
 // kErrFallback, and the caller reruns the call with the radix-sort form.
@@ -36,6 +38,8 @@
 #include "dagc_device.cuh"
 #include "dagc_kernels.h"
 #include "dagc_launch.h"
+
+#include <algorithm>
 
 namespace dagc {
 namespace {
@@ -182,6 +186,7 @@ __global__ void __launch_bounds__(256, 4) dedup_insert(DedupArgs a) {
                     aux[4ull * s[k]] = (uint32_t)i;
                     if (pos < a.uniq_cap) {
                         a.uniq_key[pos] = h[k];
+                        a.uniq_slot[pos] = s[k];
                     } else {
                         full = true;
                     }
@@ -218,34 +223,235 @@ __global__ void __launch_bounds__(256, 4) dedup_insert(DedupArgs a) {
     if (full) atomicOr(a.err, kErrFallback);
 }
 
-// Leaf masks, after the sort of the unique list: the key of rank r is the
-// r-th distinct key; the slot holding it (found by the insert's probe
-// sequence, every key being in the table) gets unique id r. The keys stay
-// until dedup_map: clearing one here could cut another key's probe sequence.
-__global__ void __launch_bounds__(256) dedup_assign(DedupArgs a, const uint64_t* sorted) {
+// ------------------------------------------- ordering the leaf masks ----
+// The distinct masks are any 64-bit values (a few bits set, or nearly all), so
+// their buckets come from a sample of them. Three launches whatever their
+// number; the first form, a radix sort of the list (eight digit passes and a
+// histogram, each gated on a one-CTA form for short lists, then a probe of the
+// table per key for its slot), was twelve, mostly latency.
+// Kernel times before / now (us): 200 masks (32^3 shell) 50 / 4; 25k (512^3
+// terrain) 116 / 28; 40k (2048^3 terrain) 106 / 31; 1.08M (8192^3 soup) 192 / 152.
+
+// Samples and buckets for u distinct masks. Up to kLeafRankMax every mask is a
+// "sample" and its rank is final. Else a bucket holds the keys between every
+// fourth sample: its size is a gamma distribution of shape 4, with a mean of at
+// most 256 keys up to 2^18 masks, 2048 at the list's limit.
+__device__ __forceinline__ void leaf_shape(uint64_t u, uint32_t* samples, uint32_t* buckets) {
+    if (u <= kLeafRankMax) { *samples = (uint32_t)u; *buckets = 0; }
+    else if (u <= kLeafMidMax) { *samples = kLeafRankMax / 2; *buckets = kLeafBuckets / 2; }
+    else { *samples = kLeafRankMax; *buckets = kLeafBuckets; }
+}
+// Position of sample i in the unique list (all different: u >= samples, which
+// are a power of two unless they are all of the list).
+__device__ __forceinline__ uint64_t sample_pos(uint32_t i, uint64_t u, uint32_t samples) {
+    return samples == u ? (uint64_t)i : ((uint64_t)i * u) >> (31 - __clz(samples));
+}
+
+// Entry room per bucket: eight times the mean or more, up to the shared memory
+// of leaf_order (four times the mean at the list's limit).
+__device__ __forceinline__ uint32_t leaf_bucket_cap(const DedupArgs& a, uint32_t buckets) {
+    const uint64_t room = a.bucket_area / buckets;
+    return (uint32_t)(room < a.leaf_keys ? room : a.leaf_keys);
+}
+
+constexpr int kRankThreads = 1024;
+constexpr int kRankPer = kRankThreads / 32;  // keys per CTA and round, a warp each
+constexpr int kRankCtas = 128;
+
+// Every CTA holds all the samples in shared memory and ranks its share of them,
+// a warp to a key: the samples' square over the GPU (8192: 67M comparisons).
+// Few large CTAs, since each fetches every sample, a sector apiece (256 CTAs of
+// 256 threads: 17 us for 4096 samples, 40 for 8192; these take 9 and 23).
+__global__ void __launch_bounds__(kRankThreads) leaf_rank(DedupArgs a) {
     pdl_prologue();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint64_t* key = reinterpret_cast<uint64_t*>(smem_raw);  // kLeafRankMax
     const uint64_t u = unique_count(a);
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.d_out_n = u < a.out_capacity ? u : a.out_capacity;
-    const uint64_t n = *a.d_n;
-    const uint64_t S = table_size_for(n, true);
-    if (S > a.table_cap || n > a.item_cap) return;  // insert did nothing (fallback set)
-    const uint32_t S32 = (uint32_t)S;
+    uint32_t ns, nb;
+    leaf_shape(u, &ns, &nb);
+    if (blockIdx.x * kRankPer >= ns) return;
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < ns; i += kRankThreads) key[i] = a.uniq_key[sample_pos(i, u, ns)];
+    __syncthreads();
     uint32_t* aux = reinterpret_cast<uint32_t*>(a.table_aux);
-    bool lost = false;
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < u; r += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t key = sorted[r];
-        uint32_t sl = (uint32_t)home_slot(key, S);
-        bool hit = false;
-        for (uint32_t probe = 0; probe < S32; ++probe) {
-            const uint64_t cur = a.table_key[2ull * sl];
-            if (cur == key) { hit = true; break; }
-            if (cur == 0) break;
-            sl = next_slot(sl, S32);
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t i = blockIdx.x * kRankPer + (threadIdx.x >> 5); i < ns; i += gridDim.x * kRankPer) {
+        const uint64_t k = key[i];
+        uint32_t r = 0;
+#pragma unroll 8
+        for (uint32_t x = lane; x < ns; x += 32) r += key[x] < k;
+        r = __reduce_add_sync(0xFFFFFFFFu, r);
+        if (lane != 0) continue;
+        if (nb == 0) {
+            if (r < a.out_capacity) {
+                a.out_keys[r] = k;
+                aux[4ull * a.uniq_slot[i] + 1] = r;
+            } else {
+                atomicOr(a.err, kErrCapacity);
+            }
+        } else if (r % (ns / nb) == 0) {
+            a.leaf->splitter[r / (ns / nb)] = k;
         }
-        if (hit && r < a.out_capacity) aux[4ull * sl + 1] = (uint32_t)r;
-        else lost = true;
     }
-    if (lost) atomicOr(a.err, kErrCapacity);
+}
+
+// Bucket b holds the keys from splitter b (b = 0: any) up to splitter b + 1.
+constexpr int kLeafIlp = 4;
+__global__ void __launch_bounds__(512) leaf_scatter(DedupArgs a) {
+    pdl_prologue();
+    __shared__ uint64_t spl[kLeafBuckets];
+    const uint64_t u = unique_count(a);
+    uint32_t ns, nb;
+    leaf_shape(u, &ns, &nb);
+    const uint64_t per = 512ull * kLeafIlp;
+    if (nb == 0 || blockIdx.x * per >= u) return;
+    for (uint32_t i = threadIdx.x; i < nb; i += 512) spl[i] = a.leaf->splitter[i];
+    __syncthreads();
+    const uint32_t cap = leaf_bucket_cap(a, nb);
+    bool full = false;
+    for (uint64_t i0 = blockIdx.x * per + threadIdx.x; i0 < u; i0 += gridDim.x * per) {
+        uint64_t k[kLeafIlp];
+        uint32_t s[kLeafIlp], b[kLeafIlp], pos[kLeafIlp];
+#pragma unroll
+        for (int q = 0; q < kLeafIlp; ++q) {
+            const uint64_t i = i0 + q * 512;
+            k[q] = i < u ? a.uniq_key[i] : 0;
+            s[q] = i < u ? a.uniq_slot[i] : 0;
+            b[q] = 0;
+        }
+        // The last splitter not above the key, among the nb - 1 after the first.
+        for (uint32_t half = nb / 2; half > 0; half /= 2) {
+#pragma unroll
+            for (int q = 0; q < kLeafIlp; ++q)
+                if (spl[b[q] + half] <= k[q]) b[q] += half;
+        }
+#pragma unroll
+        for (int q = 0; q < kLeafIlp; ++q) pos[q] = i0 + q * 512 < u ? atomicAdd(&a.leaf->count[b[q]], 1u) : 0u;
+#pragma unroll
+        for (int q = 0; q < kLeafIlp; ++q) {
+            if (i0 + q * 512 >= u) continue;
+            if (pos[q] < cap) {
+                a.bucket[(uint64_t)b[q] * cap + pos[q]] = make_uint4((uint32_t)k[q], (uint32_t)(k[q] >> 32), s[q], 0u);
+            } else {
+                full = true;  // a bucket past its room (a very uneven sample)
+            }
+        }
+    }
+    if (full) atomicOr(a.err, kErrFallback);
+}
+
+// Each CTA takes a range of buckets. A bucket's keys are put in sub-buckets
+// between kSub of them (ranked by counting) and ranked by counting within those:
+// some 20 shared-memory reads per key whatever the bucket's size (counting over
+// whole buckets, 264 keys on average at 1.08M masks, took four times as long as
+// the radix sort).
+constexpr uint32_t kSub = 64;
+constexpr uint32_t kSubMin = 96;  // up to here a bucket is counted whole
+
+// Room for 2048 keys per bucket (20 KB): 256 threads; for 8192 (80 KB, two CTAs
+// per SM): 512.
+template <int kOrderThreads>
+__global__ void __launch_bounds__(kOrderThreads) leaf_order(DedupArgs a) {
+    pdl_prologue();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint64_t* key = reinterpret_cast<uint64_t*>(smem_raw);              // leaf_keys
+    uint16_t* ord = reinterpret_cast<uint16_t*>(key + a.leaf_keys);     // keys in sub-bucket order
+    __shared__ uint64_t spl[kSub];
+    __shared__ uint32_t cnt[kSub], sub0[kSub + 1];
+    __shared__ uint32_t red[kOrderThreads / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint64_t u = unique_count(a);
+    uint32_t ns, nb;
+    leaf_shape(u, &ns, &nb);
+    const uint32_t b0 = (uint32_t)((uint64_t)nb * blockIdx.x / gridDim.x);
+    const uint32_t b1 = (uint32_t)((uint64_t)nb * (blockIdx.x + 1) / gridDim.x);
+    if (b0 >= b1) return;
+    uint32_t part = 0;
+    for (uint32_t x = tid; x < b0; x += kOrderThreads) part += a.leaf->count[x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xFFFFFFFFu, part, o);
+    if (lane == 0) red[warp] = part;
+    __syncthreads();
+    uint64_t start = 0;
+    for (int w = 0; w < kOrderThreads / 32; ++w) start += red[w];
+    const uint32_t cap = leaf_bucket_cap(a, nb);
+    uint32_t* aux = reinterpret_cast<uint32_t*>(a.table_aux);
+    bool bad = false;
+    auto put = [&](const uint4* ent, uint32_t j, uint64_t k, uint64_t uid) {
+        const uint32_t slot = ent[j].z;
+        if (uid < a.out_capacity && slot < a.table_cap) {
+            a.out_keys[uid] = k;
+            aux[4ull * slot + 1] = (uint32_t)uid;
+        } else {
+            bad = true;
+        }
+    };
+    auto sub_of = [&](uint64_t k) {  // the last of spl not above k, among those after the first
+        uint32_t s = 0;
+#pragma unroll
+        for (uint32_t half = kSub / 2; half > 0; half /= 2)
+            if (spl[s + half] <= k) s += half;
+        return s;
+    };
+    for (uint32_t b = b0; b < b1; ++b) {
+        const uint32_t total = a.leaf->count[b], c = min(total, cap);  // beyond: flagged by leaf_scatter
+        const uint4* ent = a.bucket + (uint64_t)b * cap;
+        __syncthreads();  // the bucket before is no longer read
+        for (uint32_t j = tid; j < c; j += kOrderThreads) {
+            const uint4 e = ent[j];
+            key[j] = (uint64_t)e.x | (uint64_t)e.y << 32;
+        }
+        if (tid < kSub) cnt[tid] = 0;
+        __syncthreads();
+        if (c <= kSubMin) {
+            if (tid < c) {
+                const uint64_t k = key[tid];
+                uint32_t r = 0;
+#pragma unroll 8
+                for (uint32_t x = 0; x < c; ++x) r += key[x] < k;
+                put(ent, tid, k, start + r);
+            }
+            start += total;
+            continue;
+        }
+        if (tid < kSub) {
+            const uint64_t k = key[tid * c / kSub];
+            uint32_t r = 0;
+#pragma unroll 8
+            for (uint32_t x = 0; x < kSub; ++x) r += key[x * c / kSub] < k;
+            spl[r] = k;
+        }
+        __syncthreads();
+        for (uint32_t j = tid; j < c; j += kOrderThreads) atomicAdd(&cnt[sub_of(key[j])], 1u);
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t n0 = cnt[2 * lane], n1 = cnt[2 * lane + 1];
+            uint32_t x = n0 + n1;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                if (lane >= (uint32_t)o) x += y;
+            }
+            const uint32_t s0 = x - n0 - n1;
+            cnt[2 * lane] = sub0[2 * lane] = s0;
+            cnt[2 * lane + 1] = sub0[2 * lane + 1] = s0 + n0;
+            if (lane == 31) sub0[kSub] = x;
+        }
+        __syncthreads();
+        for (uint32_t j = tid; j < c; j += kOrderThreads) ord[atomicAdd(&cnt[sub_of(key[j])], 1u)] = (uint16_t)j;
+        __syncthreads();
+        for (uint32_t i = tid; i < c; i += kOrderThreads) {
+            const uint32_t j = ord[i];
+            const uint64_t k = key[j];
+            const uint32_t s = sub_of(k), s0 = sub0[s], s1 = sub0[s + 1];
+            uint32_t r = s0;
+            for (uint32_t x = s0; x < s1; ++x) r += key[ord[x]] < k;
+            put(ent, j, k, start + r);
+        }
+        start += total;
+    }
+    if (bad) atomicOr(a.err, kErrCapacity);
 }
 
 // Each CTA takes a contiguous range of buckets; a bucket's keys are distinct,
@@ -400,6 +606,8 @@ int g_sms = 152;
 
 void dedup_configure(int sms) {
     cudaFuncSetAttribute(dedup_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kDedupTopBitCap * 8));
+    cudaFuncSetAttribute(leaf_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kLeafRankMax * 8));
+    cudaFuncSetAttribute(leaf_order<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(leaf_keys_for(kDedupMaxUnique) * 10));
     g_sms = sms > 0 ? sms : 152;
 }
 
@@ -415,10 +623,17 @@ void launch_dedup_insert(const DedupArgs& a, cudaStream_t s) {
     launch_pdl(dedup_insert, dim3(item_grid(a)), dim3(256), 0, s, a);
 }
 
-void launch_dedup_assign(const DedupArgs& a, const uint64_t* sorted, cudaStream_t s) {
-    const uint64_t want = (a.uniq_cap + 255) / 256;
-    const int g = (int)(want < (uint64_t)(8 * g_sms) ? (want > 0 ? want : 1) : 8 * g_sms);
-    launch_pdl(dedup_assign, dim3(g), dim3(256), 0, s, a, sorted);
+int launch_leaf_order(const DedupArgs& a, cudaStream_t s) {
+    const int ranks = (int)std::min<uint64_t>((a.uniq_cap + kRankPer - 1) / kRankPer, kRankCtas);
+    launch_pdl(leaf_rank, dim3(ranks), dim3(kRankThreads), std::min<uint64_t>(a.uniq_cap, kLeafRankMax) * 8, s, a);
+    if (a.uniq_cap <= kLeafRankMax) return 1;  // no list is longer
+    const uint64_t want = (a.uniq_cap + 512 * kLeafIlp - 1) / (512 * kLeafIlp);
+    launch_pdl(leaf_scatter, dim3((unsigned)std::min<uint64_t>(want, 2ull * g_sms)), dim3(512), 0, s, a);
+    if (a.uniq_cap <= kLeafMidMax)
+        launch_pdl(leaf_order<256>, dim3(kLeafBuckets / 2), dim3(256), a.leaf_keys * 10, s, a);
+    else
+        launch_pdl(leaf_order<512>, dim3(2 * g_sms), dim3(512), a.leaf_keys * 10, s, a);
+    return 3;
 }
 
 void launch_dedup_map(const DedupArgs& a, cudaStream_t s) {
