@@ -2155,6 +2155,7 @@ int dagc_context_create(int device, dagc_context* out) {
     group_configure(c->sms);
     direct_configure(c->sms);
     chunk_configure(c->sms);
+    voxelize_configure();
     *out = c.release();
     return DAGC_OK;
 }

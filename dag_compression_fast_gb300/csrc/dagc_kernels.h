@@ -404,11 +404,13 @@ constexpr int kVoxSAT = 1;  // every voxel the triangle touches (separating axis
 struct VoxArgs {
     const double* vertices; uint64_t n_tri;  // 9 doubles per triangle
     double aabb[6];                          // box mapped onto the grid: min xyz, max xyz
+    double scale[3];                         // 2^depth / extent (set by launch_voxelize)
     int depth, mode;
     uint64_t* codes; uint64_t capacity;
     uint64_t* d_total;                       // fragments produced (may exceed capacity)
     uint64_t* status; uint32_t* tile_counter; uint32_t* err;  // status: voxelize_tiles + 1 words, zero
 };
+void voxelize_configure();
 void launch_voxelize(const VoxArgs& a, int grid, cudaStream_t s);
 uint64_t voxelize_tiles(uint64_t n_tri);
 

@@ -15,30 +15,55 @@
 //           axis test (Akenine-Moller 2001); float64. The 26-connected
 //           surface used for the triangle-soup workload.
 //
-// One warp per triangle, lanes striding over the triangle's bounding box
-// (rows of pixels / voxel columns), so that large triangles spread over 32
-// lanes; per-tile fragment counts give the output offsets through a single
-// decoupled look-back, so the output order is fixed: triangles in input
-// order, each triangle's fragments in bounding-box order. This file is
-// compiled with --fmad=false: every float operation rounds once, as in the
-// CPU checkers.
+// Tiles of kVoxTile triangles: each triangle is set up by one thread (its
+// constants go to shared memory), then tested by one warp, lanes striding over
+// its bounding box (rows of pixels / voxel columns), so that large triangles
+// spread over 32 lanes. The hits found while counting are kept (packed local
+// positions, per warp) and only their codes are left to compute once the
+// per-tile counts have given the output offsets, through a single decoupled
+// look-back. The output order is fixed: triangles in input order, each
+// triangle's fragments in bounding-box order. A call without room for codes
+// only counts. This file is compiled with --fmad=false: every float operation
+// rounds once, as in the CPU checkers (but for the explicit fmaf of the SAT
+// filter, whose error bound covers it).
+//
+// Each form is bound by the arithmetic per candidate. A counting and a writing
+// call together: 500k triangles, depth 12, the GL rule, 2640 us when every lane
+// of the warp repeated the setup and a second pass repeated the tests, now 660;
+// 60k triangles, depth 11, the SAT rule, 57 ms when it ran in float64 throughout
+// (of which this part does 2 operations per SM and clock), now 0.89.
 
 #include "dagc_device.cuh"
 #include "dagc_kernels.h"
+
+#include <type_traits>
 
 namespace dagc {
 namespace {
 
 constexpr int kVoxThreads = 256;
 constexpr int kVoxWarps = kVoxThreads / 32;
-constexpr int kVoxTile = kVoxThreads;  // triangles per tile, one per thread for the scan
+// Triangles per tile: small, so that a call of a few thousand triangles
+// spreads over the GPU.
+constexpr int kVoxTile = 64;
+// Hits kept per warp from the count to the emission, and the mark of a
+// triangle whose hits were not kept (it is tested again).
+constexpr int kVoxKeep = 768;
+constexpr uint32_t kNotKept = 0xFFFFFFFFu;
 
-__device__ __forceinline__ uint64_t morton3(uint64_t x, uint64_t y, uint64_t z) {
-    uint64_t c = 0;
-#pragma unroll 1
-    for (int b = 0; b < 21; ++b)
-        c |= ((x >> b) & 1) << (3 * b + 2) | ((y >> b) & 1) << (3 * b + 1) | ((z >> b) & 1) << (3 * b);
-    return c;
+// The low 11 bits of x, each moved to three times its place.
+__device__ __forceinline__ uint64_t spread11(uint32_t x) {
+    x &= 0x7FFu;
+    const uint64_t top = (uint64_t)(x >> 10) << 30;
+    x = (x | x << 16) & 0x030000FFu;
+    x = (x | x << 8) & 0x0300F00Fu;
+    x = (x | x << 4) & 0x030C30C3u;
+    x = (x | x << 2) & 0x09249249u;
+    return top | x;
+}
+__device__ __forceinline__ uint64_t spread21(uint32_t x) { return spread11(x & 0x3FFu) | spread11((x >> 10) & 0x7FFu) << 30; }
+__device__ __forceinline__ uint64_t morton3(uint32_t x, uint32_t y, uint32_t z) {
+    return spread21(x) << 2 | spread21(y) << 1 | spread21(z);
 }
 
 // ---------------------------------------------------------------- GL rule --
@@ -118,27 +143,25 @@ __device__ GlTri gl_setup(const double* P, const double* aabb, int depth) {
     return t;
 }
 
-// Pixel (i, j): covered? and its voxel's Morton code.
-__device__ __forceinline__ bool gl_pixel(const GlTri& t, int i, int j, int G, uint64_t* code) {
+// Is pixel (i, j) covered?
+__device__ __forceinline__ bool gl_covered(const GlTri& t, int i, int j) {
     bool covered = true;
 #pragma unroll
     for (int k = 0; k < 3; ++k)
         covered = covered && t.nx[k] * ((float)i - t.U[k]) + t.ny[k] * ((float)j - t.V[k]) + t.dk[k] >= 0.0f;
-    if (!covered) return false;
+    return covered;
+}
+// The Morton code of a covered pixel's voxel.
+__device__ __forceinline__ uint64_t gl_code(const GlTri& t, int i, int j, int G) {
     const float zc = t.W[0] + t.dwdu * (((float)i + 0.5f) - t.U[0]) + t.dwdv * (((float)j + 0.5f) - t.V[0]);
     const float hx = 0.5f * t.dwdu, hy = 0.5f * t.dwdv;
     const int s0 = clamp_cell(zc, G);
     const int s1 = clamp_cell(zc + hx + hy, G), s2 = clamp_cell(zc + hx - hy, G);
     const int s3 = clamp_cell(zc - hx + hy, G), s4 = clamp_cell(zc - hx - hy, G);
     const int k = min(min(min(s0, s1), min(s2, s3)), s4);
-    uint64_t xyz[3];
-    const int ua = t.axis == 0 ? 2 : (t.axis == 1 ? 0 : 1);
-    const int va = t.axis == 0 ? 1 : (t.axis == 1 ? 2 : 0);
-    xyz[ua] = (uint64_t)i;
-    xyz[va] = (uint64_t)j;
-    xyz[t.axis] = (uint64_t)k;
-    *code = morton3(xyz[0], xyz[1], xyz[2]);
-    return true;
+    // View axes back: X (u, v, w) = (z, y, x), Y (x, z, y), Z (y, x, z).
+    const uint64_t u = spread21((uint32_t)i), v = spread21((uint32_t)j), w = spread21((uint32_t)k);
+    return t.axis == 0 ? w << 2 | v << 1 | u : t.axis == 1 ? u << 2 | w << 1 | v : v << 2 | u << 1 | w;
 }
 
 // --------------------------------------------------------------- SAT rule --
@@ -178,138 +201,302 @@ __device__ bool tri_box(D3 c, double h, D3 a, D3 b, D3 d) {
     return fabs(dist) <= r;
 }
 
+__device__ __forceinline__ D3 sat_vertex(const double* P, const double* aabb, const double* scale, int k) {
+    return {(P[3 * k + 0] - aabb[0]) * scale[0], (P[3 * k + 1] - aabb[1]) * scale[1], (P[3 * k + 2] - aabb[2]) * scale[2]};
+}
+// The rule itself, for one voxel: float64, in the checkers' order.
+__device__ __noinline__ bool sat_exact(const VoxArgs& a, uint64_t tri, int64_t x, int64_t y, int64_t z) {
+    const double* P = a.vertices + 9 * tri;
+    const D3 c{(double)x + 0.5, (double)y + 0.5, (double)z + 0.5};
+    return tri_box(c, 0.5, sat_vertex(P, a.aabb, a.scale, 0), sat_vertex(P, a.aabb, a.scale, 1),
+                   sat_vertex(P, a.aabb, a.scale, 2));
+}
+
+// A triangle's float32 filter. Its tests are tri_box's, rewritten for a fixed
+// triangle and a moving voxel centre c: the triangle's projection on an axis is
+// separated from the cube's when |axis . c - mid| > half, with mid and half
+// from the triangle alone. Coordinates are relative to an integer origin near
+// the box's centre; K bounds every |coordinate| and |c|. With u = 2^-24, the
+// float32 coordinates are off by uK, the edges by 4uK, an edge axis's
+// axis . c by 14uK^2, its mid and half by 24uK^2 (the cross products with unit
+// vectors are single components); the normal by 50uK^2, normal . c and its mid
+// by 250uK^3 each; the float64 rule itself by less than a unit of these. So
+// beyond half + 128uK^2 (1024uK^3 for the normal) an axis separates for sure,
+// below half minus that it does not; a voxel that no axis separates for sure
+// and some axis leaves open is decided by sat_exact. The three box normals
+// never separate a voxel of the bounding box. K above 2^16, or not a number:
+// every voxel by sat_exact.
 struct SatTri {
-    D3 v[3];
-    int64_t x0, y0, z0, nx, ny, nz;  // bounding box origin and extents (0 extent: empty)
+    float e[3][3];                                  // edges v1 - v0, v2 - v1, v0 - v2
+    float mid[3][3], out[3][3], in[3][3];           // per box axis i and edge j
+    float n[3], nmid, nout, nin;
+    int x0, y0, z0;                                  // bounding box origin
+    int nx, ny, nz;                                  // and extents (0: empty)
+    int ox, oy, oz;                                  // the filter's origin
+    bool exact;
 };
 
 __device__ __forceinline__ int64_t cell_floor(double m, double G) { return (int64_t)floor(dmin(dmax(m, -1.0), G)); }
 
-__device__ SatTri sat_setup(const double* P, const double* aabb, int depth) {
-    SatTri t;
-    const double G = (double)((int64_t)1 << depth);
-    const int64_t Gi = (int64_t)1 << depth;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        t.v[k].x = (P[3 * k + 0] - aabb[0]) * (G / (aabb[3] - aabb[0]));
-        t.v[k].y = (P[3 * k + 1] - aabb[1]) * (G / (aabb[4] - aabb[1]));
-        t.v[k].z = (P[3 * k + 2] - aabb[2]) * (G / (aabb[5] - aabb[2]));
-    }
-    const D3 a = t.v[0], b = t.v[1], c = t.v[2];
+__device__ void sat_setup(const VoxArgs& args, uint64_t tri, SatTri& t) {
+    const double* P = args.vertices + 9 * tri;
+    const double G = (double)((int64_t)1 << args.depth);
+    const int64_t Gi = (int64_t)1 << args.depth;
+    const D3 v[3] = {sat_vertex(P, args.aabb, args.scale, 0), sat_vertex(P, args.aabb, args.scale, 1),
+                     sat_vertex(P, args.aabb, args.scale, 2)};
+    const D3 a = v[0], b = v[1], c = v[2];
     int64_t x0 = cell_floor(dmin(a.x, dmin(b.x, c.x)), G), x1 = cell_floor(dmax(a.x, dmax(b.x, c.x)), G);
     int64_t y0 = cell_floor(dmin(a.y, dmin(b.y, c.y)), G), y1 = cell_floor(dmax(a.y, dmax(b.y, c.y)), G);
     int64_t z0 = cell_floor(dmin(a.z, dmin(b.z, c.z)), G), z1 = cell_floor(dmax(a.z, dmax(b.z, c.z)), G);
     x0 = x0 < 0 ? 0 : x0; y0 = y0 < 0 ? 0 : y0; z0 = z0 < 0 ? 0 : z0;
     x1 = x1 > Gi - 1 ? Gi - 1 : x1; y1 = y1 > Gi - 1 ? Gi - 1 : y1; z1 = z1 > Gi - 1 ? Gi - 1 : z1;
-    t.x0 = x0; t.y0 = y0; t.z0 = z0;
-    t.nx = x1 >= x0 ? x1 - x0 + 1 : 0;
-    t.ny = y1 >= y0 ? y1 - y0 + 1 : 0;
-    t.nz = z1 >= z0 ? z1 - z0 + 1 : 0;
-    return t;
+    t.nx = x1 >= x0 ? (int)(x1 - x0 + 1) : 0;
+    t.ny = y1 >= y0 ? (int)(y1 - y0 + 1) : 0;
+    t.nz = z1 >= z0 ? (int)(z1 - z0 + 1) : 0;
+    t.x0 = (int)x0; t.y0 = (int)y0; t.z0 = (int)z0;
+    t.exact = true;
+    if (t.nx == 0 || t.ny == 0 || t.nz == 0) return;
+    t.ox = t.x0 + t.nx / 2;
+    t.oy = t.y0 + t.ny / 2;
+    t.oz = t.z0 + t.nz / 2;
+    float f[3][3];
+    float K = (float)(max(t.nx, max(t.ny, t.nz)) / 2 + 2);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        f[k][0] = (float)(v[k].x - (double)t.ox);
+        f[k][1] = (float)(v[k].y - (double)t.oy);
+        f[k][2] = (float)(v[k].z - (double)t.oz);
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            if (!(fabsf(f[k][x]) <= 65536.0f)) return;  // far outside the grid, or not a number
+            K = fmaxf(K, fabsf(f[k][x]) + 1.0f);
+        }
+    }
+    if (!(K <= 65536.0f)) return;
+    t.exact = false;
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        t.e[0][x] = f[1][x] - f[0][x];
+        t.e[1][x] = f[2][x] - f[1][x];
+        t.e[2][x] = f[0][x] - f[2][x];
+    }
+    const float slack = 0x1p-17f * K * K;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        // Box axis i crossed with edge e: components y = -e_z, z = e_y in the
+        // cyclic order (i, y, z) of the coordinates.
+        const int y = (i + 1) % 3, z = (i + 2) % 3;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const float ey = t.e[j][y], ez = t.e[j][z];
+            // The edge's two ends project alike; the third vertex is j + 2.
+            const int o = (j + 2) % 3;
+            const float p = ey * f[j][z] - ez * f[j][y], q = ey * f[o][z] - ez * f[o][y];
+            const float half = 0.5f * (fabsf(ey) + fabsf(ez)) + 0.5f * fabsf(p - q);
+            t.mid[i][j] = 0.5f * (p + q);
+            t.out[i][j] = half + slack;
+            t.in[i][j] = half - slack;
+        }
+    }
+    float r = 0.0f, d = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int y = (i + 1) % 3, z = (i + 2) % 3;
+        t.n[i] = t.e[0][y] * t.e[1][z] - t.e[0][z] * t.e[1][y];
+        r += 0.5f * fabsf(t.n[i]);
+        d += t.n[i] * f[0][i];
+    }
+    const float nslack = 0x1p-14f * K * K * K;
+    t.nmid = d;
+    t.nout = r + nslack;
+    t.nin = r - nslack;
+}
+
+// Whether voxel (x, y, z) of the bounding box is hit.
+__device__ __forceinline__ bool sat_hit(const VoxArgs& a, uint64_t tri, const SatTri& t, int x, int y, int z) {
+    bool open = t.exact;
+    if (!t.exact) {
+        const float c[3] = {(float)(x - t.ox) + 0.5f, (float)(y - t.oy) + 0.5f, (float)(z - t.oz) + 0.5f};
+        const float s = fabsf(fmaf(t.n[0], c[0], fmaf(t.n[1], c[1], t.n[2] * c[2])) - t.nmid);
+        if (s > t.nout) return false;
+        open = s > t.nin;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const int u = (i + 1) % 3, w = (i + 2) % 3;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const float q = fabsf(fmaf(t.e[j][u], c[w], -(t.e[j][w] * c[u])) - t.mid[i][j]);
+                if (q > t.out[i][j]) return false;
+                open |= q > t.in[i][j];
+            }
+        }
+    }
+    return !open || sat_exact(a, tri, x, y, z);
 }
 
 // ------------------------------------------------------------------ kernel --
+template <int kMode>
 struct VoxSmem {
-    uint64_t count[kVoxTile];
+    typename std::conditional<kMode == kVoxGL, GlTri, SatTri>::type tri[kVoxTile];
+    uint64_t count[kVoxTile];             // fragments, then offsets inside the tile
+    uint32_t kept_at[kVoxTile];           // the triangle's hits in its warp's list, or kNotKept
+    uint32_t kept[kVoxWarps][kVoxKeep];
     uint64_t scan[34];
     uint32_t slot;
     uint64_t base;
 };
 
-// Fragments of triangle `tri` counted (kEmit false) or written from
-// out[pos] on (kEmit true) by the whole warp; returns the count. Every lane
-// runs the same loop trip count, so each ballot is made by all 32 lanes.
+// A triangle's candidates, walked by the lanes of a warp 32 at a time in
+// bounding-box order (z, or the pixel column, fastest): the lane's position
+// moves on without a division.
+struct BoxWalk {
+    uint32_t nz, ny;     // the two inner extents
+    uint32_t dz, dy, dx; // 32 candidates on
+    uint32_t x, y, z;
+    __device__ BoxWalk(uint32_t ny_, uint32_t nz_, uint32_t lane) : nz(nz_), ny(ny_) {
+        dz = 32 % nz;
+        const uint32_t rows = 32 / nz;
+        dy = rows % ny;
+        dx = rows / ny;
+        z = lane % nz;
+        const uint32_t row = lane / nz;
+        y = row % ny;
+        x = row / ny;
+    }
+    __device__ __forceinline__ void next() {
+        z += dz;
+        y += dy;
+        x += dx;
+        if (z >= nz) { z -= nz; ++y; }
+        if (y >= ny) { y -= ny; ++x; }
+    }
+};
+
+// The warp tests triangle k of the tile. kEmit: the hits' codes go out from
+// `pos` on. Otherwise they are counted and kept in the warp's list from
+// `at` on, where they fit and their local positions pack into a word. Every
+// lane runs the same trip count, so each ballot is made by all 32 lanes.
 template <int kMode, bool kEmit>
-__device__ uint64_t warp_triangle(const VoxArgs& a, uint64_t tri, uint64_t pos) {
-    const uint32_t lane = threadIdx.x & 31;
-    const double* P = a.vertices + 9 * tri;
+__device__ uint64_t warp_triangle(const VoxArgs& a, VoxSmem<kMode>& S, uint64_t tri, uint32_t k, uint64_t pos, uint32_t at) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const auto& t = S.tri[k];
     const int G = 1 << a.depth;
-    uint64_t n = 0;
-    if (kMode == kVoxGL) {
-        const GlTri t = gl_setup(P, a.aabb, a.depth);
+    uint64_t area;
+    uint32_t ny, nz;
+    bool packs;
+    if constexpr (kMode == kVoxGL) {
         if (t.empty) return 0;
-        const uint64_t w = (uint64_t)(t.i1 - t.i0 + 1), area = w * (uint64_t)(t.j1 - t.j0 + 1);
-        for (uint64_t b = 0; b < area; b += 32) {
-            const uint64_t idx = b + lane;
-            uint64_t code = 0;
-            const bool hit = idx < area && gl_pixel(t, t.i0 + (int)(idx % w), t.j0 + (int)(idx / w), G, &code);
-            const uint32_t m = __ballot_sync(0xFFFFFFFFu, hit);
-            if (kEmit && hit) {
-                const uint64_t o = pos + n + __popc(m & lanemask_lt());
-                if (o < a.capacity) a.codes[o] = code;
-            }
-            n += __popc(m);
-        }
+        ny = (uint32_t)(t.j1 - t.j0 + 1);
+        nz = (uint32_t)(t.i1 - t.i0 + 1);
+        area = (uint64_t)ny * nz;
+        packs = ny <= 65536 && nz <= 65536;
     } else {
-        const SatTri t = sat_setup(P, a.aabb, a.depth);
-        const uint64_t area = (uint64_t)t.nx * (uint64_t)t.ny * (uint64_t)t.nz;
-        const uint64_t yz = (uint64_t)t.ny * (uint64_t)t.nz;
-        for (uint64_t b = 0; b < area; b += 32) {
-            const uint64_t idx = b + lane;
-            bool hit = false;
-            int64_t x = 0, y = 0, z = 0;
-            if (idx < area) {
-                x = t.x0 + (int64_t)(idx / yz);
-                const uint64_t r = idx % yz;
-                y = t.y0 + (int64_t)(r / (uint64_t)t.nz);
-                z = t.z0 + (int64_t)(r % (uint64_t)t.nz);
-                const D3 c{(double)x + 0.5, (double)y + 0.5, (double)z + 0.5};
-                hit = tri_box(c, 0.5, t.v[0], t.v[1], t.v[2]);
+        ny = (uint32_t)t.ny;
+        nz = (uint32_t)t.nz;
+        area = (uint64_t)t.nx * ny * nz;
+        if (area == 0) return 0;
+        packs = t.nx <= 1024 && ny <= 1024 && nz <= 1024;
+    }
+    BoxWalk w(ny, nz, lane);
+    uint64_t n = 0;
+    for (uint64_t b = 0; b < area; b += 32, w.next()) {
+        bool hit = b + lane < area;
+        if constexpr (kMode == kVoxGL) hit = hit && gl_covered(t, t.i0 + (int)w.z, t.j0 + (int)w.y);
+        else hit = hit && sat_hit(a, tri, t, t.x0 + (int)w.x, t.y0 + (int)w.y, t.z0 + (int)w.z);
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, hit);
+        if (hit) {
+            const uint64_t o = n + __popc(m & lanemask_lt());
+            if constexpr (kEmit) {
+                uint64_t code;
+                if constexpr (kMode == kVoxGL) code = gl_code(t, t.i0 + (int)w.z, t.j0 + (int)w.y, G);
+                else code = morton3((uint32_t)t.x0 + w.x, (uint32_t)t.y0 + w.y, (uint32_t)t.z0 + w.z);
+                if (pos + o < a.capacity) a.codes[pos + o] = code;
+            } else if (packs && at + o < (uint64_t)kVoxKeep) {
+                S.kept[warp][at + o] = kMode == kVoxGL ? w.y << 16 | w.z : w.x << 20 | w.y << 10 | w.z;
             }
-            const uint32_t m = __ballot_sync(0xFFFFFFFFu, hit);
-            if (kEmit && hit) {
-                const uint64_t o = pos + n + __popc(m & lanemask_lt());
-                if (o < a.capacity) a.codes[o] = morton3((uint64_t)x, (uint64_t)y, (uint64_t)z);
-            }
-            n += __popc(m);
         }
+        n += __popc(m);
+    }
+    if constexpr (!kEmit) {
+        if (lane == 0) S.kept_at[k] = packs && at + n <= (uint64_t)kVoxKeep ? at : kNotKept;
     }
     return n;
 }
 
 template <int kMode>
 __global__ void __launch_bounds__(kVoxThreads) voxelize(VoxArgs a) {
-    __shared__ VoxSmem S;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    VoxSmem<kMode>& S = *reinterpret_cast<VoxSmem<kMode>*>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int G = 1 << a.depth;
     const uint64_t ntiles = (a.n_tri + kVoxTile - 1) / kVoxTile;
     while (true) {
         if (tid == 0) S.slot = atomicAdd(a.tile_counter, 1u);
         __syncthreads();
         const uint64_t tile = S.slot;
-        __syncthreads();
         if (tile >= ntiles) break;
         const uint64_t t0 = tile * kVoxTile;
+        if (tid < kVoxTile && t0 + tid < a.n_tri) {
+            if constexpr (kMode == kVoxGL) S.tri[tid] = gl_setup(a.vertices + 9 * (t0 + tid), a.aabb, a.depth);
+            else sat_setup(a, t0 + tid, S.tri[tid]);
+        }
+        __syncthreads();
         // Count: warp w takes triangles t0 + w, t0 + w + 8, ...
+        uint32_t at = 0;
         for (uint32_t k = warp; k < kVoxTile; k += kVoxWarps) {
             const uint64_t tri = t0 + k;
-            const uint64_t c = tri < a.n_tri ? warp_triangle<kMode, false>(a, tri, 0) : 0;
+            const uint64_t c = tri < a.n_tri ? warp_triangle<kMode, false>(a, S, tri, k, 0, at) : 0;
+            __syncwarp();
             if (lane == 0) S.count[k] = c;
+            if (c && S.kept_at[k] != kNotKept) at += (uint32_t)c;
         }
         __syncthreads();
         uint64_t total;
-        const uint64_t excl = block_exclusive_sum<uint64_t>(S.count[tid], S.scan, &total);
-        __syncthreads();
-        S.count[tid] = excl;  // now the triangle's offset inside the tile
+        const uint64_t excl = block_exclusive_sum<uint64_t>(tid < kVoxTile ? S.count[tid] : 0, S.scan, &total);
+        if (tid < kVoxTile) S.count[tid] = excl;  // now the triangle's offset inside the tile
         if (warp == 0) {
             const uint64_t b = sv_lookback(a.status, (uint32_t)tile, total, a.err);
             if (lane == 0) S.base = b;
         }
         __syncthreads();
         const uint64_t base = S.base;
-        for (uint32_t k = warp; k < kVoxTile; k += kVoxWarps) {
-            const uint64_t tri = t0 + k;
-            if (tri < a.n_tri) warp_triangle<kMode, true>(a, tri, base + S.count[k]);
-        }
         if (tid == 0 && tile == ntiles - 1) *a.d_total = base + total;
+        if (base < a.capacity) {
+            for (uint32_t k = warp; k < kVoxTile; k += kVoxWarps) {
+                const uint64_t tri = t0 + k;
+                const uint64_t o0 = S.count[k], o1 = k + 1 < (uint32_t)kVoxTile ? S.count[k + 1] : total;
+                if (o0 == o1) continue;  // also the triangles past the last
+                if (S.kept_at[k] == kNotKept) {
+                    warp_triangle<kMode, true>(a, S, tri, k, base + o0, 0);
+                    continue;
+                }
+                const auto& t = S.tri[k];
+                const uint32_t* kept = S.kept[warp] + S.kept_at[k];
+                for (uint64_t j = lane; j < o1 - o0; j += 32) {
+                    const uint32_t e = kept[j];
+                    uint64_t code;
+                    if constexpr (kMode == kVoxGL) code = gl_code(t, t.i0 + (int)(e & 0xFFFFu), t.j0 + (int)(e >> 16), G);
+                    else code = morton3((uint32_t)t.x0 + (e >> 20), (uint32_t)t.y0 + ((e >> 10) & 1023u), (uint32_t)t.z0 + (e & 1023u));
+                    if (base + o0 + j < a.capacity) a.codes[base + o0 + j] = code;
+                }
+            }
+        }
         __syncthreads();
     }
 }
 
 }  // namespace
 
-void launch_voxelize(const VoxArgs& a, int grid, cudaStream_t s) {
-    if (a.mode == kVoxGL) voxelize<kVoxGL><<<grid, kVoxThreads, 0, s>>>(a);
-    else voxelize<kVoxSAT><<<grid, kVoxThreads, 0, s>>>(a);
+void voxelize_configure() {
+    cudaFuncSetAttribute(voxelize<kVoxGL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(VoxSmem<kVoxGL>));
+    cudaFuncSetAttribute(voxelize<kVoxSAT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(VoxSmem<kVoxSAT>));
+}
+
+void launch_voxelize(const VoxArgs& args, int grid, cudaStream_t s) {
+    VoxArgs a = args;
+    for (int k = 0; k < 3; ++k) a.scale[k] = (double)((int64_t)1 << a.depth) / (a.aabb[3 + k] - a.aabb[k]);
+    if (a.mode == kVoxGL) voxelize<kVoxGL><<<grid, kVoxThreads, sizeof(VoxSmem<kVoxGL>), s>>>(a);
+    else voxelize<kVoxSAT><<<grid, kVoxThreads, sizeof(VoxSmem<kVoxSAT>), s>>>(a);
 }
 
 uint64_t voxelize_tiles(uint64_t n_tri) { return (n_tri + kVoxTile - 1) / kVoxTile; }
