@@ -10,18 +10,30 @@
 // of the bricks present: the bricks of a bin come out in ascending order by
 // walking the bitmap, with no sort. One
 // persistent grid takes work items from a device counter, in this order:
-//   COUNT(c, t)   tile t of chunk c: the chunk's bin histogram;
-//   SCATTER(c, t) tile t of chunk c, after all of c's COUNT tiles: fragments
-//                 to their bins (bin starts from the histogram, one global
-//                 reservation per bin and tile);
-//   LEAVES(c, g)  32 consecutive bins of chunk c, after all of c's SCATTER
-//                 tiles: per bin, OR every fragment's voxel bit into its
-//                 brick's mask, then emit the non-empty bricks in order.
+//   COUNT(c, t)   a run of tiles of chunk c: the chunk's bin histogram; the
+//                 last of c's COUNT items turns it into the bins' starts;
+//   SCATTER(c, t) the same run of tiles, after c's starts: fragments to their
+//                 bins (one global reservation per bin and tile). A tile is
+//                 put in bin order in shared memory first, so that a bin's
+//                 fragments leave as one run, while the next tile's are on
+//                 their way; a local code of up to 31 bits is a 4-byte word
+//                 from here on;
+//   LEAVES(c, g)  up to 32 consecutive bins of chunk c, after all of c's SCATTER
+//                 items: per bin, OR every fragment's voxel bit into its
+//                 brick's mask, then emit the non-empty bricks in order (the
+//                 next bin's first fragments on their way).
 // Small chunks (one bin) skip COUNT and SCATTER: their LEAVES item reads the
 // input. A CTA waits only on items taken before its own (taken by running
 // CTAs that wait only on earlier items still), so the waits end; each is
 // bounded anyway. Two small launches then pack the bricks of all items into
 // one ascending list: a scan of the items' brick counts and a copy.
+//
+// What bounds it: the chain of barriers and round trips of each tile and bin, at
+// 24 bytes of traffic per fragment (read for COUNT, read and 4 bytes written by
+// SCATTER, 4 read by LEAVES). 318M fragments, 256 chunks of 1024^3: 2.86 ms;
+// 6.39 when every fragment left its SCATTER tile as a scattered 8-byte store
+// and every voxel was ORed with an atomic, set or not; 3.47 without the loads
+// ahead and with a block scan per bin.
 
 #include "dagc_device.cuh"
 #include "dagc_kernels.h"
@@ -40,19 +52,25 @@ constexpr int kBitmapWords = kDirect / 32;
 static_assert(kBitmapWords <= kT, "one bitmap word per thread");
 
 struct ChunkSmem {
-    struct {
-        uint32_t tcnt[kMaxBins];   // this tile's fragments per bin (then its reservation base)
-        uint32_t start[kMaxBins];  // the chunk's bin starts (exclusive scan of its histogram)
-    } bins;
-    // One bin's leaf masks, by brick, as two 32-bit halves (native shared
-    // atomics); zero between bins (the emission clears what it reads), and a
-    // bitmap of the bricks present.
-    uint32_t masks[2 * kDirect];
-    uint32_t present[kBitmapWords];
+    union {
+        struct {
+            uint32_t cnt[kMaxBins];     // this tile's fragments per bin, then their offset in the tile
+            uint32_t delta[kMaxBins];   // output position - tile position, per bin
+            uint32_t stage[kChunkTile]; // the tile's codes in bin order
+        } tile;
+        struct {
+            // One bin's leaf masks, by brick, as two 32-bit halves (native
+            // shared atomics), and a bitmap of the bricks present; zero
+            // between bins (the emission clears the masks it reads, and the
+            // bitmap of the bin before: there are two, taken in turn).
+            uint32_t masks[2 * kDirect];
+            uint32_t present[2][kBitmapWords];
+        } bin;
+    };
     uint32_t bin_cnt[kChunkGroupBins];  // fragments of the LEAVES item's bins
     uint32_t scan[34];
     uint32_t item;
-    uint64_t running;
+    uint32_t flag;
 };
 
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
@@ -73,17 +91,17 @@ __device__ __forceinline__ void wait_counter(const uint32_t* counter, uint32_t t
     __syncthreads();
 }
 
-// The chunk of a COUNT / SCATTER tile (tile_off ascending, k + 1 entries).
-__device__ __forceinline__ uint32_t chunk_of_tile(const uint32_t* tile_off, uint32_t k, uint32_t t) {
-    uint32_t lo = 0, hi = k;  // tile_off[lo] <= t < tile_off[hi]
+// The chunk of a COUNT / SCATTER item (item_off ascending, k + 1 entries).
+__device__ __forceinline__ uint32_t chunk_of_item(const uint32_t* item_off, uint32_t k, uint32_t t) {
+    uint32_t lo = 0, hi = k;  // item_off[lo] <= t < item_off[hi]
     while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(tile_off + mid) <= t) lo = mid; else hi = mid;
+        if (__ldg(item_off + mid) <= t) lo = mid; else hi = mid;
     }
     return lo;
 }
 
-__global__ void __launch_bounds__(kT) chunk_leaves(ChunkArgs a) {
+__global__ void __launch_bounds__(kT, 2) chunk_leaves(ChunkArgs a) {
     pdl_prologue();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ChunkSmem& S = *reinterpret_cast<ChunkSmem*>(smem_raw);
@@ -93,91 +111,149 @@ __global__ void __launch_bounds__(kT) chunk_leaves(ChunkArgs a) {
     const int dbits = lb - a.bin_bits;                        // direct-mapped brick bits of a bin
     const uint32_t dsize = 1u << dbits;
     const uint64_t code_limit = 1ull << (3 * a.chunk_depth);
-    // The tile count comes from the device (tile_off[k]): a recorded graph
+    // The item count comes from the device (item_off[k]): a recorded graph
     // replayed for other chunk sizes still sees the current one.
-    const uint32_t tiles = __ldg(a.tile_off + a.k);
-    const uint32_t total = 2 * tiles + a.k * a.groups_per_chunk;
+    const uint32_t runs = __ldg(a.item_off + a.k);
+    const uint32_t total = 2 * runs + a.k * a.groups_per_chunk;
+    const uint64_t run_len = (uint64_t)a.run_tiles * kChunkTile;
+    const uint32_t lane = tid & 31, warp = tid >> 5;
+    constexpr uint32_t kWarps = kT / 32;
     bool bad = false;
-    for (uint32_t x = tid; x < 2u * kDirect; x += kT) S.masks[x] = 0;
+    bool clean = false;  // the bin arrays are zero (the tile arrays share their room)
     while (true) {
         if (tid == 0) S.item = atomicAdd(a.work, 1u);
         __syncthreads();
         const uint32_t item = S.item;
         __syncthreads();
         if (item >= total) break;
-        if (item < 2 * tiles) {
-            // ------------------------------------------- COUNT / SCATTER ----
-            const bool scatter = item >= tiles;
-            const uint32_t t = scatter ? item - tiles : item;
-            const uint32_t c = chunk_of_tile(a.tile_off, a.k, t);
-            const uint32_t tc = __ldg(a.tile_off + c + 1) - __ldg(a.tile_off + c);
-            const uint64_t c0 = __ldg(a.seg_offsets + c), c1 = __ldg(a.seg_offsets + c + 1);
-            const uint64_t f0 = c0 + (uint64_t)(t - __ldg(a.tile_off + c)) * kChunkTile;
-            const uint32_t fn = (uint32_t)min((uint64_t)kChunkTile, c1 - f0);
+        if (item < runs) {
+            // ----------------------------------------------------- COUNT ----
+            clean = false;
+            const uint32_t c = chunk_of_item(a.item_off, a.k, item);
+            const uint32_t first = __ldg(a.item_off + c), items = __ldg(a.item_off + c + 1) - first;
+            const uint64_t c1 = __ldg(a.seg_offsets + c + 1);
+            const uint64_t f0 = __ldg(a.seg_offsets + c) + (item - first) * run_len;
+            const uint64_t f1 = min(f0 + run_len, c1);
             uint32_t* hist = a.hist + (uint64_t)c * nb;
-            if (scatter) {
-                wait_counter(a.done + c, tc, a.err);
-                // Bin starts: exclusive scan of the chunk's histogram.
+            for (uint32_t b = tid; b < nb; b += kT) S.tile.cnt[b] = 0;
+            __syncthreads();
+            constexpr int kIlp = 8;
+            for (uint64_t i0 = f0 + tid; i0 < f1; i0 += kIlp * kT) {
+                uint64_t code[kIlp];
+#pragma unroll
+                for (int q = 0; q < kIlp; ++q) code[q] = i0 + q * kT < f1 ? __ldg(a.frags + i0 + q * kT) : 0ull;
+#pragma unroll
+                for (int q = 0; q < kIlp; ++q) {
+                    if (i0 + q * kT >= f1) continue;
+                    if (code[q] >= code_limit) bad = true;
+                    // (A code out of range goes where SCATTER puts it.)
+                    atomicAdd(&S.tile.cnt[(uint32_t)(code[q] & (code_limit - 1)) >> (6 + dbits)], 1u);
+                }
+            }
+            __syncthreads();
+            for (uint32_t b = tid; b < nb; b += kT) {
+                const uint32_t x = S.tile.cnt[b];
+                if (x) atomicAdd(hist + b, x);
+            }
+            __threadfence();  // every thread's counts land before the item is marked done
+            __syncthreads();
+            if (tid == 0) {
+                __threadfence();
+                S.flag = atomicAdd(a.done + c, 1u) == items - 1;
+                __threadfence();
+            }
+            __syncthreads();
+            if (S.flag) {
+                // The chunk's last COUNT item: bin starts from the histogram.
                 constexpr int kPer = kMaxBins / kT;
                 uint32_t h[kPer], sum = 0, tot;
 #pragma unroll
                 for (int q = 0; q < kPer; ++q) {
                     const uint32_t b = tid * kPer + q;
-                    h[q] = b < nb ? hist[b] : 0u;
+                    h[q] = b < nb ? ld_relaxed(hist + b) : 0u;
                     sum += h[q];
                 }
                 uint32_t run = block_exclusive_sum<uint32_t>(sum, S.scan, &tot);
 #pragma unroll
                 for (int q = 0; q < kPer; ++q) {
-                    S.bins.start[tid * kPer + q] = run;
+                    const uint32_t b = tid * kPer + q;
+                    if (b < nb) st_relaxed(a.cursor + (uint64_t)c * nb + b, run);
                     run += h[q];
                 }
-            }
-            for (uint32_t b = tid; b < nb; b += kT) S.bins.tcnt[b] = 0;
-            __syncthreads();
-            uint32_t br[kPerThread];  // bin << 16 | rank of the fragment among the tile's of its bin
-#pragma unroll
-            for (int q = 0; q < kPerThread; ++q) {
-                const uint32_t i = q * kT + tid;
-                br[q] = 0xFFFFFFFFu;
-                if (i < fn) {
-                    const uint64_t code = __ldg(a.frags + f0 + i);
-                    if (code >= code_limit) bad = true;
-                    uint32_t bin = (uint32_t)((code >> 6) >> dbits);
-                    bin = bin < nb ? bin : nb - 1;
-                    const uint32_t r = atomicAdd(&S.bins.tcnt[bin], 1u);
-                    br[q] = bin << 16 | r;
-                }
-            }
-            __syncthreads();
-            if (!scatter) {
-                for (uint32_t b = tid; b < nb; b += kT) {
-                    const uint32_t x = S.bins.tcnt[b];
-                    if (x) atomicAdd(hist + b, x);
-                }
-                __threadfence();  // every thread's counts land before the tile is marked done
+                __threadfence();
                 __syncthreads();
                 if (tid == 0) {
                     __threadfence();
-                    atomicAdd(a.done + c, 1u);
+                    atomicAdd(a.done + 2 * a.k + c, 1u);
                 }
-                continue;
             }
-            // One reservation per bin and tile.
-            for (uint32_t b = tid; b < nb; b += kT) {
-                const uint32_t x = S.bins.tcnt[b];
-                if (x) S.bins.tcnt[b] = atomicAdd(a.cursor + (uint64_t)c * nb + b, x);
-            }
-            __syncthreads();
+            continue;
+        }
+        if (item < 2 * runs) {
+            // --------------------------------------------------- SCATTER ----
+            clean = false;
+            const uint32_t t = item - runs;
+            const uint32_t c = chunk_of_item(a.item_off, a.k, t);
+            const uint64_t c0 = __ldg(a.seg_offsets + c), c1 = __ldg(a.seg_offsets + c + 1);
+            const uint64_t f0 = c0 + (t - __ldg(a.item_off + c)) * run_len;
+            const uint64_t f1 = min(f0 + run_len, c1);
+            uint32_t* out = a.scratch + c0;
+            const uint32_t room = (uint32_t)(c1 - c0);
+            const int bin_shift = 6 + dbits;
+            const uint32_t code_mask = (uint32_t)(code_limit - 1);  // the low 32 bits hold a code whole (3 * chunk_depth <= 31)
+            uint32_t code[kPerThread], rank[kPerThread];
+            uint32_t fn = (uint32_t)min((uint64_t)kChunkTile, f1 - f0);
 #pragma unroll
-            for (int q = 0; q < kPerThread; ++q) {
-                if (br[q] == 0xFFFFFFFFu) continue;
-                const uint32_t i = q * kT + tid, bin = br[q] >> 16;
-                const uint64_t dst = c0 + S.bins.start[bin] + S.bins.tcnt[bin] + (br[q] & 0xFFFFu);
-                if (dst < c1) a.scratch[dst] = __ldg(a.frags + f0 + i);
-                else bad = true;  // only after a timed-out wait
+            for (int q = 0; q < kPerThread; ++q)
+                code[q] = q * kT + tid < fn ? (uint32_t)__ldcs(a.frags + f0 + q * kT + tid) & code_mask : 0u;
+            for (uint32_t b = tid; b < nb; b += kT) S.tile.cnt[b] = 0;
+            wait_counter(a.done + 2 * a.k + c, 1u, a.err);  // the bins' starts; also orders the zeros above
+            for (uint64_t f = f0; f < f1; f += kChunkTile) {
+#pragma unroll
+                for (int q = 0; q < kPerThread; ++q)
+                    if (q * kT + tid < fn) rank[q] = atomicAdd(&S.tile.cnt[code[q] >> bin_shift], 1u);
+                __syncthreads();
+                constexpr int kPer = kMaxBins / kT;
+                uint32_t n[kPer], g[kPer], sum = 0, tot;
+#pragma unroll
+                for (int q = 0; q < kPer; ++q) {
+                    const uint32_t b = tid * kPer + q;
+                    n[q] = b < nb ? S.tile.cnt[b] : 0u;
+                    g[q] = n[q] ? atomicAdd(a.cursor + (uint64_t)c * nb + b, n[q]) : 0u;
+                    sum += n[q];
+                }
+                uint32_t run = block_exclusive_sum<uint32_t>(sum, S.scan, &tot);
+#pragma unroll
+                for (int q = 0; q < kPer; ++q) {
+                    const uint32_t b = tid * kPer + q;
+                    if (b < nb) {
+                        S.tile.cnt[b] = run;
+                        S.tile.delta[b] = g[q] - run;
+                    }
+                    run += n[q];
+                }
+                __syncthreads();
+#pragma unroll
+                for (int q = 0; q < kPerThread; ++q)
+                    if (q * kT + tid < fn) S.tile.stage[S.tile.cnt[code[q] >> bin_shift] + rank[q]] = code[q];
+                __syncthreads();
+                const uint32_t m = fn;
+                const uint64_t next = f + kChunkTile;
+                fn = next < f1 ? (uint32_t)min((uint64_t)kChunkTile, f1 - next) : 0u;
+#pragma unroll
+                for (int q = 0; q < kPerThread; ++q)
+                    code[q] = q * kT + tid < fn ? (uint32_t)__ldcs(a.frags + next + q * kT + tid) & code_mask : 0u;
+                for (uint32_t b = tid; b < nb; b += kT) S.tile.cnt[b] = 0;
+#pragma unroll 4
+                for (uint32_t q = tid; q < m; q += kT) {
+                    const uint32_t x = S.tile.stage[q];
+                    const uint32_t dst = S.tile.delta[x >> bin_shift] + q;
+                    if (dst < room) out[dst] = x;
+                    else bad = true;  // only after a timed-out wait
+                }
+                __syncthreads();
             }
-            __threadfence();  // every thread's fragments land before the tile is marked done
+            __threadfence();  // every thread's fragments land before the item is marked done
             __syncthreads();
             if (tid == 0) {
                 __threadfence();
@@ -186,80 +262,128 @@ __global__ void __launch_bounds__(kT) chunk_leaves(ChunkArgs a) {
             continue;
         }
         // --------------------------------------------------------- LEAVES ----
-        const uint32_t gi = item - 2 * tiles;
+        if (!clean) {
+            for (uint32_t x = tid; x < 2u * kDirect; x += kT) S.bin.masks[x] = 0;
+            if (tid < 2u * kBitmapWords) (&S.bin.present[0][0])[tid] = 0;
+            clean = true;
+        }
+        const uint32_t gi = item - 2 * runs;
         const uint32_t c = gi / a.groups_per_chunk, g = gi % a.groups_per_chunk;
         const uint64_t c0 = __ldg(a.seg_offsets + c), c1 = __ldg(a.seg_offsets + c + 1);
-        const uint32_t b0 = g * kChunkGroupBins, b1 = min(nb, b0 + kChunkGroupBins);
+        const uint32_t b0 = g * a.group_bins, b1 = min(nb, b0 + a.group_bins);
         const uint64_t pbase = __ldg(a.seg_code + c) << (a.seg_shift - 6);  // global brick of local brick 0
         const uint32_t* hist = a.hist + (uint64_t)c * nb;
-        const uint64_t* src = nb > 1 ? a.scratch : a.frags;
         uint64_t gstart = c0;  // fragment offset of bin b0 (and of the group's bricks)
         if (nb > 1) {
-            const uint32_t tc = __ldg(a.tile_off + c + 1) - __ldg(a.tile_off + c);
-            if (tc) wait_counter(a.done + a.k + c, tc, a.err);
-            uint32_t part = 0;
-            for (uint32_t b = tid; b < b0; b += kT) part += hist[b];
-            uint32_t tot;
-            block_exclusive_sum<uint32_t>(part, S.scan, &tot);
-            gstart += tot;
+            const uint32_t items = __ldg(a.item_off + c + 1) - __ldg(a.item_off + c);
+            if (items) wait_counter(a.done + a.k + c, items, a.err);
+            if (tid < b1 - b0) S.bin_cnt[tid] = ld_relaxed(hist + b0 + tid);
+            // A bin's cursor ends at its start plus its count.
+            if (items) gstart += ld_relaxed(a.cursor + (uint64_t)c * nb + b0) - ld_relaxed(hist + b0);
         }
-        if (tid == 0) S.running = 0;
-        if (nb > 1 && tid < b1 - b0) S.bin_cnt[tid] = hist[b0 + tid];
         __syncthreads();
+        // The first kIlp fragments per thread of a bin are fetched while the
+        // bin before is emitted.
+        constexpr int kIlp = 8;
+        uint32_t code[kIlp];
+        auto bin_count = [&](uint32_t b) -> uint64_t { return nb > 1 ? (uint64_t)S.bin_cnt[b - b0] : c1 - c0; };
+        auto next_bin = [&](uint32_t b) -> uint32_t {  // the first nonempty bin from b on
+            while (b < b1 && bin_count(b) == 0) ++b;
+            return b;
+        };
+        auto fetch = [&](uint64_t from, uint64_t i0, uint64_t cnt) {
+#pragma unroll
+            for (int u = 0; u < kIlp; ++u) {
+                const uint64_t i = i0 + (uint64_t)u * kT;
+                code[u] = 0;
+                if (i >= cnt) continue;
+                if (nb > 1) {
+                    code[u] = __ldcg(a.scratch + from + i);
+                } else {
+                    const uint64_t full = __ldg(a.frags + from + i);
+                    if (full >= code_limit) bad = true;
+                    code[u] = (uint32_t)full;
+                }
+            }
+        };
+        uint32_t running = 0, turn = 0;
         uint64_t fstart = gstart;
-        for (uint32_t b = b0; b < b1; ++b) {
-            const uint64_t cnt = nb > 1 ? S.bin_cnt[b - b0] : c1 - c0;
-            if (cnt == 0) continue;
-            if (tid < (uint32_t)kBitmapWords) S.present[tid] = 0;
-            __syncthreads();
-            // Four fragments per thread in flight, then their updates: the
-            // voxel bit goes to its brick's low or high half; the first bit
-            // of a half marks the brick present.
-            for (uint64_t i0 = tid; i0 < cnt; i0 += 4 * kT) {
-                uint64_t code[4];
-                bool in[4];
+        uint32_t b = next_bin(b0);
+        uint64_t cnt = b < b1 ? bin_count(b) : 0;
+        if (fstart + cnt > c1) { bad = true; b = b1; }  // only after a timed-out wait
+        if (b < b1) fetch(fstart, tid, cnt);
+        while (b < b1) {
+            // The voxel bit goes to its brick's low or high half where it is
+            // not set yet (voxels repeat); the first bit of a half marks the
+            // brick present.
+            uint32_t* present = S.bin.present[turn];
+            for (uint64_t i0 = tid;;) {
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const uint64_t i = i0 + (uint64_t)u * kT;
-                    in[u] = i < cnt;
-                    code[u] = in[u] ? src[fstart + i] : 0ull;
+                for (int u = 0; u < kIlp; ++u) {
+                    if (i0 + (uint64_t)u * kT >= cnt) continue;
+                    const uint32_t e = (code[u] >> 6) & (dsize - 1);
+                    uint32_t* half = &S.bin.masks[2 * e + ((code[u] >> 5) & 1u)];
+                    const uint32_t bit = 1u << (code[u] & 31u);
+                    const uint32_t seen = *reinterpret_cast<volatile uint32_t*>(half);
+                    if (seen & bit) continue;
+                    if (atomicOr(half, bit) == 0) atomicOr(&present[e >> 5], 1u << (e & 31));
                 }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (!in[u]) continue;
-                    if (nb == 1 && code[u] >= code_limit) bad = true;
-                    const uint32_t e = (uint32_t)(code[u] >> 6) & (dsize - 1);
-                    const uint32_t v = (uint32_t)code[u] & 63u;
-                    const uint32_t old = atomicOr(&S.masks[2 * e + (v >> 5)], 1u << (v & 31));
-                    if (old == 0) atomicOr(&S.present[e >> 5], 1u << (e & 31));
-                }
+                i0 += kIlp * kT;
+                if (i0 >= cnt) break;
+                fetch(fstart, i0, cnt);
             }
+            const uint32_t bin = b;
             fstart += cnt;
+            b = next_bin(b + 1);
+            cnt = b < b1 ? bin_count(b) : 0;
+            if (fstart + cnt > c1) { bad = true; b = b1; }
+            if (b < b1) fetch(fstart, tid, cnt);
             __syncthreads();
-            // The bin's bricks in order: thread t owns bitmap word t (bricks
-            // 32t .. 32t + 31); a block scan of the words' counts gives the
-            // output positions. Every mask read is cleared for the next bin.
-            const uint32_t word = tid < (uint32_t)kBitmapWords ? S.present[tid] : 0u;
-            uint32_t tot;
-            uint32_t pos = block_exclusive_sum<uint32_t>((uint32_t)__popc(word), S.scan, &tot);
-            const uint64_t out0 = gstart + S.running;
-            for (uint32_t w = word; w; w &= w - 1) {
-                const uint32_t e = tid * 32 + (__ffs(w) - 1);
-                const uint64_t m = (uint64_t)S.masks[2 * e] | (uint64_t)S.masks[2 * e + 1] << 32;
-                S.masks[2 * e] = 0;
-                S.masks[2 * e + 1] = 0;
-                const uint64_t o = out0 + pos++;
-                if (o < c1) {
-                    a.stage_parent[o] = pbase | ((uint64_t)b << dbits) | e;
-                    a.stage_mask[o] = m;
-                }
+            // The bin's bricks in order: warp w emits bitmap words [16w, 16w +
+            // 16), a lane per brick. Every warp counts the bricks before its
+            // words, and all of them, from the bitmap.
+            constexpr uint32_t kWordsPerWarp = kBitmapWords / kWarps;
+            static_assert(kWordsPerWarp <= 32, "a lane per word of a warp");
+            const uint32_t w0 = warp * kWordsPerWarp;
+            const uint32_t own = lane < kWordsPerWarp ? present[w0 + lane] : 0u;
+            uint32_t before = 0, all = 0;
+#pragma unroll
+            for (uint32_t x = lane; x < (uint32_t)kBitmapWords; x += 32) {
+                const uint32_t n = __popc(present[x]);
+                all += n;
+                if (x < w0) before += n;
             }
+            before = __reduce_add_sync(0xFFFFFFFFu, before);
+            all = __reduce_add_sync(0xFFFFFFFFu, all);
+            uint64_t out0 = gstart + running + before;
+            for (uint32_t words = __ballot_sync(0xFFFFFFFFu, own != 0); words; words &= words - 1) {
+                const uint32_t w = __ffs(words) - 1;
+                const uint32_t bits = __shfl_sync(0xFFFFFFFFu, own, w);
+                if ((bits >> lane) & 1u) {
+                    const uint32_t e = (w0 + w) * 32 + lane;
+                    const uint64_t m = (uint64_t)S.bin.masks[2 * e] | (uint64_t)S.bin.masks[2 * e + 1] << 32;
+                    S.bin.masks[2 * e] = 0;
+                    S.bin.masks[2 * e + 1] = 0;
+                    const uint64_t o = out0 + __popc(bits & lanemask_lt());
+                    if (o < c1) {
+                        a.stage_parent[o] = pbase | ((uint64_t)bin << dbits) | e;
+                        a.stage_mask[o] = m;
+                    }
+                }
+                out0 += __popc(bits);
+            }
+            // The other bitmap, of the bin before, is no longer read.
+            turn ^= 1u;
+            if (tid < (uint32_t)kBitmapWords) S.bin.present[turn][tid] = 0;
+            running += all;
             __syncthreads();
-            if (tid == 0) S.running += tot;
+        }
+        if (running) {
+            if (tid < (uint32_t)kBitmapWords) S.bin.present[turn ^ 1u][tid] = 0;  // the last bin's
             __syncthreads();
         }
         if (tid == 0) {
-            a.group_bricks[gi] = (uint32_t)S.running;
+            a.group_bricks[gi] = running;
             a.group_src[gi] = gstart;
         }
     }
@@ -290,28 +414,41 @@ __global__ void __launch_bounds__(1024) chunk_scan(ChunkArgs a) {
     }
 }
 
-// Packs the items' bricks into the ascending list: every thread moves a run
-// of consecutive output bricks (balanced whatever the items' sizes), finding
-// the item of its first brick by binary search over the items' output
-// starts and walking forward from there.
+// Packs the items' bricks into the ascending list: a CTA moves kCopyTile
+// consecutive output bricks (balanced whatever the items' sizes), each row of
+// threads consecutive ones. The items of the tile are those from the last that
+// starts at or before its first brick on; a thread follows its bricks through
+// them. (184 us for 13M bricks when each thread moved a run of eight.)
+constexpr int kCopyThreads = 256;
 constexpr int kCopyPer = 8;
-__global__ void __launch_bounds__(256) chunk_copy(ChunkArgs a) {
+constexpr int kCopyTile = kCopyThreads * kCopyPer;
+__global__ void __launch_bounds__(kCopyThreads) chunk_copy(ChunkArgs a) {
     pdl_prologue();
     const uint32_t g = a.k * a.groups_per_chunk;
     const uint64_t total = *a.d_out_n;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x * kCopyPer;
-    for (uint64_t j0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * kCopyPer; j0 < total; j0 += stride) {
-        uint32_t lo = 0, hi = g;  // group_dst[lo] <= j0 < group_dst[hi] (ascending)
+    for (uint64_t t0 = (uint64_t)blockIdx.x * kCopyTile; t0 < total; t0 += (uint64_t)gridDim.x * kCopyTile) {
+        uint32_t lo = 0, hi = g;  // group_dst[lo] <= t0 < group_dst[hi] (ascending)
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) >> 1;
-            if (a.group_dst[mid] <= j0) lo = mid; else hi = mid;
+            if (__ldg(a.group_dst + mid) <= t0) lo = mid; else hi = mid;
         }
         uint32_t w = lo;
-        for (uint64_t j = j0; j < j0 + kCopyPer && j < total; ++j) {
-            while (w + 1 < g && a.group_dst[w + 1] <= j) ++w;
-            const uint64_t src = a.group_src[w] + (j - a.group_dst[w]);
-            a.parents[j] = a.stage_parent[src];
-            a.leaves[j] = a.stage_mask[src];
+        uint64_t p[kCopyPer], m[kCopyPer];
+#pragma unroll
+        for (int q = 0; q < kCopyPer; ++q) {
+            const uint64_t j = t0 + q * kCopyThreads + threadIdx.x;
+            if (j >= total) continue;
+            while (w + 1 < g && __ldg(a.group_dst + w + 1) <= j) ++w;
+            const uint64_t src = __ldg(a.group_src + w) + (j - __ldg(a.group_dst + w));
+            p[q] = a.stage_parent[src];
+            m[q] = a.stage_mask[src];
+        }
+#pragma unroll
+        for (int q = 0; q < kCopyPer; ++q) {
+            const uint64_t j = t0 + q * kCopyThreads + threadIdx.x;
+            if (j >= total) continue;
+            a.parents[j] = p[q];
+            a.leaves[j] = m[q];
         }
     }
 }
@@ -327,20 +464,36 @@ void chunk_configure(int sms) {
     g_chunk_ctas = (occ > 0 ? occ : 1) * (sms > 0 ? sms : 152);
 }
 
+int chunk_run_tiles(uint64_t n) {
+    // Runs of up to four tiles (the next tile's fragments are fetched while one
+    // is written), but at least two per resident CTA.
+    const uint64_t runs = n / ((uint64_t)kChunkTile * 2 * (g_chunk_ctas > 0 ? g_chunk_ctas : 1));
+    return (int)(runs < 1 ? 1 : (runs < 4 ? runs : 4));
+}
+
+uint32_t chunk_group_bins(uint64_t k, uint32_t bins) {
+    // Enough items that the fullest (an item's bins come one after another) is
+    // a small part of a CTA's share: 16 per resident CTA where the bins allow
+    // (150 chunks of 256^3, 32 bins each: 119 us with one bin per item, 185
+    // with all of a chunk's).
+    const uint64_t per = k * bins / (16ull * (g_chunk_ctas > 0 ? g_chunk_ctas : 1));
+    return (uint32_t)(per < 1 ? 1 : (per < kChunkGroupBins ? per : kChunkGroupBins));
+}
+
 int chunk_bin_bits(int chunk_depth) {
     const int lb = 3 * chunk_depth - 6;
     return lb > kChunkDirectBits ? lb - kChunkDirectBits : 0;
 }
 
 void launch_chunk_leaves(const ChunkArgs& a, cudaStream_t s) {
-    const uint64_t items = 2ull * a.tiles + (uint64_t)a.k * a.groups_per_chunk;
+    const uint64_t items = 2ull * a.items + (uint64_t)a.k * a.groups_per_chunk;
     const int grid = (int)(items < (uint64_t)g_chunk_ctas ? (items ? items : 1) : g_chunk_ctas);
     launch_pdl(chunk_leaves, dim3(grid), dim3(kT), sizeof(ChunkSmem), s, a);
     launch_pdl(chunk_scan, dim3(1), dim3(1024), 0, s, a);
     // The brick total is on the device: the grid covers the bound and extra
-    // threads leave at once.
-    const uint64_t blocks = (a.out_capacity + 256ull * kCopyPer - 1) / (256ull * kCopyPer);
-    launch_pdl(chunk_copy, dim3((unsigned)(blocks < 8192 ? (blocks ? blocks : 1) : 8192)), dim3(256), 0, s, a);
+    // CTAs leave at once.
+    const uint64_t blocks = (a.out_capacity + kCopyTile - 1) / kCopyTile;
+    launch_pdl(chunk_copy, dim3((unsigned)(blocks < 4096 ? (blocks ? blocks : 1) : 4096)), dim3(kCopyThreads), 0, s, a);
 }
 
 }  // namespace dagc

@@ -353,7 +353,7 @@ struct dagc_context_t {
     bool use_dedup = true;
     int group_mode = 1;  // DAGC_OPT_GROUP
     int batch_path = 1;  // DAGC_OPT_BATCH_PATH
-    std::vector<uint32_t> ck_tile_host;  // chunk path: first tile of each chunk (host copy for the upload)
+    std::vector<uint32_t> ck_item_host;  // chunk path: first item of each chunk (host copy for the upload)
     bool pdl = false;    // DAGC_OPT_PDL
     uint64_t dedup_unique_limit = kDedupMaxUnique;  // lowered only to exercise the rerun
     void* table = nullptr;
@@ -815,13 +815,13 @@ struct CreateLayout {
     size_t o_islot = 0, o_ukey = 0, o_uslot = 0;
     size_t o_bcnt = 0, o_bent = 0;
     // Persistent per-chunk leaves (batched form): zeroed chunk state
-    // (histograms, cursors, done counters, item counter), tile offsets, the
+    // (histograms, cursors, done counters, item counter), item offsets, the
     // mask stage and per-item brick counts / offsets.
     // Direct-mapped leaves: block counters (zeroed) and the occupied blocks.
     size_t o_dcount = 0, o_dsv = 0, o_dlist = 0;
-    uint32_t ck_bins = 0, ck_groups = 0;
+    uint32_t ck_bins = 0, ck_group_bins = 1, ck_groups = 0;
     size_t o_ck_state = 0, ck_state_bytes = 0, o_ck_hist = 0, o_ck_cursor = 0, o_ck_done = 0, o_ck_work = 0;
-    size_t o_ck_tile = 0, o_ck_mask = 0, o_ck_gb = 0, o_ck_gs = 0, o_ck_gd = 0;
+    size_t o_ck_item = 0, o_ck_mask = 0, o_ck_gb = 0, o_ck_gs = 0, o_ck_gd = 0;
     CreateLayout(uint64_t n, int depth, uint32_t k_batch, bool use_dedup, uint64_t unique_limit = kDedupMaxUnique,
                  bool grouping = false, int chunk_depth = 0, bool direct_table = false, bool direct = false) {
         const int nl = depth - 2;
@@ -889,14 +889,15 @@ struct CreateLayout {
         o_seg_code = L.take<uint64_t>(k_batch);
         if (chunk_depth > 0 && k_batch) {
             ck_bins = 1u << chunk_bin_bits(chunk_depth);
-            ck_groups = (ck_bins + kChunkGroupBins - 1) / kChunkGroupBins;
+            ck_group_bins = chunk_group_bins(k_batch, ck_bins);
+            ck_groups = (ck_bins + ck_group_bins - 1) / ck_group_bins;
             o_ck_hist = L.take<uint32_t>((uint64_t)k_batch * ck_bins);
             o_ck_state = o_ck_hist;
             o_ck_cursor = L.take<uint32_t>((uint64_t)k_batch * ck_bins);
-            o_ck_done = L.take<uint32_t>(2ull * k_batch);
+            o_ck_done = L.take<uint32_t>(3ull * k_batch);
             o_ck_work = L.take<uint32_t>(1);
             ck_state_bytes = L.off - o_ck_state;
-            o_ck_tile = L.take<uint32_t>(k_batch + 1ull);
+            o_ck_item = L.take<uint32_t>(k_batch + 1ull);
             o_ck_mask = L.take<uint64_t>(n);
             o_ck_gb = L.take<uint32_t>((uint64_t)k_batch * ck_groups);
             o_ck_gs = L.take<uint64_t>((uint64_t)k_batch * ck_groups);
@@ -1029,18 +1030,19 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
                                        cudaMemcpyHostToDevice, s));
         DAGC_CUDA(ctx, cudaMemcpyAsync(P64(Lo.o_seg_code), batch->h_morton, batch->k * 8, cudaMemcpyHostToDevice, s));
     }
-    // Chunk path: the first COUNT/SCATTER tile of every chunk (none when a
+    // Chunk path: the first COUNT / SCATTER item of every chunk (none when a
     // chunk is a single bin).
-    uint32_t ck_tiles = 0;
+    uint32_t ck_items = 0;
+    const uint64_t ck_run = chunk_run_tiles(n);
     if (chunk_path) {
-        ctx->ck_tile_host.assign(batch->k + 1, 0);
+        ctx->ck_item_host.assign(batch->k + 1, 0);
         for (uint32_t c = 0; c < batch->k; ++c) {
             const uint64_t nc = batch->h_offsets[c + 1] - batch->h_offsets[c];
-            const uint64_t t = Lo.ck_bins > 1 ? (nc + kChunkTile - 1) / kChunkTile : 0;
-            ctx->ck_tile_host[c + 1] = ctx->ck_tile_host[c] + (uint32_t)t;
+            const uint64_t t = Lo.ck_bins > 1 ? (nc + ck_run * kChunkTile - 1) / (ck_run * kChunkTile) : 0;
+            ctx->ck_item_host[c + 1] = ctx->ck_item_host[c] + (uint32_t)t;
         }
-        ck_tiles = ctx->ck_tile_host[batch->k];
-        DAGC_CUDA(ctx, cudaMemcpyAsync(P32(Lo.o_ck_tile), ctx->ck_tile_host.data(), (batch->k + 1) * 4,
+        ck_items = ctx->ck_item_host[batch->k];
+        DAGC_CUDA(ctx, cudaMemcpyAsync(P32(Lo.o_ck_item), ctx->ck_item_host.data(), (batch->k + 1) * 4,
                                        cudaMemcpyHostToDevice, s));
     }
 
@@ -1073,14 +1075,16 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
             ca.chunk_depth = batch->chunk_depth;
             ca.seg_shift = seg_shift;
             ca.bin_bits = chunk_bin_bits(batch->chunk_depth);
-            ca.tile_off = P32(Lo.o_ck_tile);
-            ca.tiles = ck_tiles;
+            ca.run_tiles = (uint32_t)ck_run;
+            ca.item_off = P32(Lo.o_ck_item);
+            ca.items = ck_items;
+            ca.group_bins = Lo.ck_group_bins;
             ca.groups_per_chunk = Lo.ck_groups;
             ca.hist = P32(Lo.o_ck_hist);
             ca.cursor = P32(Lo.o_ck_cursor);
             ca.done = P32(Lo.o_ck_done);
             ca.work = P32(Lo.o_ck_work);
-            ca.scratch = P64(Lo.o_B);
+            ca.scratch = P32(Lo.o_B);
             ca.stage_parent = P64(Lo.o_A);
             ca.stage_mask = P64(Lo.o_ck_mask);
             ca.group_bricks = P32(Lo.o_ck_gb);
@@ -1445,10 +1449,10 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
         set_pending_bytes(ctx, DAGC_STAGE_GROUP_SCATTER, (8 + entry) * n);
         set_pending_bytes(ctx, DAGC_STAGE_GROUP_AGGREGATE, entry * n + 20 * p0);
         set_pending_bytes(ctx, DAGC_STAGE_GROUP, direct_table ? 32 * p0 + 4 * direct_blocks(depth) : 60 * p0);
-        // Chunk leaves: COUNT reads the fragments, SCATTER reads and writes
-        // them, LEAVES reads them and writes 16 bytes per brick, the pack
-        // moves those bricks once more.
-        set_pending_bytes(ctx, DAGC_STAGE_CHUNK_LEAVES, (Lo.ck_bins > 1 ? 32 : 8) * n + 48 * p0);
+        // Chunk leaves: COUNT reads the fragments, SCATTER reads them and
+        // writes 4 bytes each, LEAVES reads those and writes 16 bytes per
+        // brick, the pack moves those bricks once more.
+        set_pending_bytes(ctx, DAGC_STAGE_CHUNK_LEAVES, (Lo.ck_bins > 1 ? 24 : 8) * n + 48 * p0);
         set_pending_bytes(ctx, DAGC_STAGE_LEAF_DEDUP, 216 * p0 + 8 * lv);
         uint64_t lb = 0;
         for (int l = 0; l < nl; ++l) {

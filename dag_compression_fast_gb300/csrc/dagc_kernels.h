@@ -232,28 +232,31 @@ int launch_direct_compact(const DirectArgs& a, cudaStream_t s);
 // A chunk's local bricks (local code >> 6) fall in 2^bin_bits bins of at most
 // 2^kChunkDirectBits bricks, direct-mapped in shared memory.
 constexpr int kChunkThreads = 512;
-constexpr int kChunkTile = 8192;       // fragments per COUNT / SCATTER item
+constexpr int kChunkTile = 8192;       // fragments per tile (a COUNT / SCATTER item is a run of tiles)
 constexpr int kChunkDirectBits = 13;   // bricks of one bin
-constexpr int kChunkMaxBinBits = 12;   // bins per chunk (chunk depth <= 10)
-constexpr int kChunkGroupBins = 32;    // bins per LEAVES item
+constexpr int kChunkMaxBinBits = 11;   // bins per chunk (chunk depth <= 10)
+constexpr int kChunkGroupBins = 32;    // most bins per LEAVES item
 struct ChunkArgs {
     const uint64_t* frags;                          // chunk-local codes, chunks back to back
     const uint64_t* seg_offsets; const uint64_t* seg_code;  // k + 1 offsets, k Morton indices (device)
     uint32_t k; int chunk_depth; int seg_shift;     // seg_shift = 3 * chunk_depth
     int bin_bits;                                   // chunk_bin_bits(chunk_depth)
-    const uint32_t* tile_off;                       // k + 1: first COUNT/SCATTER tile of each chunk (device)
-    uint32_t tiles;                                 // tile_off[k] (host copy, for the grid only)
-    uint32_t groups_per_chunk;                      // LEAVES items per chunk
-    uint32_t* hist; uint32_t* cursor;               // k << bin_bits each, zero
-    uint32_t* done;                                 // 2k: COUNT tiles done, SCATTER tiles done (zero)
+    uint32_t run_tiles;                             // tiles per COUNT / SCATTER item (chunk_run_tiles)
+    const uint32_t* item_off;                       // k + 1: first COUNT (and SCATTER) item of each chunk (device)
+    uint32_t items;                                 // item_off[k] (host copy, for the grid only)
+    uint32_t group_bins, groups_per_chunk;          // bins per LEAVES item (chunk_group_bins), items per chunk
+    uint32_t* hist; uint32_t* cursor;               // k << bin_bits each, hist zero
+    uint32_t* done;                                 // 3k: COUNT items done, SCATTER items done, starts known (zero)
     uint32_t* work;                                 // item counter (zero)
-    uint64_t* scratch;                              // fragments by bin (n)
+    uint32_t* scratch;                              // fragments' local codes by bin (n)
     uint64_t* stage_parent; uint64_t* stage_mask;   // n each: each item's bricks at its fragment offset
     uint32_t* group_bricks; uint64_t* group_src; uint32_t* group_dst;  // per LEAVES item
     uint64_t* parents; uint64_t* leaves; uint64_t out_capacity; uint64_t* d_out_n;
     uint32_t* err;
 };
 void chunk_configure(int sms);
+int chunk_run_tiles(uint64_t n);
+uint32_t chunk_group_bins(uint64_t k, uint32_t bins);
 int chunk_bin_bits(int chunk_depth);  // -> bins of at most 2^kChunkDirectBits bricks
 void launch_chunk_leaves(const ChunkArgs& a, cudaStream_t s);  // three launches
 
