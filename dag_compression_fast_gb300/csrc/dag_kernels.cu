@@ -192,7 +192,7 @@ __global__ void leaf_fixup(LeafBuildArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Extract one level + node hash. Child codes are unique and sorted, so a
+// Extract one level + node hash (the radix form). Child codes are unique and sorted, so a
 // parent owns at most 8 consecutive children. Each step is one round trip
 // for the whole tile rather than a chain per thread: the tile's child codes
 // and ids, then all their hashes (gathered at once into shared memory); the
@@ -219,27 +219,7 @@ __global__ void __launch_bounds__(kT, 3) extract_level(ExtractArgs a) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint64_t n = load_count(a.d_n, a.n_bound);
     const uint32_t ntiles = scan_tiles(n);
-    // Fused insert (node levels of the hash-set form): table and buckets sized
-    // by the child count n, which bounds the node count.
-    const DedupArgs& dd = a.dedup;
-    bool fuse = a.fuse_insert != 0 && n <= kFuseInsertMax;
-    uint64_t tslots = 0;
-    int shift = 64;
-    uint32_t nb = 0;
-    if (fuse) {
-        tslots = table_size_for(n, false);
-        nb = topbit_buckets(n, &shift);
-        if (tslots > dd.table_cap || n > dd.item_cap || (uint64_t)nb * kDedupTopBitCap > dd.bucket_area) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) { atomicOr(a.err, kErrFallback); dd.state->nbuckets = 0; }
-            fuse = false;
-        } else if (blockIdx.x == 0 && threadIdx.x == 0) {
-            dd.state->nbuckets = nb;
-            dd.state->inserted = 1u;
-        }
-    }
-    const bool read_first = n > kDedupClaimFirstMax;
-    uint32_t* aux = reinterpret_cast<uint32_t*>(dd.table_aux);  // slot s: [4s] representative, [4s+1] unique id
-    bool bad = false, full = false, overflow = false;
+    bool overflow = false;
     if (blockIdx.x >= ntiles) return;  // grids are sized by an upper bound on n
     while (true) {
         const uint32_t tile = next_tile(a.tile_counter, &S.slot);
@@ -337,36 +317,6 @@ __global__ void __launch_bounds__(kT, 3) extract_level(ExtractArgs a) {
             dst[0] = make_uint4(ch[0], ch[1], ch[2], ch[3]);
             dst[1] = make_uint4(ch[4], ch[5], ch[6], ch[7]);
             a.node_hashes[p] = hv;
-            if (fuse) {
-                // The node's hash into the dedup table; the first inserter of
-                // a hash is its representative and appends it to its bucket.
-                uint64_t sl = home_slot(hv, tslots);
-                bool won = false, placed = false;
-                if (hv == 0) {
-                    bad = true;  // 0 marks an empty slot
-                } else {
-                    for (uint64_t probe = 0; probe < tslots; ++probe) {
-                        uint64_t cur = read_first ? ld_relaxed(dd.table_key + 2 * sl) : 0ull;
-                        if (cur == 0)
-                            cur = atomicCAS((unsigned long long*)(dd.table_key + 2 * sl), 0ull, (unsigned long long)hv);
-                        if (cur == 0 || cur == hv) { won = cur == 0; placed = true; break; }
-                        sl = next_slot(sl, tslots);
-                    }
-                }
-                if (!placed && hv != 0) full = true;
-                dd.item_slot[p] = placed ? (uint32_t)sl : 0xFFFFFFFFu;
-                if (won) {
-                    aux[4 * sl] = (uint32_t)p;
-                    const uint32_t b = shift >= 64 ? 0u : (uint32_t)(hv >> shift);
-                    const uint32_t bs = atomicAdd(dd.bucket_count + b, 1u);
-                    if (bs < kDedupTopBitCap) {
-                        const uint64_t be = (uint64_t)b * kDedupTopBitCap + bs;
-                        dd.bucket[be] = make_uint4((uint32_t)hv, (uint32_t)(hv >> 32), (uint32_t)sl, (uint32_t)p);
-                    } else {
-                        full = true;
-                    }
-                }
-            }
         }
         if (tid == 0 && base + tile_n == n) {
             const uint64_t cnt = p_base + total_heads;
@@ -375,8 +325,6 @@ __global__ void __launch_bounds__(kT, 3) extract_level(ExtractArgs a) {
         __syncthreads();
     }
     if (overflow) atomicOr(a.err, kErrCapacity);
-    if (bad) atomicOr(a.err, kErrBadInput);
-    if (full) atomicOr(a.err, kErrFallback);
 }
 
 // ---------------------------------------------------------------------------
@@ -492,7 +440,7 @@ __global__ void __launch_bounds__(kT) unique_runs(UniqueArgs a) {
 
 
 // ---------------------------------------------------------------------------
-// Tail: all levels with at most kTailCap nodes, in one CTA.
+// Tail of the radix form: all levels with at most kTailCap nodes, in one CTA.
 // ---------------------------------------------------------------------------
 struct TailSmem {
     uint64_t code[2][kTailCap];   // node codes of the level being built / its children

@@ -55,7 +55,7 @@ struct CallHeader {
     uint64_t counts[64];
     uint32_t tile_counters[kMaxTileCounters];
     uint32_t hist[kMaxSorts][kSortHistWords];
-    DedupState dedup[kMaxDepth + 1];  // leaves + one per level
+    DedupState dedup;
     uint32_t sketch[kGroupSketchRegs];  // distinct-brick sketch of the fragment grouping's probe
     uint32_t gover[kGroupMaxParts];     // its partitions that spilled past their slabs
     uint64_t gcursor[kGroupMaxParts];   // its partition starts, then ends
@@ -322,6 +322,10 @@ struct dagc_context_t {
     bool profiling = false;
     bool use_graphs = true;
     cudaStream_t capture_stream = nullptr;
+    // A call's node extraction runs beside its leaf order: on this stream,
+    // between these events (null: one after the other).
+    cudaStream_t side_stream = nullptr;
+    cudaEvent_t side_fork = nullptr, side_join = nullptr;
     std::vector<GraphEntry> graphs;
     std::vector<GraphKey> graph_seen;  // call shapes launched directly once; recorded when seen again
     // Digit-pass plans. A forced shape / width (dagc_set_option, >= 0)
@@ -533,13 +537,12 @@ int device_error_status(uint32_t err, std::string& msg) {
 // for its tile bound; the regions are carved in launch order.
 struct CallSlots {
     CallHeader* h;
-    int next_counter = 0, next_hist = 0, next_dedup = 0;
+    int next_counter = 0, next_hist = 0;
     uint64_t* sv_next = nullptr;
     uint64_t* sv_end = nullptr;
     uint32_t* counter() { return &h->tile_counters[next_counter++]; }
     uint32_t* counters(int k) { uint32_t* p = &h->tile_counters[next_counter]; next_counter += k; return p; }
     uint32_t* hist() { return h->hist[next_hist++]; }
-    DedupState* dedup() { return &h->dedup[next_dedup++]; }
     uint64_t* sv(uint64_t n_bound) {
         uint64_t* p = sv_next;
         sv_next += scan_tiles(n_bound) + 1;
@@ -811,9 +814,16 @@ struct CreateLayout {
     std::vector<size_t> o_ph, o_pc, o_pm;
     // Hash-set dedup (when `dedup`): per-item slots, the unique list, buckets.
     bool dedup = false;
-    uint64_t item_cap = 0, uniq_cap = 0, bucket_area = 0, table_slots = 0;
+    uint64_t item_cap = 0, uniq_cap = 0, leaf_area = 0, bucket_area = 0, table_slots = 0;
     size_t o_islot = 0, o_ukey = 0, o_uslot = 0;
     size_t o_bcnt = 0, o_bent = 0;
+    // Its node levels: per level the nodes' hashes, child masks and first
+    // children; groups of levels deduplicated together, (last, first) bottom up.
+    std::vector<size_t> o_nh, o_nm, o_nf;
+    std::vector<std::pair<int, int>> groups;
+    uint64_t slot_cap = 0, bucket_cap = 0;
+    // Nodes of a level that the dedup can hold.
+    uint64_t items_of(int l) const { return std::min<uint64_t>(cap[l], kDedupMaxItems); }
     // Persistent per-chunk leaves (batched form): zeroed chunk state
     // (histograms, cursors, done counters, item counter), item offsets, the
     // mask stage and per-item brick counts / offsets.
@@ -837,6 +847,30 @@ struct CreateLayout {
             o_dcount = L.take<uint32_t>(direct_blocks(depth));
             o_dsv = L.take<uint64_t>(direct_plan_tiles(depth));
         }
+        if (use_dedup) {
+            item_cap = std::min<uint64_t>(p0cap, kDedupMaxItems);
+            table_slots = table_slots_upto(item_cap);
+            uint64_t area = 0;
+            for (int hi = nl - 1; hi >= 0;) {
+                uint64_t items = 0, slots = 0, buckets = 0, places = 0;
+                int lo = hi + 1;
+                while (lo > 0 && (lo == hi + 1 || items + items_of(lo - 1) <= kGroupItems)) {
+                    --lo;
+                    items += items_of(lo);
+                    slots += table_size_for(items_of(lo), false);
+                    buckets += node_buckets_upto(items_of(lo));
+                    places += group_slot_items(items_of(lo));
+                }
+                groups.push_back({hi, lo});
+                table_slots = std::max(table_slots, slots);
+                bucket_cap = std::max(bucket_cap, buckets);
+                slot_cap = std::max(slot_cap, places);
+                area = std::max(area, buckets * kDedupTopBitCap);
+                hi = lo - 1;
+            }
+            bucket_area = area;
+            o_bcnt = L.take<uint32_t>(bucket_cap);
+        }
         zero_bytes = L.off;
         if (direct_table) o_dlist = L.take<uint2>(direct_blocks(depth));
         const bool sorts = !direct || !use_dedup;
@@ -858,24 +892,29 @@ struct CreateLayout {
         o_V = L.take<uint32_t>(sort_cap);
         o_Va = L.take<uint32_t>(sort_cap);
         if (dedup) {
-            // Items per level are at most p0cap (leaves) or cap[l] <= p0cap.
-            item_cap = std::min<uint64_t>(p0cap, kDedupMaxItems);
             uniq_cap = std::min<uint64_t>(p0cap, std::min<uint64_t>(unique_limit, kDedupMaxUnique));
-            bucket_area = dedup_bucket_area(uniq_cap);
-            table_slots = table_slots_upto(item_cap);
-            o_islot = L.take<uint32_t>(item_cap);
+            leaf_area = dedup_bucket_area(uniq_cap);
+            o_islot = L.take<uint32_t>(std::max(item_cap, slot_cap));
             o_ukey = L.take<uint64_t>(uniq_cap);
             o_uslot = L.take<uint32_t>(uniq_cap);
-            o_bcnt = L.take<uint32_t>(kDedupMaxBuckets);
-            o_bent = L.take<uint4>(bucket_area);
+            o_bent = L.take<uint4>(std::max(leaf_area, bucket_area));
         }
         o_M0 = L.take<uint32_t>(p0cap);
         o_M1 = L.take<uint32_t>(p0cap);
         o_NC0 = L.take<uint64_t>(capmax);
         o_NC1 = L.take<uint64_t>(capmax);
-        o_NM = L.take<uint8_t>(capmax);
-        o_NCH = L.take<uint32_t>(std::max<uint64_t>(capmax, kTailCap) * 8);
-        o_NH = L.take<uint64_t>(capmax);
+        if (dedup) {
+            o_nh.resize(nl); o_nm.resize(nl); o_nf.resize(nl);
+            for (int l = 0; l < nl; ++l) {
+                o_nh[l] = L.take<uint64_t>(cap[l]);
+                o_nf[l] = L.take<uint32_t>(cap[l]);
+                o_nm[l] = L.take<uint8_t>(cap[l]);
+            }
+        } else {
+            o_NM = L.take<uint8_t>(capmax);
+            o_NCH = L.take<uint32_t>(std::max<uint64_t>(capmax, kTailCap) * 8);
+            o_NH = L.take<uint64_t>(capmax);
+        }
         o_PL = L.take<uint64_t>(p0cap);
         o_ph.resize(nl); o_pc.resize(nl); o_pm.resize(nl);
         for (int l = 0; l < nl; ++l) {
@@ -1233,17 +1272,73 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
             t.stop();
         }
         // 3. Leaf dedup: SortLevel on the leaf masks (the mask is its own hash).
-        StageTimer t_dedup(ctx, DAGC_STAGE_LEAF_DEDUP, s);
-        // Hash-set dedup arguments shared by the leaves and every level.
-        auto dedup_args = [&](const uint64_t* keys, uint64_t* d_n, const uint8_t* masks, const uint32_t* children,
-                              uint64_t* out_keys, uint8_t* out_masks, uint32_t* out_children, uint64_t out_cap,
-                              uint64_t* d_out_n, uint32_t* map) {
+        // 4. Level loop, bottom-up.
+        if (use_dedup) {
+            // The nodes of every level: their hashes need the leaf masks by
+            // brick and nothing of the leaf dedup, so they are extracted
+            // beside it (on the side stream, but for profiled calls, whose
+            // stages are timed one after the other, and programmatic launches,
+            // which follow one stream).
+            auto nodes_of = [&](int l) {
+                return NodeArrays{P64(Lo.o_nh[l]), P8(Lo.o_nm[l]), P32(Lo.o_nf[l])};
+            };
+            auto extract_all = [&](cudaStream_t s) {
+                TailNodesArgs ta{};
+                ta.levels = nl;
+                ta.err = err;
+                uint64_t* node_codes[2] = {P64(Lo.o_NC0), P64(Lo.o_NC1)};
+                for (int l = nl - 1, it = 0; l >= 0; --l, ++it) {
+                    const bool bottom = l == nl - 1;
+                    const uint64_t bound = bottom ? p0cap : cap[l + 1];
+                    NodesArgs e{};
+                    e.child_codes = bottom ? P64(Lo.o_P) : node_codes[(it & 1) ^ 1];
+                    e.child_hashes = bottom ? P64(Lo.o_LM) : P64(Lo.o_nh[l + 1]);
+                    e.d_n = bottom ? cs.count(kCntBricks) : cs.count(kCntNodes + l + 1);
+                    TailNodesLevel& t = ta.lv[l];
+                    t.child_codes = e.child_codes;
+                    t.child_hashes = e.child_hashes;
+                    t.d_child_n = e.d_n;
+                    t.out = nodes_of(l);
+                    t.capacity = cap[l];
+                    t.d_nodes = cs.count(kCntNodes + l);
+                    if (bound <= (uint64_t)kTailCap) continue;  // always the tail's
+                    e.n_bound = bound;
+                    e.node_codes = node_codes[it & 1];
+                    e.out = t.out;
+                    e.out_capacity = cap[l];
+                    e.d_out_n = t.d_nodes;
+                    e.tail_max = (uint64_t)kTailCap;
+                    e.status = cs.sv(bound);
+                    e.tile_counter = cs.counter();
+                    e.err = err;
+                    launch_extract_nodes(e, s);
+                    ++ctx->launches;
+                }
+                if (nl > 0) {
+                    launch_tail_nodes(ta, s);
+                    ++ctx->launches;
+                }
+            };
+            const bool beside = ctx->side_stream && !ctx->profiling && !ctx->pdl && nl > 0;
+            if (beside) {
+                DAGC_CUDA(ctx, cudaEventRecord(ctx->side_fork, s));
+                DAGC_CUDA(ctx, cudaStreamWaitEvent(ctx->side_stream, ctx->side_fork, 0));
+                extract_all(ctx->side_stream);
+                DAGC_CUDA(ctx, cudaEventRecord(ctx->side_join, ctx->side_stream));
+                DAGC_LAUNCHED(ctx);
+            } else {
+                StageTimer t(ctx, DAGC_STAGE_LEVELS, s);
+                extract_all(s);
+                DAGC_LAUNCHED(ctx);
+                t.stop(1);  // the levels' bytes are counted with their dedup below
+            }
+            // Distinct masks into the table and the unique list; the list
+            // ordered into the leaf array, each mask's rank to its slot as
+            // unique id; every brick its id.
+            StageTimer t_dedup(ctx, DAGC_STAGE_LEAF_DEDUP, s);
             DedupArgs d{};
-            d.keys = keys;
-            d.d_n = d_n;
-            d.masks = masks;
-            d.children = children;
-            d.to_list = masks == nullptr;  // leaf masks are not uniformly distributed; node hashes are
+            d.keys = P64(Lo.o_LM);
+            d.d_n = cs.count(kCntBricks);
             d.item_cap = Lo.item_cap;
             d.table_key = static_cast<uint64_t*>(ctx->table);
             d.table_aux = static_cast<uint64_t*>(ctx->table) + 1;
@@ -1254,166 +1349,168 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
             d.leaf = &cs.h->leaf;
             d.leaf_keys = leaf_keys_for(Lo.uniq_cap);
             d.uniq_cap = Lo.uniq_cap;
-            d.bucket_count = P32(Lo.o_bcnt);
             d.bucket = reinterpret_cast<uint4*>(b + Lo.o_bent);
-            d.bucket_area = Lo.bucket_area;
-            d.state = cs.dedup();
-            d.out_keys = out_keys;
-            d.out_masks = out_masks;
-            d.out_children = out_children;
-            d.out_capacity = out_cap;
-            d.d_out_n = d_out_n;
-            d.map = map;
+            d.bucket_area = Lo.leaf_area;
+            d.state = &cs.h->dedup;
+            d.out_keys = P64(Lo.o_PL);
+            d.out_capacity = p0cap;
+            d.d_out_n = cs.count(kCntLeaves);
+            d.map = P32(Lo.o_M0);
             d.err = err;
-            return d;
-        };
-        if (use_dedup) {
-            // Distinct masks into the table and the unique list; the list
-            // ordered into the leaf array, each mask's rank to its slot as
-            // unique id; every brick its id.
-            const DedupArgs d = dedup_args(P64(Lo.o_LM), cs.count(kCntBricks), nullptr, nullptr, P64(Lo.o_PL), nullptr,
-                                           nullptr, p0cap, cs.count(kCntLeaves), P32(Lo.o_M0));
             launch_dedup_insert(d, s);
             ctx->launches += launch_leaf_order(d, s);
             launch_dedup_map(d, s);
             ctx->launches += 2;
             DAGC_LAUNCHED(ctx);
-        } else {
-        st = run_sort(ctx, cs, sb, P64(Lo.o_LM), P64(Lo.o_SK), P64(Lo.o_SKa), nullptr, P32(Lo.o_V), P32(Lo.o_Va), true, p0cap,
-                      cs.count(kCntBricks), 0, 64, 0, s);
-        if (st) return st;
-        {
-            UniqueArgs a{};
-            a.keys = P64(Lo.o_SK);
-            a.perm = P32(Lo.o_V);
-            a.d_n = cs.count(kCntBricks);
-            a.n_bound = p0cap;
-            a.map = P32(Lo.o_M0);
-            a.out_keys = P64(Lo.o_PL);
-            a.out_capacity = p0cap;
-            a.d_out_n = cs.count(kCntLeaves);
-            a.status = cs.sv(p0cap);
-            a.tile_counter = cs.counter();
-            a.err = err;
-            a.grid = grid_for(ctx->grid_unique / ctx->sms, ctx->sms, scan_tiles(p0cap));
-            launch_unique(a, s);
-            ++ctx->launches;
-            DAGC_LAUNCHED(ctx);
-        }
-        }
-        t_dedup.stop();
-        // 4. Level loop, bottom-up.
-        StageTimer t_levels(ctx, DAGC_STAGE_LEVELS, s);
-        const uint64_t* child_codes = P64(Lo.o_P);
-        const uint32_t* child_map = P32(Lo.o_M0);
-        const uint64_t* child_hashes = P64(Lo.o_PL);
-        const uint64_t* d_child_n = cs.count(kCntBricks);
-        uint64_t child_bound = p0cap;
-        uint64_t* node_codes[2] = {P64(Lo.o_NC0), P64(Lo.o_NC1)};
-        uint32_t* maps[2] = {P32(Lo.o_M1), P32(Lo.o_M0)};
-        // Levels whose node bound fits one CTA's shared memory go to the tail
-        // kernel; the bound only grows with the level index, so they are the top
-        // tail_first + 1 levels.
-        int tail_first = -1;
-        while (tail_first + 1 < nl && tail_first + 1 < kMaxTailLevels && cap[tail_first + 1] <= (uint64_t)kTailCap)
-            ++tail_first;
-        // The tail's first level reads all of its children in one CTA: a level
-        // that may have many (8^5 bound at depth >= 8 with dense top levels)
-        // goes to the multi-CTA path instead.
-        while (tail_first >= 0 && (tail_first + 1 < nl ? cap[tail_first + 1] : p0cap) > (uint64_t)kTailChildCap)
-            --tail_first;
-        for (int l = nl - 1, it = 0; l > tail_first; --l, ++it) {
-            ExtractArgs e{};
-            e.child_codes = child_codes;
-            e.child_map = child_map;
-            e.d_n = d_child_n;
-            e.n_bound = child_bound;
-            e.child_hashes = child_hashes;
-            e.node_codes = node_codes[it & 1];
-            e.node_masks = P8(Lo.o_NM);
-            e.node_children = P32(Lo.o_NCH);
-            e.node_hashes = P64(Lo.o_NH);
-            e.out_capacity = cap[l];
-            e.d_out_n = cs.count(kCntNodes + l);
-            e.status = cs.sv(child_bound);
-            e.tile_counter = cs.counter();
-            e.err = err;
-            e.grid = grid_for(ctx->grid_extract / ctx->sms, ctx->sms, scan_tiles(child_bound));
-            DedupArgs d{};
-            if (use_dedup) {
-                // The node hashes go into the dedup table inside extract_level.
-                d = dedup_args(P64(Lo.o_NH), cs.count(kCntNodes + l), P8(Lo.o_NM), P32(Lo.o_NCH), P64(Lo.o_ph[l]),
-                               P8(Lo.o_pm[l]), P32(Lo.o_pc[l]), cap[l], cs.count(kCntUnique + l), maps[it & 1]);
-                e.fuse_insert = 1;
-                e.dedup = d;
-            }
-            launch_extract(e, s);
-            ++ctx->launches;
-            DAGC_LAUNCHED(ctx);
-
-            if (use_dedup) {
-                ctx->launches += launch_dedup(d, s);
+            t_dedup.stop();
+            if (beside) DAGC_CUDA(ctx, cudaStreamWaitEvent(s, ctx->side_join, 0));
+            // The node levels' dedup, a group of levels at a time, bottom up.
+            StageTimer t_levels(ctx, DAGC_STAGE_LEVELS, s);
+            uint32_t* maps[2] = {P32(Lo.o_M0), P32(Lo.o_M1)};
+            for (size_t g = 0; g < Lo.groups.size(); ++g) {
+                const int hi = Lo.groups[g].first, lo = Lo.groups[g].second;
+                GroupDedupArgs ga{};
+                uint64_t items = 0;
+                ga.levels = hi - lo + 1;
+                for (int l = lo; l <= hi; ++l) {
+                    ga.lv[l - lo] = GroupLevel{nodes_of(l), cs.count(kCntNodes + l), P64(Lo.o_ph[l]), P8(Lo.o_pm[l]),
+                                               P32(Lo.o_pc[l]), cap[l], cs.count(kCntUnique + l)};
+                    items += Lo.items_of(l);
+                }
+                ga.child_map = maps[g & 1];
+                ga.map = lo > 0 ? maps[(g & 1) ^ 1] : nullptr;
+                ga.table_key = d.table_key;
+                ga.table_aux = d.table_aux;
+                ga.table_cap = d.table_cap;
+                ga.item_slot = d.item_slot;
+                ga.slot_cap = Lo.slot_cap;
+                ga.bucket_count = P32(Lo.o_bcnt);
+                ga.bucket_cap = (uint32_t)Lo.bucket_cap;
+                ga.bucket = d.bucket;
+                ga.bucket_area = Lo.bucket_area;
+                ga.uniq_cap = Lo.uniq_cap;
+                ga.err = err;
+                ctx->launches += launch_group_dedup(ga, items, s);
                 DAGC_LAUNCHED(ctx);
+            }
+            t_levels.stop();
+        } else {
+            StageTimer t_dedup(ctx, DAGC_STAGE_LEAF_DEDUP, s);
+            st = run_sort(ctx, cs, sb, P64(Lo.o_LM), P64(Lo.o_SK), P64(Lo.o_SKa), nullptr, P32(Lo.o_V), P32(Lo.o_Va), true, p0cap,
+                          cs.count(kCntBricks), 0, 64, 0, s);
+            if (st) return st;
+            {
+                UniqueArgs a{};
+                a.keys = P64(Lo.o_SK);
+                a.perm = P32(Lo.o_V);
+                a.d_n = cs.count(kCntBricks);
+                a.n_bound = p0cap;
+                a.map = P32(Lo.o_M0);
+                a.out_keys = P64(Lo.o_PL);
+                a.out_capacity = p0cap;
+                a.d_out_n = cs.count(kCntLeaves);
+                a.status = cs.sv(p0cap);
+                a.tile_counter = cs.counter();
+                a.err = err;
+                a.grid = grid_for(ctx->grid_unique / ctx->sms, ctx->sms, scan_tiles(p0cap));
+                launch_unique(a, s);
+                ++ctx->launches;
+                DAGC_LAUNCHED(ctx);
+            }
+            t_dedup.stop();
+            StageTimer t_levels(ctx, DAGC_STAGE_LEVELS, s);
+            const uint64_t* child_codes = P64(Lo.o_P);
+            const uint32_t* child_map = P32(Lo.o_M0);
+            const uint64_t* child_hashes = P64(Lo.o_PL);
+            const uint64_t* d_child_n = cs.count(kCntBricks);
+            uint64_t child_bound = p0cap;
+            uint64_t* node_codes[2] = {P64(Lo.o_NC0), P64(Lo.o_NC1)};
+            uint32_t* maps[2] = {P32(Lo.o_M1), P32(Lo.o_M0)};
+            // Levels whose node bound fits one CTA's shared memory go to the tail
+            // kernel; the bound only grows with the level index, so they are the top
+            // tail_first + 1 levels.
+            int tail_first = -1;
+            while (tail_first + 1 < nl && tail_first + 1 < kMaxTailLevels && cap[tail_first + 1] <= (uint64_t)kTailCap)
+                ++tail_first;
+            // The tail's first level reads all of its children in one CTA: a level
+            // that may have many (8^5 bound at depth >= 8 with dense top levels)
+            // goes to the multi-CTA path instead.
+            while (tail_first >= 0 && (tail_first + 1 < nl ? cap[tail_first + 1] : p0cap) > (uint64_t)kTailChildCap)
+                --tail_first;
+            for (int l = nl - 1, it = 0; l > tail_first; --l, ++it) {
+                ExtractArgs e{};
+                e.child_codes = child_codes;
+                e.child_map = child_map;
+                e.d_n = d_child_n;
+                e.n_bound = child_bound;
+                e.child_hashes = child_hashes;
+                e.node_codes = node_codes[it & 1];
+                e.node_masks = P8(Lo.o_NM);
+                e.node_children = P32(Lo.o_NCH);
+                e.node_hashes = P64(Lo.o_NH);
+                e.out_capacity = cap[l];
+                e.d_out_n = cs.count(kCntNodes + l);
+                e.status = cs.sv(child_bound);
+                e.tile_counter = cs.counter();
+                e.err = err;
+                e.grid = grid_for(ctx->grid_extract / ctx->sms, ctx->sms, scan_tiles(child_bound));
+                launch_extract(e, s);
+                ++ctx->launches;
+                DAGC_LAUNCHED(ctx);
+
+                st = run_sort(ctx, cs, sb, P64(Lo.o_NH), P64(Lo.o_SK), P64(Lo.o_SKa), nullptr, P32(Lo.o_V), P32(Lo.o_Va), true,
+                              cap[l], cs.count(kCntNodes + l), 0, 64, 0, s);
+                if (st) return st;
+
+                UniqueArgs u{};
+                u.keys = P64(Lo.o_SK);
+                u.perm = P32(Lo.o_V);
+                u.d_n = cs.count(kCntNodes + l);
+                u.n_bound = cap[l];
+                u.masks = P8(Lo.o_NM);
+                u.children = P32(Lo.o_NCH);
+                u.map = maps[it & 1];
+                u.out_keys = P64(Lo.o_ph[l]);
+                u.out_masks = P8(Lo.o_pm[l]);
+                u.out_children = P32(Lo.o_pc[l]);
+                u.out_capacity = cap[l];
+                u.d_out_n = cs.count(kCntUnique + l);
+                u.status = cs.sv(cap[l]);
+                u.tile_counter = cs.counter();
+                u.err = err;
+                u.grid = grid_for(ctx->grid_unique / ctx->sms, ctx->sms, scan_tiles(cap[l]));
+                launch_unique(u, s);
+                ++ctx->launches;
+                DAGC_LAUNCHED(ctx);
+
                 child_codes = node_codes[it & 1];
                 child_map = maps[it & 1];
                 child_hashes = P64(Lo.o_ph[l]);
                 d_child_n = cs.count(kCntNodes + l);
                 child_bound = cap[l];
-                continue;
             }
-            st = run_sort(ctx, cs, sb, P64(Lo.o_NH), P64(Lo.o_SK), P64(Lo.o_SKa), nullptr, P32(Lo.o_V), P32(Lo.o_Va), true,
-                          cap[l], cs.count(kCntNodes + l), 0, 64, 0, s);
-            if (st) return st;
-
-            UniqueArgs u{};
-            u.keys = P64(Lo.o_SK);
-            u.perm = P32(Lo.o_V);
-            u.d_n = cs.count(kCntNodes + l);
-            u.n_bound = cap[l];
-            u.masks = P8(Lo.o_NM);
-            u.children = P32(Lo.o_NCH);
-            u.map = maps[it & 1];
-            u.out_keys = P64(Lo.o_ph[l]);
-            u.out_masks = P8(Lo.o_pm[l]);
-            u.out_children = P32(Lo.o_pc[l]);
-            u.out_capacity = cap[l];
-            u.d_out_n = cs.count(kCntUnique + l);
-            u.status = cs.sv(cap[l]);
-            u.tile_counter = cs.counter();
-            u.err = err;
-            u.grid = grid_for(ctx->grid_unique / ctx->sms, ctx->sms, scan_tiles(cap[l]));
-            launch_unique(u, s);
-            ++ctx->launches;
-            DAGC_LAUNCHED(ctx);
-
-            child_codes = node_codes[it & 1];
-            child_map = maps[it & 1];
-            child_hashes = P64(Lo.o_ph[l]);
-            d_child_n = cs.count(kCntNodes + l);
-            child_bound = cap[l];
-        }
-        if (tail_first >= 0) {
-            TailArgs ta{};
-            ta.first_level = tail_first;
-            ta.child_codes = child_codes;
-            ta.child_map = child_map;
-            ta.child_hashes = child_hashes;
-            ta.d_child_n = d_child_n;
-            for (int l = 0; l <= tail_first; ++l) {
-                ta.lv[l].hashes = P64(Lo.o_ph[l]);
-                ta.lv[l].masks = P8(Lo.o_pm[l]);
-                ta.lv[l].children = P32(Lo.o_pc[l]);
-                ta.lv[l].capacity = cap[l];
-                ta.lv[l].d_nodes = cs.count(kCntNodes + l);
-                ta.lv[l].d_unique = cs.count(kCntUnique + l);
+            if (tail_first >= 0) {
+                TailArgs ta{};
+                ta.first_level = tail_first;
+                ta.child_codes = child_codes;
+                ta.child_map = child_map;
+                ta.child_hashes = child_hashes;
+                ta.d_child_n = d_child_n;
+                for (int l = 0; l <= tail_first; ++l) {
+                    ta.lv[l].hashes = P64(Lo.o_ph[l]);
+                    ta.lv[l].masks = P8(Lo.o_pm[l]);
+                    ta.lv[l].children = P32(Lo.o_pc[l]);
+                    ta.lv[l].capacity = cap[l];
+                    ta.lv[l].d_nodes = cs.count(kCntNodes + l);
+                    ta.lv[l].d_unique = cs.count(kCntUnique + l);
+                }
+                ta.err = err;
+                launch_tail(ta, s);
+                ++ctx->launches;
+                DAGC_LAUNCHED(ctx);
             }
-            ta.err = err;
-            launch_tail(ta, s);
-            ++ctx->launches;
-            DAGC_LAUNCHED(ctx);
+            t_levels.stop();
         }
-
-        t_levels.stop();
         if (cs.sv_next > cs.sv_end) return set_error(ctx, DAGC_ERR_CUDA, "look-back status regions miscounted");
     return DAGC_OK;
     };
@@ -2109,6 +2206,15 @@ int dagc_context_create(int device, dagc_context* out) {
         cudaGetLastError();
         c->capture_stream = nullptr;  // graphs off; calls launch directly
     }
+    if (cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->side_fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->side_join, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        if (c->side_stream) cudaStreamDestroy(c->side_stream);
+        if (c->side_fork) cudaEventDestroy(c->side_fork);
+        c->side_stream = nullptr;
+        c->side_fork = c->side_join = nullptr;
+    }
     if (const char* g = std::getenv("DAGC_GRAPHS")) c->use_graphs = std::atoi(g) != 0;
     if (const char* d = std::getenv("DAGC_DEDUP")) c->use_dedup = std::atoi(d) != 0;
     if (const char* gm = std::getenv("DAGC_GROUP")) c->group_mode = std::min(2, std::max(0, std::atoi(gm)));
@@ -2158,6 +2264,7 @@ int dagc_context_create(int device, dagc_context* out) {
     dedup_configure(c->sms);
     group_configure(c->sms);
     direct_configure(c->sms);
+    levels_configure(c->sms);
     chunk_configure(c->sms);
     voxelize_configure();
     *out = c.release();
@@ -2174,6 +2281,9 @@ void dagc_context_destroy(dagc_context ctx) {
     if (ctx->arena_copy) cudaEventDestroy(ctx->arena_copy);
     drop_graphs(ctx);
     if (ctx->capture_stream) cudaStreamDestroy(ctx->capture_stream);
+    if (ctx->side_stream) cudaStreamDestroy(ctx->side_stream);
+    if (ctx->side_fork) cudaEventDestroy(ctx->side_fork);
+    if (ctx->side_join) cudaEventDestroy(ctx->side_join);
     ctx->arena.release();
     if (ctx->table) cudaFree(ctx->table);
     if (ctx->gtable) cudaFree(ctx->gtable);

@@ -280,11 +280,9 @@ struct UniqueArgs {
 };
 void launch_unique(const UniqueArgs& a, cudaStream_t s);
 
-// ExtractLevel + ComputeHashes: from the sorted unique codes of the child
-// level and their child ids, build one parent node per distinct code >> 3.
-
-// Level dedup by hash set + ordering of the distinct keys (dedup.cu): same
-// outputs as sort pairs + unique_runs on (key, item) for one level.
+// Level dedup by hash set + ordering of the distinct keys (dedup.cu the leaf
+// masks, levels.cu the node levels): same outputs as sort pairs + unique_runs on
+// (key, item) for one level.
 constexpr uint32_t kDedupPerBucket = 256;            // expected distinct keys per bucket (node hashes)
 constexpr uint32_t kDedupTopBitCap = 1024;           // bucket room (128-256 expected)
 constexpr uint32_t kDedupMaxBuckets = 16384;
@@ -296,6 +294,11 @@ DAGC_HD uint64_t dedup_bucket_area(uint64_t uniq_cap) {
     const uint64_t a = 8 * uniq_cap > kDedupTopBitCap ? 8 * uniq_cap : kDedupTopBitCap;
     const uint64_t most = (uint64_t)kDedupMaxBuckets * kDedupTopBitCap;
     return a < most ? a : most;
+}
+// The same for one node level of up to n items: its buckets' room.
+DAGC_HD uint64_t node_buckets_upto(uint64_t n) {
+    const uint64_t b = n / (kDedupPerBucket / 2) + 1;
+    return b < kDedupMaxBuckets ? b : kDedupMaxBuckets;
 }
 // Table slots for n items. Leaf masks repeat (about one distinct mask per ten
 // bricks): 1.25 n slots, at most 0.8 full even when every mask is distinct,
@@ -319,9 +322,7 @@ DAGC_HD uint64_t table_slots_upto(uint64_t items) {
     return most > sparse ? most : sparse;
 }
 struct DedupState {
-    unsigned long long u;  // distinct keys found (zero before the level)
-    uint32_t nbuckets, pad0;
-    uint32_t inserted, pad;  // 1: extract_level already inserted the level's hashes
+    unsigned long long u;  // distinct keys found (zero on entry)
 };
 // Ordering of the distinct leaf masks: up to kLeafRankMax of them are ranked
 // at once, more go through buckets between samples (half as many buckets up to
@@ -337,11 +338,7 @@ struct LeafOrder {
 // hold uniq_cap: the mean is at most 256 up to kLeafMidMax, then uniq_cap / 2048.
 DAGC_HD uint32_t leaf_keys_for(uint64_t uniq_cap) { return uniq_cap <= kLeafMidMax ? 2048u : 8192u; }
 struct DedupArgs {
-    const uint64_t* keys; const uint64_t* d_n;       // items: key per item
-    const uint8_t* masks; const uint32_t* children;  // item payloads (null for leaves)
-    // Leaf masks (far from uniform): winners go to the unique list, ordered by
-    // launch_leaf_order. Node hashes: winners go to the bucket of their top bits.
-    bool to_list;
+    const uint64_t* keys; const uint64_t* d_n;  // the bricks' leaf masks
     uint64_t item_cap;
     // Table of table_cap slots, 16 bytes each so that a
     // slot's key and aux share a sector: table_key[2s] = key, 0 = empty (all
@@ -349,29 +346,75 @@ struct DedupArgs {
     // << 32 (table_aux = table_key + 1).
     uint64_t* table_key; uint64_t* table_aux; uint64_t table_cap;
     uint32_t* item_slot;
-    uint64_t* uniq_key; uint32_t* uniq_slot; uint64_t uniq_cap;  // the unique list (leaf masks) and its slots
+    uint64_t* uniq_key; uint32_t* uniq_slot; uint64_t uniq_cap;  // the unique list and its slots
     LeafOrder* leaf; uint32_t leaf_keys;                         // its ordering; leaf_keys_for(uniq_cap)
-    uint32_t* bucket_count;                                       // kDedupMaxBuckets
-    // Bucket entries, one 16-byte store each: key (two words), slot, representative.
-    uint4* bucket; uint64_t bucket_area;
+    uint4* bucket; uint64_t bucket_area;                         // bucket entries: key (two words), slot
     DedupState* state;
-    uint64_t* out_keys; uint8_t* out_masks; uint32_t* out_children; uint64_t out_capacity;
+    uint64_t* out_keys; uint64_t out_capacity;
     uint64_t* d_out_n;
     uint32_t* map;  // item -> unique id
     uint32_t* err;
 };
 void dedup_configure(int sms);
-// Node levels: insert (unless extract_level did), bucket sort, map; returns
-// the number of launches.
-int launch_dedup(const DedupArgs& a, cudaStream_t s);
-// Leaf masks: insert into the table and the unique list; order the list into
-// the leaf array and assign the unique ids (returns the number of launches);
-// then map.
+// Insert into the table and the unique list; order the list into the leaf array
+// and assign the unique ids (returns the number of launches); then map.
 void launch_dedup_insert(const DedupArgs& a, cudaStream_t s);
 int launch_leaf_order(const DedupArgs& a, cudaStream_t s);
 void launch_dedup_map(const DedupArgs& a, cudaStream_t s);
 
-constexpr uint64_t kFuseInsertMax = 1ull << 20;
+// Node levels of the hash-set form (levels.cu): nodes of a level, in the order
+// of their codes.
+constexpr int kNodeLevels = 19;  // levels of the deepest DAG
+struct NodeArrays {
+    uint64_t* hash;
+    uint8_t* mask;     // children present
+    uint32_t* first;   // index of the first child among the level below's nodes (or bricks); the others follow it
+};
+struct NodesArgs {
+    const uint64_t* child_codes; const uint64_t* child_hashes;  // of every child (not only the distinct ones)
+    const uint64_t* d_n; uint64_t n_bound;
+    uint64_t* node_codes; NodeArrays out; uint64_t out_capacity;
+    uint64_t* d_out_n;
+    uint64_t tail_max;  // up to this many children the level is left to the tail
+    uint64_t* status; uint32_t* tile_counter; uint32_t* err;
+};
+void launch_extract_nodes(const NodesArgs& a, cudaStream_t s);
+// Every level from the largest one of at most kTailCap children up to the root.
+struct TailNodesLevel {
+    const uint64_t* child_codes; const uint64_t* child_hashes; const uint64_t* d_child_n;
+    NodeArrays out; uint64_t capacity;
+    uint64_t* d_nodes;
+};
+struct TailNodesArgs {
+    int levels;
+    TailNodesLevel lv[kNodeLevels];  // root first
+    uint32_t* err;
+};
+void launch_tail_nodes(const TailNodesArgs& a, cudaStream_t s);
+// Dedup of consecutive levels at once, into one table and one set of buckets.
+struct GroupLevel {
+    NodeArrays nodes; const uint64_t* d_n;
+    uint64_t* out_keys; uint8_t* out_masks; uint32_t* out_children; uint64_t capacity;
+    uint64_t* d_out_n;
+};
+constexpr uint64_t kGroupItems = 1ull << 24;  // levels share a group while their bounds add up to this
+struct GroupDedupArgs {
+    int levels;
+    GroupLevel lv[kNodeLevels];    // the group's levels, the one nearest the root first
+    const uint32_t* child_map;     // unique ids of the items below the group's last level
+    uint32_t* map;                 // null, or the unique ids of the first level's nodes (the next group's child_map)
+    uint64_t* table_key; uint64_t* table_aux; uint64_t table_cap;  // as DedupArgs
+    uint32_t* item_slot; uint64_t slot_cap;
+    uint32_t* bucket_count; uint32_t bucket_cap;                   // zero on entry and exit
+    uint4* bucket; uint64_t bucket_area;                           // kDedupTopBitCap entries each: key (two words), slot
+    uint64_t uniq_cap;
+    uint32_t* err;
+};
+void levels_configure(int sms);
+uint64_t group_slot_items(uint64_t n);  // item_slot entries of a level of n nodes
+int launch_group_dedup(const GroupDedupArgs& a, uint64_t items_bound, cudaStream_t s);  // returns the number of launches
+
+// One level of the radix form: nodes with their child ids and hashes.
 struct ExtractArgs {
     const uint64_t* child_codes; const uint32_t* child_map; const uint64_t* d_n; uint64_t n_bound;
     const uint64_t* child_hashes;  // unique child hashes (or leaf masks), indexed by child id
@@ -379,13 +422,6 @@ struct ExtractArgs {
     uint64_t out_capacity;
     uint64_t* d_out_n;
     uint64_t* status; uint32_t* tile_counter; uint32_t* err; int grid;
-    // Node levels of the hash-set form with at most kFuseInsertMax children:
-    // every node's hash goes straight into the dedup table and its top-bit
-    // bucket here (table and bucket count sized by the child count, a bound
-    // on the node count), and the level's dedup_insert returns at once.
-    // Larger levels keep the separate insert, whose probes overlap.
-    int fuse_insert;
-    DedupArgs dedup;
 };
 void launch_extract(const ExtractArgs& a, cudaStream_t s);
 
@@ -417,7 +453,7 @@ void voxelize_configure();
 void launch_voxelize(const VoxArgs& a, int grid, cudaStream_t s);
 uint64_t voxelize_tiles(uint64_t n_tri);
 
-// The top levels in one single-CTA launch: every level l <= first_level has at
+// The radix form's top levels in one single-CTA launch: every level l <= first_level has at
 // most kTailCap nodes, so extract + hash + sort + unique run in shared memory.
 constexpr int kTailThreads = 1024;
 constexpr int kTailCap = 4096;

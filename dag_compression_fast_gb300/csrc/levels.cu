@@ -1,0 +1,639 @@
+// The node levels of the hash-set form, for sm_103a. Replaces, per level, the
+// reference's ExtractLevel + ComputeHashes (src/DAGCompression.cu:916-974,
+// :827-833, :765-774) and SortLevel (:864-914): one node per distinct child
+// code >> 3, its hash, the distinct hashes in ascending order with their masks
+// and child ids.
+//
+// A node's hash needs its children's hashes, not their ids, so the levels fall
+// into two parts:
+//
+//   extract_nodes, one launch per level, bottom up: from the children's sorted
+//   codes and their hashes (the leaf masks below the last level), both read in
+//   order, the nodes' codes and hashes, child masks and first child;
+//   tail_nodes: the same for every level from the first one of at most
+//   kTailCap children up to the root, in one CTA;
+//
+//   then, for a whole group of levels at once (all of them, unless the bounds
+//   are large):
+//   nodes_insert  every node's hash into its level's part of the hash table
+//                 (linear probing, atomicCAS); the first inserter is the
+//                 hash's representative and appends it to the bucket of its
+//                 top bits;
+//   nodes_order   ranks each bucket: the distinct hashes in order, and their
+//                 ids to the table;
+//   nodes_finish  every node reads its id and its children's ids through the
+//                 table; representatives write their mask and children at
+//                 their id, the others are compared with theirs in full.
+//
+// Nothing here waits for the leaves' order until nodes_finish, so the first
+// part can run beside it. When each level was deduplicated before the next was
+// extracted (four launches per level, and the tail's sorts one after another),
+// the levels of a 512^3 terrain took 107 us, now 78 (and half of that beside the
+// leaves: the call 217 -> 157); of the 8192^3 soup 2.36 ms, now 1.89.
+
+#include "dagc_device.cuh"
+#include "dagc_kernels.h"
+#include "dagc_launch.h"
+
+#include <algorithm>
+
+namespace dagc {
+namespace {
+
+// ------------------------------------------------------------- extraction --
+constexpr int kXThreads = 256;
+constexpr int kXWarps = kXThreads / 32;
+constexpr int kXRows = kScanTile / kXThreads;  // rows of 256 children per tile
+constexpr int kXHalo = 7;                      // children of the tile's last node in the next tile
+static_assert(kXRows * kXWarps == 64, "two counts per lane of the scanning warp");
+
+struct NodesSmem {
+    uint64_t codes[kScanTile + 8];
+    uint64_t hash[kScanTile + 8];
+    uint16_t head[kScanTile];     // first child of each node that starts in the tile, in order
+    uint32_t cnt[64];             // heads per row and warp, then the heads before
+    uint32_t slot, heads;
+    uint64_t p_base;
+};
+
+// The node whose first child is at i of (codes, hash), with children below
+// `end` of the arrays: its mask and hash. Codes ascend, so a node's children
+// are in slot order.
+__device__ __forceinline__ uint64_t node_hash(const uint64_t* codes, const uint64_t* hash, uint32_t i, uint32_t end,
+                                              uint32_t* mask) {
+    const uint64_t par = codes[i] >> 3;
+    uint32_t m = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k)
+        if (i + k < end && (codes[i + k] >> 3) == par) m |= 1u << (uint32_t)(codes[i + k] & 7);
+    uint64_t h[8];
+#pragma unroll
+    for (uint32_t c = 0; c < 8; ++c) h[c] = (m >> c) & 1u ? hash[i + __popc(m & ((1u << c) - 1u))] : 0ull;
+    *mask = m;
+    return hash_children(h);
+}
+
+// What bounds it: at large levels the barriers of a tile around its look-back
+// (20 bytes read per child, 21 written per node); at small ones its chain of
+// round trips.
+__global__ void __launch_bounds__(kXThreads, 4) extract_nodes(NodesArgs a) {
+    pdl_prologue();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    NodesSmem& S = *reinterpret_cast<NodesSmem*>(smem_raw);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint64_t count = *a.d_n, n = count < a.n_bound ? count : a.n_bound;
+    if (n <= a.tail_max) return;  // the tail takes this level and those above it
+    const uint32_t ntiles = scan_tiles(n);
+    if (blockIdx.x >= ntiles) return;  // grids are sized by an upper bound on n
+    bool overflow = false;
+    while (true) {
+        if (tid == 0) S.slot = atomicAdd(a.tile_counter, 1u);
+        __syncthreads();
+        const uint32_t tile = S.slot;
+        if (tile >= ntiles) break;
+        const uint64_t base = (uint64_t)tile * kScanTile;
+        const uint32_t tile_n = (uint32_t)(n - base < (uint64_t)kScanTile ? n - base : (uint64_t)kScanTile);
+        // The tile and the few children after it that may belong to its last node.
+        const uint32_t have = (uint32_t)(n - base < (uint64_t)(kScanTile + kXHalo) ? n - base : (uint64_t)(kScanTile + kXHalo));
+        uint64_t c[kXRows], h[kXRows];
+#pragma unroll
+        for (int k = 0; k < kXRows; ++k) {
+            const uint32_t i = k * kXThreads + tid;
+            if (i < tile_n) { c[k] = a.child_codes[base + i]; h[k] = a.child_hashes[base + i]; }
+        }
+        if (tid < kXHalo && kScanTile + tid < have) {
+            S.codes[kScanTile + tid] = a.child_codes[base + kScanTile + tid];
+            S.hash[kScanTile + tid] = a.child_hashes[base + kScanTile + tid];
+        }
+        const uint64_t before = base > 0 ? a.child_codes[base - 1] >> 3 : ~0ull;
+#pragma unroll
+        for (int k = 0; k < kXRows; ++k) {
+            const uint32_t i = k * kXThreads + tid;
+            if (i < tile_n) { S.codes[i] = c[k]; S.hash[i] = h[k]; }
+        }
+        __syncthreads();
+        uint32_t heads[kXRows];
+#pragma unroll
+        for (int k = 0; k < kXRows; ++k) {
+            const uint32_t i = k * kXThreads + tid;
+            const bool head = i < tile_n && (c[k] >> 3) != (i ? S.codes[i - 1] >> 3 : before);
+            heads[k] = __ballot_sync(0xFFFFFFFFu, head);
+            if (lane == 0) S.cnt[k * kXWarps + warp] = __popc(heads[k]);
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t n0 = S.cnt[2 * lane], n1 = S.cnt[2 * lane + 1];
+            uint32_t x = n0 + n1;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                if (lane >= (uint32_t)o) x += y;
+            }
+            S.cnt[2 * lane] = x - n0 - n1;
+            S.cnt[2 * lane + 1] = x - n1;
+            const uint32_t total = __shfl_sync(0xFFFFFFFFu, x, 31);
+            if (lane == 0) S.heads = total;
+            const uint64_t pb = sv_lookback(a.status, tile, total, a.err);
+            if (lane == 0) S.p_base = pb;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kXRows; ++k)
+            if ((heads[k] >> lane) & 1u)
+                S.head[S.cnt[k * kXWarps + warp] + __popc(heads[k] & lanemask_lt())] = (uint16_t)(k * kXThreads + tid);
+        __syncthreads();
+        const uint32_t total = S.heads;
+        const uint64_t p_base = S.p_base;
+        for (uint32_t x = tid; x < total; x += kXThreads) {
+            const uint64_t p = p_base + x;
+            if (p >= a.out_capacity) { overflow = true; break; }
+            const uint32_t i = S.head[x];
+            uint32_t mask;
+            const uint64_t hv = node_hash(S.codes, S.hash, i, have, &mask);
+            a.node_codes[p] = S.codes[i] >> 3;
+            a.out.hash[p] = hv;
+            a.out.mask[p] = (uint8_t)mask;
+            a.out.first[p] = (uint32_t)(base + i);
+        }
+        if (tid == 0 && base + tile_n == n) {
+            const uint64_t cnt = p_base + total;
+            *a.d_out_n = cnt < a.out_capacity ? cnt : a.out_capacity;
+        }
+        __syncthreads();
+    }
+    if (overflow) atomicOr(a.err, kErrCapacity);
+}
+
+// ------------------------------------------------------------------- tail --
+// Children and nodes of a level in shared memory; the nodes are the next
+// level's children.
+struct TailNodesSmem {
+    uint64_t code[2][kTailCap], hash[2][kTailCap];
+    uint16_t first[kTailCap];
+    uint32_t cnt[kTailCap / 32];  // heads per row and warp
+};
+static_assert(sizeof(TailNodesSmem) <= 227 * 1024, "tail state fits one CTA's shared memory");
+constexpr int kTailRows = kTailCap / kTailThreads;
+
+// One level of at most 32 children, by one warp: a lane per child, then a lane
+// per node. Returns the number of nodes.
+__device__ __forceinline__ uint32_t tail_level_warp(TailNodesSmem& S, int from, uint32_t nc, const TailNodesLevel& out) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t* codes = S.code[from];
+    const bool head = lane < nc && (lane == 0 || (codes[lane] >> 3) != (codes[lane - 1] >> 3));
+    const uint32_t heads = __ballot_sync(0xFFFFFFFFu, head);
+    if (head) S.first[__popc(heads & lanemask_lt())] = (uint16_t)lane;
+    __syncwarp();
+    const uint32_t n = __popc(heads);
+    if (lane < n && lane < out.capacity) {
+        const uint32_t i = S.first[lane];
+        uint32_t mask;
+        const uint64_t hv = node_hash(codes, S.hash[from], i, nc, &mask);
+        S.code[from ^ 1][lane] = codes[i] >> 3;
+        S.hash[from ^ 1][lane] = hv;
+        out.out.hash[lane] = hv;
+        out.out.mask[lane] = (uint8_t)mask;
+        out.out.first[lane] = i;
+    }
+    __syncwarp();
+    return n;
+}
+
+// Bound by latency: three barriers per level, none once a level has at most 32
+// children (one warp does the rest).
+__global__ void __launch_bounds__(kTailThreads) tail_nodes(TailNodesArgs a) {
+    pdl_prologue();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TailNodesSmem& S = *reinterpret_cast<TailNodesSmem*>(smem_raw);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // The first level: the largest one whose children fit (every warp looks).
+    uint64_t cnt_l = 0;
+    if ((int)lane < a.levels) cnt_l = *a.lv[lane].d_child_n;
+    const uint32_t fit = __ballot_sync(0xFFFFFFFFu, cnt_l > 0 && cnt_l <= (uint64_t)kTailCap);
+    if (!fit) return;  // no child of any level: nothing was extracted
+    const int first = 31 - __clz(fit);
+    uint32_t nc = (uint32_t)__shfl_sync(0xFFFFFFFFu, cnt_l, first);
+    const uint64_t* gc = a.lv[first].child_codes;
+    const uint64_t* gh = a.lv[first].child_hashes;
+#pragma unroll
+    for (int k = 0; k < kTailRows; ++k) {
+        const uint32_t i = k * kTailThreads + tid;
+        if (i < nc) { S.code[0][i] = gc[i]; S.hash[0][i] = gh[i]; }
+    }
+    __syncthreads();
+    bool overflow = false;
+    int from = 0, l = first;
+    for (; l >= 0 && nc > 32; --l, from ^= 1) {
+        const TailNodesLevel& out = a.lv[l];
+        const uint64_t* codes = S.code[from];
+        uint32_t heads[kTailRows];
+#pragma unroll
+        for (int k = 0; k < kTailRows; ++k) {
+            const uint32_t i = k * kTailThreads + tid;
+            const bool head = i < nc && (i == 0 || (codes[i] >> 3) != (codes[i - 1] >> 3));
+            heads[k] = __ballot_sync(0xFFFFFFFFu, head);
+            if (lane == 0) S.cnt[k * 32 + warp] = __popc(heads[k]);
+        }
+        __syncthreads();
+        // Every warp scans the counts (kTailRows per lane, rows before warps).
+        uint32_t v[kTailRows], sum = 0;
+#pragma unroll
+        for (int q = 0; q < kTailRows; ++q) { v[q] = S.cnt[lane * kTailRows + q]; sum += v[q]; }
+        uint32_t x = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= (uint32_t)o) x += y;
+        }
+        const uint32_t n = __shfl_sync(0xFFFFFFFFu, x, 31);
+        x -= sum;
+#pragma unroll
+        for (int k = 0; k < kTailRows; ++k) {
+            // Heads before (row k, this warp): entry k * 32 + warp.
+            const uint32_t e = k * 32 + warp;
+            uint32_t before = x;
+#pragma unroll
+            for (int q = 0; q < kTailRows; ++q)
+                if ((uint32_t)q < e % kTailRows) before += v[q];
+            before = __shfl_sync(0xFFFFFFFFu, before, e / kTailRows);
+            if ((heads[k] >> lane) & 1u) S.first[before + __popc(heads[k] & lanemask_lt())] = (uint16_t)(k * kTailThreads + tid);
+        }
+        __syncthreads();
+        for (uint32_t p = tid; p < n; p += kTailThreads) {
+            if (p >= out.capacity) { overflow = true; break; }
+            const uint32_t i = S.first[p];
+            uint32_t mask;
+            const uint64_t hv = node_hash(codes, S.hash[from], i, nc, &mask);
+            S.code[from ^ 1][p] = codes[i] >> 3;
+            S.hash[from ^ 1][p] = hv;
+            out.out.hash[p] = hv;
+            out.out.mask[p] = (uint8_t)mask;
+            out.out.first[p] = i;
+        }
+        nc = n < out.capacity ? n : (uint32_t)out.capacity;
+        if (tid == 0) *out.d_nodes = nc;
+        __syncthreads();
+    }
+    if (warp == 0) {
+        for (; l >= 0; --l, from ^= 1) {
+            const TailNodesLevel& out = a.lv[l];
+            const uint32_t n = tail_level_warp(S, from, nc, out);
+            if (n > out.capacity) overflow = true;
+            nc = n < out.capacity ? n : (uint32_t)out.capacity;
+            if (lane == 0) *out.d_nodes = nc;
+        }
+    }
+    if (overflow) atomicOr(a.err, kErrCapacity);
+}
+
+// ------------------------------------------------------------------ dedup --
+// The group's levels on the device: nodes, and where each level's 128-item
+// chunks, buckets and table slots start.
+constexpr int kGIlp = 4;                  // items per lane in flight
+constexpr uint32_t kGChunk = 32 * kGIlp;  // items of a warp and round, of one level
+struct GroupSmem {
+    uint32_t n[kNodeLevels];
+    uint32_t chunk0[kNodeLevels + 1], bucket0[kNodeLevels + 1];
+    uint64_t table0[kNodeLevels + 1];
+    int shift[kNodeLevels];               // bucket of a hash: hash >> shift
+    uint32_t ok;
+};
+static_assert(kNodeLevels < 32, "a lane per level");
+
+// The whole CTA; false when the group does not fit its table or buckets (every
+// kernel of the group then returns; nodes_insert flags it).
+__device__ __forceinline__ bool load_group(const GroupDedupArgs& a, GroupSmem& G) {
+    if (threadIdx.x < 32) {
+        const uint32_t l = threadIdx.x;
+        uint64_t n = 0;
+        uint32_t nb = 0;
+        int shift = 64;
+        uint64_t slots = 0;
+        bool fits = true;
+        if ((int)l < a.levels) {
+            n = *a.lv[l].d_n;
+            if (n > a.lv[l].capacity) n = a.lv[l].capacity;
+            fits = n <= kDedupMaxItems;
+            if (n) {
+                nb = topbit_buckets(n, &shift);
+                slots = table_size_for(n, false);
+            }
+        }
+        uint32_t chunks = (uint32_t)((n + kGChunk - 1) / kGChunk), c = chunks, b = nb;
+        uint64_t t = slots;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t yc = __shfl_up_sync(0xFFFFFFFFu, c, o), yb = __shfl_up_sync(0xFFFFFFFFu, b, o);
+            const uint64_t yt = __shfl_up_sync(0xFFFFFFFFu, t, o);
+            if (l >= (uint32_t)o) { c += yc; b += yb; t += yt; }
+        }
+        if ((int)l < a.levels) {
+            G.n[l] = (uint32_t)n;
+            G.shift[l] = shift;
+            G.chunk0[l + 1] = c;
+            G.bucket0[l + 1] = b;
+            G.table0[l + 1] = t;
+        }
+        if (l == 0) { G.chunk0[0] = 0; G.bucket0[0] = 0; G.table0[0] = 0; }
+        const bool all = __all_sync(0xFFFFFFFFu, fits);
+        const uint32_t nbt = __shfl_sync(0xFFFFFFFFu, b, 31);
+        const uint64_t tt = __shfl_sync(0xFFFFFFFFu, t, 31);
+        const uint32_t ct = __shfl_sync(0xFFFFFFFFu, c, 31);
+        if (l == 0)
+            G.ok = all && tt <= a.table_cap && (uint64_t)nbt * kDedupTopBitCap <= a.bucket_area && nbt <= a.bucket_cap &&
+                   (uint64_t)ct * kGChunk <= a.slot_cap;
+    }
+    __syncthreads();
+    return G.ok != 0;
+}
+__device__ __forceinline__ int level_of_chunk(const GroupSmem& G, int levels, uint32_t c) {
+    int l = 0;
+    while (l + 1 < levels && c >= G.chunk0[l + 1]) ++l;
+    return l;
+}
+
+// Large levels are bound by the table's random accesses (a slot and the next
+// one per probe, an atomicCAS per new hash), small ones by the chain of a
+// probe, a claim and a bucket reservation. Each lane runs kGIlp probe chains
+// side by side; levels of up to 2^20 nodes claim at once (one round trip),
+// larger ones read first (L2 atomic throughput).
+__global__ void __launch_bounds__(256, 4) nodes_insert(GroupDedupArgs a) {
+    pdl_prologue();
+    __shared__ GroupSmem G;
+    if (!load_group(a, G)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.err, kErrFallback);
+        return;
+    }
+    uint32_t* aux = reinterpret_cast<uint32_t*>(a.table_aux);  // slot s: [4s] representative, [4s+1] unique id
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    bool full = false;
+    for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < G.chunk0[a.levels]; c += warps) {
+        const int l = level_of_chunk(G, a.levels, c);
+        const uint32_t n = G.n[l], i0 = (c - G.chunk0[l]) * kGChunk + lane;
+        const uint32_t S = (uint32_t)(G.table0[l + 1] - G.table0[l]);
+        uint64_t* keys = a.table_key + 2 * G.table0[l];
+        const uint64_t* hashes = a.lv[l].nodes.hash;
+        const bool read_first = n > kDedupClaimFirstMax;
+        uint64_t h[kGIlp];
+        uint32_t s[kGIlp];
+        bool pend[kGIlp], won[kGIlp];
+#pragma unroll
+        for (int k = 0; k < kGIlp; ++k) {
+            const uint32_t i = i0 + k * 32;
+            pend[k] = i < n;
+            won[k] = false;
+            h[k] = pend[k] ? hashes[i] : 0;  // hashes are never 0 (an empty slot)
+            s[k] = (uint32_t)home_slot(h[k], S);
+        }
+        for (uint32_t round = 0; round < S; ++round) {
+            bool claim[kGIlp];
+            uint64_t cur[kGIlp], nxt[kGIlp];
+#pragma unroll
+            for (int k = 0; k < kGIlp; ++k) {
+                claim[k] = pend[k];
+                cur[k] = 0;
+                nxt[k] = 0;
+            }
+            if (read_first) {
+#pragma unroll
+                for (int k = 0; k < kGIlp; ++k) {
+                    if (!pend[k]) continue;
+                    cur[k] = ld_relaxed(keys + 2ull * s[k]);
+                    nxt[k] = ld_relaxed(keys + 2ull * next_slot(s[k], S));
+                }
+                // In probe order: a match ends the search; the first empty
+                // slot is claimed; two other keys move the probe on by two.
+#pragma unroll
+                for (int k = 0; k < kGIlp; ++k) {
+                    if (!pend[k]) continue;
+                    if (cur[k] == h[k]) { pend[k] = claim[k] = false; continue; }
+                    if (cur[k] == 0) continue;
+                    s[k] = next_slot(s[k], S);
+                    if (nxt[k] == h[k]) { pend[k] = claim[k] = false; continue; }
+                    if (nxt[k] != 0) { s[k] = next_slot(s[k], S); claim[k] = false; }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kGIlp; ++k)
+                if (claim[k]) cur[k] = atomicCAS((unsigned long long*)(keys + 2ull * s[k]), 0ull, (unsigned long long)h[k]);
+            bool any = false;
+#pragma unroll
+            for (int k = 0; k < kGIlp; ++k) {
+                if (!pend[k]) continue;
+                if (claim[k] && (cur[k] == 0 || cur[k] == h[k])) { won[k] = cur[k] == 0; pend[k] = false; continue; }
+                if (claim[k]) s[k] = next_slot(s[k], S);
+                any = true;
+            }
+            if (!any) break;
+        }
+        // Every winner's bucket slot is reserved before any is used.
+        uint32_t bslot[kGIlp], b[kGIlp];
+#pragma unroll
+        for (int k = 0; k < kGIlp; ++k) {
+            b[k] = G.bucket0[l] + (G.shift[l] >= 64 ? 0u : (uint32_t)(h[k] >> G.shift[l]));
+            bslot[k] = won[k] ? atomicAdd(a.bucket_count + b[k], 1u) : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < kGIlp; ++k) {
+            const uint32_t i = i0 + k * 32;
+            if (i >= n) continue;
+            if (pend[k]) full = true;  // cannot happen at half load; rerun rather than guess
+            const uint32_t slot = (uint32_t)G.table0[l] + s[k];
+            a.item_slot[(uint64_t)G.chunk0[l] * kGChunk + i] = pend[k] ? 0xFFFFFFFFu : slot;
+            if (!won[k]) continue;
+            aux[4ull * slot] = i;
+            if (bslot[k] < kDedupTopBitCap)
+                a.bucket[(uint64_t)b[k] * kDedupTopBitCap + bslot[k]] = make_uint4((uint32_t)h[k], (uint32_t)(h[k] >> 32), slot, 0u);
+            else
+                full = true;
+        }
+    }
+    if (full) atomicOr(a.err, kErrFallback);
+}
+
+// Each CTA takes a contiguous range of the group's buckets; a bucket's keys are
+// distinct, so a key's rank is the number of smaller keys in its bucket.
+constexpr int kOThreads = 256;
+__global__ void __launch_bounds__(kOThreads) nodes_order(GroupDedupArgs a) {
+    pdl_prologue();
+    __shared__ GroupSmem G;
+    __shared__ uint64_t key[kDedupTopBitCap];
+    __shared__ uint32_t red[kOThreads / 32];
+    if (!load_group(a, G)) return;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t nb = G.bucket0[a.levels];
+    const uint32_t b0 = (uint32_t)((uint64_t)nb * blockIdx.x / gridDim.x);
+    const uint32_t b1 = (uint32_t)((uint64_t)nb * (blockIdx.x + 1) / gridDim.x);
+    if (b0 >= b1) return;
+    int l = 0;
+    while (b0 >= G.bucket0[l + 1]) ++l;
+    // Keys in the level's buckets before this range (8 independent loads per
+    // thread in flight).
+    uint32_t part = 0;
+    for (uint32_t x0 = G.bucket0[l]; x0 < b0; x0 += 8 * kOThreads) {
+        uint32_t c[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const uint32_t x = x0 + u * kOThreads + tid;
+            c[u] = x < b0 ? a.bucket_count[x] : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) part += min(c[u], kDedupTopBitCap);
+    }
+    part = __reduce_add_sync(0xFFFFFFFFu, part);
+    if (lane == 0) red[warp] = part;
+    __syncthreads();
+    uint64_t start = 0;
+    for (int w = 0; w < kOThreads / 32; ++w) start += red[w];
+    uint32_t* aux = reinterpret_cast<uint32_t*>(a.table_aux);
+    bool bad = false;
+    for (uint32_t b = b0; b < b1; ++b) {
+        while (b >= G.bucket0[l + 1]) { ++l; start = 0; }
+        const GroupLevel& lv = a.lv[l];
+        const uint32_t cnt = min(a.bucket_count[b], kDedupTopBitCap);
+        const uint4* ent = a.bucket + (uint64_t)b * kDedupTopBitCap;
+        __syncthreads();  // the previous bucket's keys are no longer read
+        for (uint32_t j = tid; j < cnt; j += kOThreads) {
+            const uint4 e = ent[j];
+            key[j] = (uint64_t)e.x | (uint64_t)e.y << 32;
+        }
+        __syncthreads();
+        for (uint32_t j = tid; j < cnt; j += kOThreads) {
+            const uint32_t s = ent[j].z;
+            const uint64_t k = key[j];
+            uint32_t r = 0;
+#pragma unroll 8
+            for (uint32_t x = 0; x < cnt; ++x) r += key[x] < k;
+            const uint64_t uid = start + r;
+            if (uid < lv.capacity && s < a.table_cap) {
+                lv.out_keys[uid] = k;
+                aux[4ull * s + 1] = (uint32_t)uid;
+                a.table_key[2ull * s] = 0;  // empty for the next group (nodes_finish reads only aux)
+            } else {
+                bad = true;
+            }
+        }
+        start += cnt;
+        if (tid == 0 && b + 1 == G.bucket0[l + 1]) {  // the level's last bucket
+            if (start > a.uniq_cap) atomicOr(a.err, kErrFallback);
+            *lv.d_out_n = start < lv.capacity ? start : lv.capacity;
+        }
+    }
+    if (bad) atomicOr(a.err, kErrCapacity);
+}
+
+// A node's child ids by slot (the children are consecutive items of the level
+// below): of the group's lowest level through the map of the level below it,
+// else through the table.
+__device__ __forceinline__ void child_ids(const GroupDedupArgs& a, const GroupSmem& G, int l, uint32_t mask, uint32_t first,
+                                          uint32_t (&id)[8]) {
+    if (l + 1 == a.levels) {
+#pragma unroll
+        for (uint32_t c = 0; c < 8; ++c) {
+            id[c] = kEmptyChild;
+            if ((mask >> c) & 1u) id[c] = a.child_map[(uint64_t)first + __popc(mask & ((1u << c) - 1u))];
+        }
+        return;
+    }
+    const uint32_t* slots = a.item_slot + (uint64_t)G.chunk0[l + 1] * kGChunk;
+    uint32_t s[8];
+#pragma unroll
+    for (uint32_t c = 0; c < 8; ++c)
+        s[c] = (mask >> c) & 1u ? slots[first + __popc(mask & ((1u << c) - 1u))] : 0xFFFFFFFFu;
+#pragma unroll
+    for (uint32_t c = 0; c < 8; ++c)
+        id[c] = s[c] < a.table_cap ? reinterpret_cast<const uint32_t*>(a.table_aux)[4ull * s[c] + 1] : kEmptyChild;
+}
+
+// Bound by random reads: per node its slot's aux word and, as somebody's child,
+// one more. (Each node is a child once, so no map of a level is needed but for
+// the group above.)
+__global__ void __launch_bounds__(256) nodes_finish(GroupDedupArgs a) {
+    pdl_prologue();
+    __shared__ GroupSmem G;
+    if (!load_group(a, G)) return;
+    // The bucket counters, read by nodes_order, start the next group at zero.
+    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < G.bucket0[a.levels]; b += gridDim.x * blockDim.x)
+        a.bucket_count[b] = 0;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    bool collision = false;
+    for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < G.chunk0[a.levels]; c += warps) {
+        const int l = level_of_chunk(G, a.levels, c);
+        const GroupLevel& lv = a.lv[l];
+        const uint32_t n = G.n[l], i0 = (c - G.chunk0[l]) * kGChunk + lane;
+        const uint32_t* slots = a.item_slot + (uint64_t)G.chunk0[l] * kGChunk;
+        uint32_t s[kGIlp], mask[kGIlp], first[kGIlp];
+        uint64_t aux[kGIlp];
+#pragma unroll
+        for (int k = 0; k < kGIlp; ++k) {
+            const uint32_t i = i0 + k * 32;
+            s[k] = i < n ? slots[i] : 0xFFFFFFFFu;
+            mask[k] = i < n ? lv.nodes.mask[i] : 0u;
+            first[k] = i < n ? lv.nodes.first[i] : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < kGIlp; ++k) aux[k] = s[k] < a.table_cap ? a.table_aux[2ull * s[k]] : ~0ull;
+#pragma unroll
+        for (int k = 0; k < kGIlp; ++k) {
+            const uint32_t i = i0 + k * 32, rep = (uint32_t)aux[k], uid = (uint32_t)(aux[k] >> 32);
+            if (i >= n) continue;
+            // Ids stay inside the next level's arrays even when a fallback or
+            // an error discards this call.
+            if (l == 0 && a.map) a.map[i] = uid < lv.capacity ? uid : (uint32_t)(lv.capacity - 1);
+            if (s[k] >= a.table_cap || rep >= n || uid >= lv.capacity) continue;  // flagged by the insert or the order
+            uint32_t id[8];
+            child_ids(a, G, l, mask[k], first[k], id);
+            if (rep == i) {
+                lv.out_masks[uid] = (uint8_t)mask[k];
+                uint4* d4 = reinterpret_cast<uint4*>(lv.out_children + (uint64_t)uid * 8);
+                d4[0] = make_uint4(id[0], id[1], id[2], id[3]);
+                d4[1] = make_uint4(id[4], id[5], id[6], id[7]);
+            } else {
+                uint32_t other[8];
+                const uint32_t m = lv.nodes.mask[rep];
+                child_ids(a, G, l, m, lv.nodes.first[rep], other);
+                collision |= m != mask[k];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) collision |= id[q] != other[q];
+            }
+        }
+    }
+    if (collision) atomicOr(a.err, kErrCollision);
+}
+
+int g_levels_sms = 152, g_extract_ctas = 4;
+
+}  // namespace
+
+void levels_configure(int sms) {
+    g_levels_sms = sms > 0 ? sms : 152;
+    cudaFuncSetAttribute(extract_nodes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NodesSmem));
+    cudaFuncSetAttribute(tail_nodes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TailNodesSmem));
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, extract_nodes, kXThreads, sizeof(NodesSmem)) != cudaSuccess)
+        cudaGetLastError();
+    g_extract_ctas = occ > 0 ? occ : 1;
+}
+
+uint64_t group_slot_items(uint64_t n) { return (n + kGChunk - 1) / kGChunk * kGChunk; }
+
+void launch_extract_nodes(const NodesArgs& a, cudaStream_t s) {
+    const uint64_t tiles = scan_tiles(a.n_bound), most = (uint64_t)g_extract_ctas * g_levels_sms;
+    launch_pdl(extract_nodes, dim3((unsigned)(tiles < most ? (tiles ? tiles : 1) : most)), dim3(kXThreads), sizeof(NodesSmem), s, a);
+}
+void launch_tail_nodes(const TailNodesArgs& a, cudaStream_t s) {
+    launch_pdl(tail_nodes, dim3(1), dim3(kTailThreads), sizeof(TailNodesSmem), s, a);
+}
+int launch_group_dedup(const GroupDedupArgs& a, uint64_t items_bound, cudaStream_t s) {
+    const uint64_t want = (items_bound + 255) / 256, most = 8ull * g_levels_sms;
+    const unsigned g = (unsigned)(want < most ? (want ? want : 1) : most);
+    launch_pdl(nodes_insert, dim3(g), dim3(256), 0, s, a);
+    const uint64_t buckets = items_bound / 128 + a.levels;
+    launch_pdl(nodes_order, dim3((unsigned)(buckets < most ? buckets : most)), dim3(kOThreads), 0, s, a);
+    launch_pdl(nodes_finish, dim3(g), dim3(256), 0, s, a);
+    return 3;
+}
+
+}  // namespace dagc
