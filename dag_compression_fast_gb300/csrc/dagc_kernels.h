@@ -431,6 +431,9 @@ struct TraceArgs {
     const uint32_t* words; uint64_t n_words; int depth;
     uint32_t debug_level, width, height;
     double camera[3], ray_min[3], ray_ddx[3], ray_ddy[3];
+    // ray_min - camera, ray_ddx and ray_ddy as float32 pairs, and a bound of
+    // what makes up a ray's components (set by launch_trace).
+    float base[6], ddx[6], ddy[6], magnitude;
     uint32_t* colors;  // width * height, row-major
     uint64_t* hits;    // optional: Morton code of the voxel hit, ~0 for a miss
     uint32_t* err;

@@ -14,12 +14,23 @@
 // every operation is one IEEE rounding and the result is reproducible on the
 // CPU.
 //
+// A ray's direction is normalised in float64 (the rule), of which this part
+// does 2 operations per SM and clock. It is computed in pairs of float32
+// instead, with an error bound, and only where a float32 rounding lies within
+// the bound does the float64 form decide (ray_direction). The rest is bound by
+// the instructions of a step (3300 per warp, half of them compares and selects
+// on the ALU pipe, 23 of 32 lanes busy) and the last rays of a frame.
+// 1920x1080 on the 2048^3 terrain: 337 us with float64 throughout, now 309.
+//
 // Reads of the word array are bounds-checked and each ray stops after
 // kTraceMaxSteps descents: a malformed array sets kErrBadInput, never a read
 // outside it.
 
 #include "dagc_device.cuh"
 #include "dagc_kernels.h"
+
+#include <algorithm>
+#include <cmath>
 
 namespace dagc {
 namespace {
@@ -89,6 +100,66 @@ __device__ __forceinline__ uint64_t pack(uint32_t index, uint32_t cm, uint32_t v
     return (uint64_t)index | (uint64_t)cm << 32 | (uint64_t)vm << 40;
 }
 
+// ------------------------------------------------ pairs of float32 values ----
+// hi + lo, |lo| <= ulp(hi) / 2: the usual error-free sums and products (Dekker
+// 1971, Knuth) with fmaf.
+struct F2 { float hi, lo; };
+__device__ __forceinline__ F2 quick_sum(float a, float b) { const float s = a + b; return {s, b - (s - a)}; }  // |a| >= |b|
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+    const float s = a.hi + b.hi, t = s - a.hi;
+    const float e = (a.hi - (s - t)) + (b.hi - t);
+    return quick_sum(s, e + (a.lo + b.lo));
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+    const float p = a.hi * b.hi, e = fmaf(a.hi, b.hi, -p);
+    return quick_sum(p, fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, e)));
+}
+__device__ __forceinline__ F2 f2_scale(F2 a, float b) {
+    const float p = a.hi * b;
+    return quick_sum(p, fmaf(a.lo, b, fmaf(a.hi, b, -p)));
+}
+
+// The rule (src/DAGTracer.cu:310-318): direction normalised in double, then float.
+__device__ __noinline__ float3 ray_direction_exact(const TraceArgs& a, uint32_t px, uint32_t py) {
+    const double vx = a.ray_min[0] + double(px) * a.ray_ddx[0] + double(py) * a.ray_ddy[0] - a.camera[0];
+    const double vy = a.ray_min[1] + double(px) * a.ray_ddx[1] + double(py) * a.ray_ddy[1] - a.camera[1];
+    const double vz = a.ray_min[2] + double(px) * a.ray_ddx[2] + double(py) * a.ray_ddy[2] - a.camera[2];
+    const double s = 1 / sqrt(vx * vx + vy * vy + vz * vz);
+    return make_float3(float(s * vx), float(s * vy), float(s * vz));
+}
+
+// The same value. With T a bound of the magnitudes that make up a component of
+// v (so that the rule's v is off by less than 2^-50 T), the pairs hold v to
+// 2^-45 T, its square sum and the reciprocal root to relative
+// 2^-44 + 2^-44 T/|v|, and so the direction to 2^-42.5 T/|v|. A component whose
+// rounding to float32 is the same on both sides of 2^-41 T/|v| is the rule's.
+__device__ __forceinline__ float3 ray_direction(const TraceArgs& a, uint32_t px, uint32_t py) {
+    const float x = (float)px, y = (float)py, T = a.magnitude;
+    F2 v[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        v[k] = f2_add(f2_add({a.base[2 * k], a.base[2 * k + 1]}, f2_scale({a.ddx[2 * k], a.ddx[2 * k + 1]}, x)),
+                      f2_scale({a.ddy[2 * k], a.ddy[2 * k + 1]}, y));
+    const F2 n2 = f2_add(f2_add(f2_mul(v[0], v[0]), f2_mul(v[1], v[1])), f2_mul(v[2], v[2]));
+    // 1 / sqrt(n2): the approximation r0 (error below 2^-21), then
+    // r0 * (1 + d / 2 + 3 d^2 / 8) with d = 1 - n2 * r0^2.
+    const float r0 = rsqrtf(n2.hi);
+    const F2 t = f2_mul(n2, f2_mul({r0, 0.0f}, {r0, 0.0f}));
+    const float d = (1.0f - t.hi) - t.lo;
+    const F2 r = quick_sum(r0, r0 * d * fmaf(0.375f, d, 0.5f));
+    const float err = 0x1p-41f * T * r0;
+    float out[3];
+    bool sure = T > 0.0f && n2.hi >= T * T * 0x1p-24f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const F2 c = f2_mul(v[k], r);
+        out[k] = c.hi;
+        sure = sure && c.hi + (c.lo + err) == c.hi && c.hi + (c.lo - err) == c.hi;
+    }
+    if (!sure) return ray_direction_exact(a, px, py);
+    return make_float3(out[0], out[1], out[2]);
+}
+
 __global__ void __launch_bounds__(128) trace_rays(TraceArgs a) {
     const uint32_t px = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t py = blockIdx.y * blockDim.y + threadIdx.y;
@@ -102,14 +173,12 @@ __global__ void __launch_bounds__(128) trace_rays(TraceArgs a) {
         return __ldg(w + i);
     };
 
-    // Ray: direction normalised in double, then float (src/DAGTracer.cu:310-318).
-    const double vx = a.ray_min[0] + double(px) * a.ray_ddx[0] + double(py) * a.ray_ddy[0] - a.camera[0];
-    const double vy = a.ray_min[1] + double(px) * a.ray_ddx[1] + double(py) * a.ray_ddy[1] - a.camera[1];
-    const double vz = a.ray_min[2] + double(px) * a.ray_ddx[2] + double(py) * a.ray_ddy[2] - a.camera[2];
-    const double s = 1 / sqrt(vx * vx + vy * vy + vz * vz);
     const float3 org = make_float3(float(a.camera[0]), float(a.camera[1]), float(a.camera[2]));
-    const float3 dir = make_float3(float(s * vx), float(s * vy), float(s * vz));
-    const float3 inv = make_float3(float(1. / double(dir.x)), float(1. / double(dir.y)), float(1. / double(dir.z)));
+    const float3 dir = ray_direction(a, px, py);
+    // 1 / double(dir), rounded to float: the float32 quotient is the same (a
+    // double holds more than twice a float's bits, and no quotient of a
+    // component below 2 is subnormal).
+    const float3 inv = make_float3(__frcp_rn(dir.x), __frcp_rn(dir.y), __frcp_rn(dir.z));
     const uint32_t order = (dir.x < 0.f ? 4u : 0u) + (dir.y < 0.f ? 2u : 0u) + (dir.z < 0.f ? 1u : 0u);
 
     uint64_t stack[kTraceMaxDepth];
@@ -141,9 +210,11 @@ __global__ void __launch_bounds__(128) trace_rays(TraceArgs a) {
         level = nl;
         // Next child in the ray's order: the first set bit of vm after
         // relabelling the children by child ^ order.
-        uint32_t child = 0;
-        for (uint32_t c = 0; c < 8; ++c)
-            if (vm & (1u << (c ^ order))) { child = c ^ order; break; }
+        uint32_t seen = vm;
+        if (order & 1u) seen = ((seen & 0x55u) << 1) | ((seen >> 1) & 0x55u);
+        if (order & 2u) seen = ((seen & 0x33u) << 2) | ((seen >> 2) & 0x33u);
+        if (order & 4u) seen = ((seen & 0x0Fu) << 4) | (seen >> 4);
+        const uint32_t child = (uint32_t)(__ffs(seen) - 1) ^ order;
         vm &= ~(1u << child);
         path[0] = (path[0] << 1) | ((child >> 2) & 1u);
         path[1] = (path[1] << 1) | ((child >> 1) & 1u);
@@ -192,7 +263,26 @@ __global__ void __launch_bounds__(128) trace_rays(TraceArgs a) {
 
 }  // namespace
 
-void launch_trace(const TraceArgs& a, cudaStream_t s) {
+void launch_trace(const TraceArgs& args, cudaStream_t s) {
+    // The direction's float32 pairs; magnitude 0 (float64 for every ray) where
+    // they would leave the range in which float32 products are exact.
+    TraceArgs a = args;
+    double most = 0.0;
+    bool finite = true;
+    for (int k = 0; k < 3; ++k) {
+        const double v[3] = {a.ray_min[k] - a.camera[k], a.ray_ddx[k], a.ray_ddy[k]};
+        float* to[3] = {a.base + 2 * k, a.ddx + 2 * k, a.ddy + 2 * k};
+        for (int q = 0; q < 3; ++q) {
+            finite = finite && std::fabs(v[q]) < 1e15;
+            to[q][0] = (float)v[q];
+            to[q][1] = (float)(v[q] - (double)to[q][0]);
+        }
+        most = std::max(most, std::fabs(a.ray_min[k]) + std::fabs(a.camera[k]) + a.width * std::fabs(v[1]) +
+                                  a.height * std::fabs(v[2]));
+    }
+    a.magnitude = finite && most > 1e-6 && most < 1e15 && a.width < (1u << 24) && a.height < (1u << 24)
+                      ? (float)(most * 1.0001)
+                      : 0.0f;
     const dim3 block(8, 16);
     const dim3 grid((a.width + block.x - 1) / block.x, (a.height + block.y - 1) / block.y);
     trace_rays<<<grid, block, 0, s>>>(a);
