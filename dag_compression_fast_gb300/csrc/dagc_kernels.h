@@ -369,6 +369,9 @@ struct NodeArrays {
     uint64_t* hash;
     uint8_t* mask;     // children present
     uint32_t* first;   // index of the first child among the level below's nodes (or bricks); the others follow it
+    // Or (first null; the union of several DAGs): all eight children as indices
+    // among the level below's items, kEmptyChild where there is none.
+    uint32_t* children;
 };
 struct NodesArgs {
     const uint64_t* child_codes; const uint64_t* child_hashes;  // of every child (not only the distinct ones)
@@ -410,6 +413,24 @@ struct GroupDedupArgs {
     uint64_t uniq_cap;
     uint32_t* err;
 };
+// Union of several DAGs: their levels' nodes and leaves one after another, as
+// the items of the leaf dedup and of launch_group_dedup.
+struct MergeArgs {
+    uint32_t k; int levels;          // inputs, node levels
+    // Per input: hashes, children, masks, leaves (device pointers), all inputs'
+    // hashes first; then per input and level the level's first node; then per
+    // level (the leaves last) and input, k + 1 each: its first item.
+    const uint64_t* table;
+    uint64_t level0[kNodeLevels + 2];   // items before each level (the leaves after the last; then the total)
+    NodeArrays out[kNodeLevels];
+    uint64_t* leaves;
+    uint64_t* d_n[kNodeLevels + 1];     // item counts to set: levels, then leaves
+    // Roots: the map of level 0 (or of the leaves), then per input its root's id and hash.
+    const uint32_t* root_map; uint32_t* root_uid; uint64_t* root_hash;
+    uint32_t* err;
+};
+void launch_merge_gather(const MergeArgs& a, cudaStream_t s);
+void launch_merge_roots(const MergeArgs& a, cudaStream_t s);
 void levels_configure(int sms);
 uint64_t group_slot_items(uint64_t n);  // item_slot entries of a level of n nodes
 int launch_group_dedup(const GroupDedupArgs& a, uint64_t items_bound, cudaStream_t s);  // returns the number of launches

@@ -523,24 +523,34 @@ __global__ void __launch_bounds__(kOThreads) nodes_order(GroupDedupArgs a) {
     if (bad) atomicOr(a.err, kErrCapacity);
 }
 
-// A node's child ids by slot (the children are consecutive items of the level
-// below): of the group's lowest level through the map of the level below it,
-// else through the table.
-__device__ __forceinline__ void child_ids(const GroupDedupArgs& a, const GroupSmem& G, int l, uint32_t mask, uint32_t first,
+// A node's child ids by slot, of the items below it: through the map of the
+// level below the group for its lowest level, else through the table. The
+// children are consecutive items, or (kRefs) any.
+template <bool kRefs>
+__device__ __forceinline__ void child_ids(const GroupDedupArgs& a, const GroupSmem& G, int l, uint32_t i, uint32_t mask,
                                           uint32_t (&id)[8]) {
+    const NodeArrays& nodes = a.lv[l].nodes;
+    uint32_t item[8];
+    if (kRefs) {
+        const uint4* p = reinterpret_cast<const uint4*>(nodes.children + (uint64_t)i * 8);
+        const uint4 c0 = p[0], c1 = p[1];
+        item[0] = c0.x; item[1] = c0.y; item[2] = c0.z; item[3] = c0.w;
+        item[4] = c1.x; item[5] = c1.y; item[6] = c1.z; item[7] = c1.w;
+    } else {
+        const uint32_t first = nodes.first[i];
+#pragma unroll
+        for (uint32_t c = 0; c < 8; ++c)
+            item[c] = (mask >> c) & 1u ? first + __popc(mask & ((1u << c) - 1u)) : kEmptyChild;
+    }
     if (l + 1 == a.levels) {
 #pragma unroll
-        for (uint32_t c = 0; c < 8; ++c) {
-            id[c] = kEmptyChild;
-            if ((mask >> c) & 1u) id[c] = a.child_map[(uint64_t)first + __popc(mask & ((1u << c) - 1u))];
-        }
+        for (uint32_t c = 0; c < 8; ++c) id[c] = item[c] != kEmptyChild ? a.child_map[item[c]] : kEmptyChild;
         return;
     }
     const uint32_t* slots = a.item_slot + (uint64_t)G.chunk0[l + 1] * kGChunk;
     uint32_t s[8];
 #pragma unroll
-    for (uint32_t c = 0; c < 8; ++c)
-        s[c] = (mask >> c) & 1u ? slots[first + __popc(mask & ((1u << c) - 1u))] : 0xFFFFFFFFu;
+    for (uint32_t c = 0; c < 8; ++c) s[c] = item[c] != kEmptyChild ? slots[item[c]] : 0xFFFFFFFFu;
 #pragma unroll
     for (uint32_t c = 0; c < 8; ++c)
         id[c] = s[c] < a.table_cap ? reinterpret_cast<const uint32_t*>(a.table_aux)[4ull * s[c] + 1] : kEmptyChild;
@@ -549,6 +559,7 @@ __device__ __forceinline__ void child_ids(const GroupDedupArgs& a, const GroupSm
 // Bound by random reads: per node its slot's aux word and, as somebody's child,
 // one more. (Each node is a child once, so no map of a level is needed but for
 // the group above.)
+template <bool kRefs>
 __global__ void __launch_bounds__(256) nodes_finish(GroupDedupArgs a) {
     pdl_prologue();
     __shared__ GroupSmem G;
@@ -564,14 +575,13 @@ __global__ void __launch_bounds__(256) nodes_finish(GroupDedupArgs a) {
         const GroupLevel& lv = a.lv[l];
         const uint32_t n = G.n[l], i0 = (c - G.chunk0[l]) * kGChunk + lane;
         const uint32_t* slots = a.item_slot + (uint64_t)G.chunk0[l] * kGChunk;
-        uint32_t s[kGIlp], mask[kGIlp], first[kGIlp];
+        uint32_t s[kGIlp], mask[kGIlp];
         uint64_t aux[kGIlp];
 #pragma unroll
         for (int k = 0; k < kGIlp; ++k) {
             const uint32_t i = i0 + k * 32;
             s[k] = i < n ? slots[i] : 0xFFFFFFFFu;
             mask[k] = i < n ? lv.nodes.mask[i] : 0u;
-            first[k] = i < n ? lv.nodes.first[i] : 0u;
         }
 #pragma unroll
         for (int k = 0; k < kGIlp; ++k) aux[k] = s[k] < a.table_cap ? a.table_aux[2ull * s[k]] : ~0ull;
@@ -584,7 +594,7 @@ __global__ void __launch_bounds__(256) nodes_finish(GroupDedupArgs a) {
             if (l == 0 && a.map) a.map[i] = uid < lv.capacity ? uid : (uint32_t)(lv.capacity - 1);
             if (s[k] >= a.table_cap || rep >= n || uid >= lv.capacity) continue;  // flagged by the insert or the order
             uint32_t id[8];
-            child_ids(a, G, l, mask[k], first[k], id);
+            child_ids<kRefs>(a, G, l, i, mask[k], id);
             if (rep == i) {
                 lv.out_masks[uid] = (uint8_t)mask[k];
                 uint4* d4 = reinterpret_cast<uint4*>(lv.out_children + (uint64_t)uid * 8);
@@ -593,7 +603,7 @@ __global__ void __launch_bounds__(256) nodes_finish(GroupDedupArgs a) {
             } else {
                 uint32_t other[8];
                 const uint32_t m = lv.nodes.mask[rep];
-                child_ids(a, G, l, m, lv.nodes.first[rep], other);
+                child_ids<kRefs>(a, G, l, rep, m, other);
                 collision |= m != mask[k];
 #pragma unroll
                 for (int q = 0; q < 8; ++q) collision |= id[q] != other[q];
@@ -601,6 +611,75 @@ __global__ void __launch_bounds__(256) nodes_finish(GroupDedupArgs a) {
         }
     }
     if (collision) atomicOr(a.err, kErrCollision);
+}
+
+// ------------------------------------------------------------------ union --
+// The input of item j (off ascending, k + 1 entries).
+__device__ __forceinline__ uint32_t input_of(const uint64_t* off, uint32_t k, uint64_t j) {
+    uint32_t lo = 0, hi = k;  // off[lo] <= j < off[hi]
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (__ldg(off + mid) <= j) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+struct MergeTable {
+    const uint64_t *hashes, *children, *masks, *leaves, *first, *item;
+    __device__ explicit MergeTable(const MergeArgs& a)
+        : hashes(a.table), children(a.table + a.k), masks(a.table + 2ull * a.k), leaves(a.table + 3ull * a.k),
+          first(a.table + 4ull * a.k), item(a.table + (4ull + a.levels) * a.k) {}
+    __device__ const uint64_t* items(const MergeArgs& a, int l) const { return item + (uint64_t)l * (a.k + 1); }
+};
+
+// Every node of every input: hash and mask as they are, children as items of
+// the level below. A hash or leaf of 0 would mark an empty slot of the table:
+// those go to the radix form.
+__global__ void __launch_bounds__(256) merge_gather(MergeArgs a) {
+    pdl_prologue();
+    const MergeTable t(a);
+    if (blockIdx.x == 0 && (int)threadIdx.x <= a.levels) *a.d_n[threadIdx.x] = a.level0[threadIdx.x + 1] - a.level0[threadIdx.x];
+    const uint64_t total = a.level0[a.levels + 1];
+    bool zero = false;
+    for (uint64_t g = (uint64_t)blockIdx.x * 256 + threadIdx.x; g < total; g += (uint64_t)gridDim.x * 256) {
+        int l = 0;
+        while (l < a.levels && g >= a.level0[l + 1]) ++l;
+        const uint64_t j = g - a.level0[l];
+        const uint64_t* off = t.items(a, l);
+        const uint32_t i = input_of(off, a.k, j);
+        const uint64_t r = j - __ldg(off + i);
+        if (l == a.levels) {
+            const uint64_t leaf = reinterpret_cast<const uint64_t*>(__ldg(t.leaves + i))[r];
+            a.leaves[j] = leaf;
+            zero |= leaf == 0;
+            continue;
+        }
+        const uint64_t src = __ldg(t.first + (uint64_t)i * a.levels + l) + r;
+        const uint32_t below = (uint32_t)__ldg(t.items(a, l + 1) + i);
+        const uint64_t h = reinterpret_cast<const uint64_t*>(__ldg(t.hashes + i))[src];
+        const uint4* c = reinterpret_cast<const uint4*>(__ldg(t.children + i)) + 2 * src;
+        uint4 c0 = c[0], c1 = c[1];
+        auto up = [&](uint32_t& x) { if (x != kEmptyChild) x += below; };
+        up(c0.x); up(c0.y); up(c0.z); up(c0.w);
+        up(c1.x); up(c1.y); up(c1.z); up(c1.w);
+        a.out[l].hash[j] = h;
+        a.out[l].mask[j] = reinterpret_cast<const uint8_t*>(__ldg(t.masks + i))[src];
+        uint4* d = reinterpret_cast<uint4*>(a.out[l].children + 8 * j);
+        d[0] = c0;
+        d[1] = c1;
+        zero |= h == 0;
+    }
+    if (zero) atomicOr(a.err, kErrFallback);
+}
+
+__global__ void __launch_bounds__(256) merge_roots(MergeArgs a) {
+    pdl_prologue();
+    const MergeTable t(a);
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < a.k; i += gridDim.x * 256) {
+        const uint64_t j = t.items(a, 0)[i];
+        const bool any = t.items(a, 0)[i + 1] > j;
+        a.root_uid[i] = any ? a.root_map[j] : kEmptyChild;
+        a.root_hash[i] = any ? (a.levels ? a.out[0].hash[j] : a.leaves[j]) : 0ull;
+    }
 }
 
 int g_levels_sms = 152, g_extract_ctas = 4;
@@ -632,8 +711,17 @@ int launch_group_dedup(const GroupDedupArgs& a, uint64_t items_bound, cudaStream
     launch_pdl(nodes_insert, dim3(g), dim3(256), 0, s, a);
     const uint64_t buckets = items_bound / 128 + a.levels;
     launch_pdl(nodes_order, dim3((unsigned)(buckets < most ? buckets : most)), dim3(kOThreads), 0, s, a);
-    launch_pdl(nodes_finish, dim3(g), dim3(256), 0, s, a);
+    if (a.lv[0].nodes.children) launch_pdl(nodes_finish<true>, dim3(g), dim3(256), 0, s, a);
+    else launch_pdl(nodes_finish<false>, dim3(g), dim3(256), 0, s, a);
     return 3;
+}
+
+void launch_merge_gather(const MergeArgs& a, cudaStream_t s) {
+    const uint64_t want = (a.level0[a.levels + 1] + 255) / 256, most = 8ull * g_levels_sms;
+    launch_pdl(merge_gather, dim3((unsigned)(want < most ? (want ? want : 1) : most)), dim3(256), 0, s, a);
+}
+void launch_merge_roots(const MergeArgs& a, cudaStream_t s) {
+    launch_pdl(merge_roots, dim3((a.k + 255) / 256), dim3(256), 0, s, a);
 }
 
 }  // namespace dagc
