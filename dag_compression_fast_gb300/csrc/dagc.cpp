@@ -812,7 +812,7 @@ struct LevelGroups {
             while (lo > 0 && (lo == hi + 1 || sum + items[lo - 1] <= kGroupItems)) {
                 --lo;
                 sum += items[lo];
-                slots += table_size_for(items[lo], false);
+                slots += node_slots_upto(items[lo]);
                 buckets += node_buckets_upto(items[lo]);
                 places += group_slot_items(items[lo]);
             }
@@ -878,7 +878,7 @@ struct CreateLayout {
             for (int l = 0; l < nl; ++l) items[l] = items_of(l);
             LevelGroups G(items);
             groups = std::move(G.groups);
-            table_slots = std::max(table_slots_upto(item_cap), G.table_slots);
+            table_slots = std::max(leaf_slots_upto(item_cap), G.table_slots);
             bucket_cap = G.bucket_cap;
             slot_cap = G.slot_cap;
             bucket_area = bucket_cap * kDedupTopBitCap;
@@ -2039,7 +2039,7 @@ int union_hash(dagc_context ctx, dagc_dag* in, uint64_t k_all, cudaStream_t s, u
     const size_t o_root_hash = L.take<uint64_t>(k), o_root_uid = L.take<uint32_t>(k);
     DAGC_CUDA(ctx, ctx->arena.reserve(L.off));
     arena_wait(ctx, s);
-    int st = reserve_table(ctx, std::max(table_slots_upto(total_leaves), G.table_slots), s, false);
+    int st = reserve_table(ctx, std::max(leaf_slots_upto(total_leaves), G.table_slots), s, false);
     if (st) return st;
     for (uint32_t j = 0; j < k; ++j) dag_ready_wait(in[live[j]], s);
     char* b = static_cast<char*>(ctx->arena.base);

@@ -306,20 +306,29 @@ DAGC_HD uint64_t node_buckets_upto(uint64_t n) {
 // table is in the L2 anyway and the insert's time is its longest probe chain, a
 // round trip per two slots: 4 n slots (25k distinct masks of 36k bricks: the
 // insert takes 12 us, 25 with 1.25 n). Node hashes are about half distinct
-// and each probe step is a dependent round trip: kNodeTableQuarters / 4 * n
-// slots keep the load low. At least 1024 slots, a multiple of 32.
-constexpr uint64_t kNodeTableQuarters = 8;
+// and each probe step is a dependent round trip: 2 n slots at sizes beyond the
+// L2, where emptier tables cost more than they save, 4 n and 8 n below
+// (kNodeSparseMax, kNodeEmptyMax nodes; 12k nodes of a 512^3 terrain: the
+// insert takes 10 us, 29 with 2 n). At least 1024 slots, a multiple of 32.
 constexpr uint64_t kLeafSparseMax = 1ull << 20;
+constexpr uint64_t kNodeSparseMax = 1ull << 20, kNodeEmptyMax = 1ull << 17;
 DAGC_HD uint64_t table_size_for(uint64_t n, bool leaf_masks) {
-    const uint64_t want = !leaf_masks ? n * kNodeTableQuarters / 4 : n <= kLeafSparseMax ? 4 * n : n + (n >> 2);
+    const uint64_t want = leaf_masks ? (n <= kLeafSparseMax ? 4 * n : n + (n >> 2))
+                                     : (n <= kNodeEmptyMax ? 8 * n : n <= kNodeSparseMax ? 4 * n : 2 * n);
     return want < 1024 ? 1024 : (want + 31) & ~31ull;
 }
-// Slots that hold any count of up to `items` items of either kind.
-DAGC_HD uint64_t table_slots_upto(uint64_t items) {
+// Slots that hold any count of up to `items` items.
+DAGC_HD uint64_t node_slots_upto(uint64_t items) {
+    uint64_t most = table_size_for(items, false);
+    const uint64_t a = table_size_for(items < kNodeEmptyMax ? items : kNodeEmptyMax, false);
+    const uint64_t b = table_size_for(items < kNodeSparseMax ? items : kNodeSparseMax, false);
+    if (a > most) most = a;
+    return b > most ? b : most;
+}
+DAGC_HD uint64_t leaf_slots_upto(uint64_t items) {
     const uint64_t sparse = table_size_for(items < kLeafSparseMax ? items : kLeafSparseMax, true);
-    const uint64_t leaf = table_size_for(items, true), node = table_size_for(items, false);
-    const uint64_t most = leaf > node ? leaf : node;
-    return most > sparse ? most : sparse;
+    const uint64_t all = table_size_for(items, true);
+    return all > sparse ? all : sparse;
 }
 struct DedupState {
     unsigned long long u;  // distinct keys found (zero on entry)
@@ -409,7 +418,7 @@ struct GroupDedupArgs {
     uint64_t* table_key; uint64_t* table_aux; uint64_t table_cap;  // as DedupArgs
     uint32_t* item_slot; uint64_t slot_cap;
     uint32_t* bucket_count; uint32_t bucket_cap;                   // zero on entry and exit
-    uint4* bucket; uint64_t bucket_area;                           // kDedupTopBitCap entries each: key (two words), slot
+    uint4* bucket; uint64_t bucket_area;                           // kDedupTopBitCap entries each: key (two words), slot, representative
     uint64_t uniq_cap;
     uint32_t* err;
 };
