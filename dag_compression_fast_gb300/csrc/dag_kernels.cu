@@ -692,7 +692,21 @@ struct FinalLevels {
 __device__ __forceinline__ void load_levels(const FinalArgs& a, FinalLevels& L) {
     const int t = threadIdx.x;
     if (t < a.num_levels) { L.masks[t] = a.lv_masks[t]; L.children[t] = a.lv_children[t]; }
-    if (t <= a.num_levels) L.off[t] = a.lv_off[t];
+    if (a.d_level_n) {
+        if (t < 32) {
+            // A call that failed leaves no counts to go by.
+            uint64_t n = t < a.num_levels && *a.err == 0 ? a.d_level_n[t] : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint64_t y = __shfl_up_sync(0xFFFFFFFFu, n, o);
+                if (t >= o) n += y;
+            }
+            if (t < a.num_levels) L.off[t + 1] = n;
+            if (t == 0) L.off[0] = 0;
+        }
+    } else if (t <= a.num_levels) {
+        L.off[t] = a.lv_off[t];
+    }
     __syncthreads();
 }
 // Level of node i, searching up from level l (nodes are visited in order).
@@ -707,10 +721,10 @@ __global__ void __launch_bounds__(kT) final_positions(FinalArgs a) {
     __shared__ FinalScanSmem S;
     __shared__ FinalLevels LV;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint64_t n = a.num_nodes;
+    load_levels(a, LV);
+    const uint64_t n = a.d_level_n ? LV.off[a.num_levels] : a.num_nodes;
     const uint32_t ntiles = scan_tiles(n);
     if (blockIdx.x >= ntiles) return;  // grids are sized by an upper bound on n
-    load_levels(a, LV);
     while (true) {
         const uint32_t tile = next_tile(a.tile_counter, &S.slot);
         if (tile >= ntiles) break;

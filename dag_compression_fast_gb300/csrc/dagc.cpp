@@ -34,7 +34,6 @@ namespace {
 
 constexpr int kMaxDepth = 21;
 constexpr uint64_t kMaxFragments = (1ull << 31) - 2;  // digit counts + 1 in the sort's 31-bit status
-constexpr int kMaxSorts = 48;
 constexpr int kMaxTileCounters = 1024;
 
 // Device-count slots of one call.
@@ -45,6 +44,7 @@ enum : int {
     kCntNodes = 3,                 // + level
     kCntUnique = 3 + kMaxDepth,    // + level
     kCntSlots = 3 + 2 * kMaxDepth + 1,
+    kCntWords = 61,                // words of all nodes (final layout)
     kCntDirectBlocks = 62,         // occupied blocks of the direct-mapped brick table
     kCntOverflow = 63,             // fragments the grouping spilled past their partition's slab
 };
@@ -54,7 +54,6 @@ struct CallHeader {
     uint32_t pad;
     uint64_t counts[64];
     uint32_t tile_counters[kMaxTileCounters];
-    uint32_t hist[kMaxSorts][kSortHistWords];
     DedupState dedup;
     uint32_t sketch[kGroupSketchRegs];  // distinct-brick sketch of the fragment grouping's probe
     uint32_t gover[kGroupMaxParts];     // its partitions that spilled past their slabs
@@ -62,7 +61,7 @@ struct CallHeader {
     uint32_t path[4];                   // [0] 1: fragments grouped by hash, 0: sorted; [1], [2] its shape
     LeafOrder leaf;                     // ordering of the distinct leaf masks
 };
-static_assert(kCntSlots <= kCntDirectBlocks, "count slots");
+static_assert(kCntSlots <= kCntWords, "count slots");
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -304,10 +303,11 @@ struct GraphKey {
     void* table;       // the dedup table block
     int group;         // fragment grouping mode
     void* direct;      // the direct-mapped brick table (null: not used)
+    bool words;        // the final layout's positions included
     bool operator==(const GraphKey& o) const {
         return frag == o.frag && n == o.n && depth == o.depth && arena == o.arena && chunks == o.chunks &&
                chunk_depth == o.chunk_depth && chunk_path == o.chunk_path && dedup == o.dedup && table == o.table &&
-               group == o.group && direct == o.direct;
+               group == o.group && direct == o.direct && words == o.words;
     }
 };
 struct GraphEntry {
@@ -538,11 +538,13 @@ int device_error_status(uint32_t err, std::string& msg) {
 struct CallSlots {
     CallHeader* h;
     int next_counter = 0, next_hist = 0;
+    uint32_t* hist_base = nullptr;  // zeroed, hist_count x kSortHistWords
+    int hist_count = 0;
     uint64_t* sv_next = nullptr;
     uint64_t* sv_end = nullptr;
     uint32_t* counter() { return &h->tile_counters[next_counter++]; }
     uint32_t* counters(int k) { uint32_t* p = &h->tile_counters[next_counter]; next_counter += k; return p; }
-    uint32_t* hist() { return h->hist[next_hist++]; }
+    uint32_t* hist() { return hist_base + (size_t)kSortHistWords * next_hist++; }
     uint64_t* sv(uint64_t n_bound) {
         uint64_t* p = sv_next;
         sv_next += scan_tiles(n_bound) + 1;
@@ -591,7 +593,7 @@ int run_sort(dagc_context ctx, CallSlots& cs, const SortBuffers& sb, const uint6
              int validate_bits, cudaStream_t s, int hist_stage = -1, int pass_stage = -1,
              const SegmentSpec* seg = nullptr, const uint32_t* gate = nullptr, uint32_t gate_run = 0) {
     t_pdl = ctx->pdl;
-    if (cs.next_hist >= kMaxSorts || cs.next_counter + kMaxPasses > kMaxTileCounters)
+    if (cs.next_hist >= cs.hist_count || cs.next_counter + kMaxPasses > kMaxTileCounters)
         return set_error(ctx, DAGC_ERR_TOO_LARGE, "too many sorts in one call");
     SortArgs a{};
     a.keys_in = keys_in;
@@ -783,6 +785,10 @@ struct CreatePools {
     uint64_t* leaves = nullptr;
     std::vector<uint64_t> unique;  // u_l
     uint64_t num_leaves = 0;
+    // The final layout's positions (null: not made by the call): word_pos of
+    // every node and their words in all.
+    uint32_t* word_pos = nullptr;
+    uint64_t node_words = 0;
 };
 
 // Batched input (see dagc_create_batched): chunk offsets into the fragment
@@ -830,6 +836,9 @@ struct CreateLayout {
     std::vector<uint64_t> cap;  // node bound per level
     uint64_t capmax = 1, p0cap = 0, sv_total = 0;
     size_t zero_bytes = 0, total = 0;
+    int sorts = 0;
+    uint64_t node_bound = 0;  // nodes of all levels
+    size_t o_hist = 0, o_fsv = 0;
     size_t o_hdr, o_sv, o_ss0, o_ss1, o_A, o_B, o_P, o_LM, o_SK, o_SKa, o_V, o_Va, o_M0, o_M1;
     size_t o_NC0, o_NC1, o_NM, o_NCH, o_NH, o_PL, o_lead_or, o_lead_run, o_seg_off, o_seg_code;
     // Fragment grouping (when `grouping`): the partition slabs.
@@ -868,6 +877,15 @@ struct CreateLayout {
         Layout L;
         o_hdr = L.take<CallHeader>(1);
         o_sv = L.take<uint64_t>(sv_total);
+        // Digit histograms: the brick and the fragment sort; the radix form
+        // also sorts the leaves and every level.
+        sorts = !use_dedup ? 2 + nl : direct || (chunk_depth > 0 && k_batch) ? 0 : 2;
+        o_hist = L.take<uint32_t>((uint64_t)sorts * kSortHistWords);
+        // Words of the final layout (hash-set form): look-back of the positions.
+        if (use_dedup && nl > 0) {
+            for (int l = 0; l < nl; ++l) node_bound += cap[l];
+            o_fsv = L.take<uint64_t>(scan_tiles(node_bound) + 1);
+        }
         if (direct_table) {
             o_dcount = L.take<uint32_t>(direct_blocks(depth));
             o_dsv = L.take<uint64_t>(direct_plan_tiles(depth));
@@ -886,7 +904,6 @@ struct CreateLayout {
         }
         zero_bytes = L.off;
         if (direct_table) o_dlist = L.take<uint2>(direct_blocks(depth));
-        const bool sorts = !direct || !use_dedup;
         o_ss0 = L.take<uint32_t>(sorts ? sort_status_words(n) : 0);
         o_ss1 = L.take<uint32_t>(sorts ? sort_status_words(n) : 0);
         o_A = L.take<uint64_t>(direct ? 0 : n);
@@ -1041,7 +1058,8 @@ int load_tune_file(dagc_context ctx, const char* path);
 constexpr int kStatusFallback = -1000;
 
 int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int depth, cudaStream_t s,
-                    CreatePools& out, const BatchSpec* batch, bool use_dedup, bool allow_direct = true) {
+                    CreatePools& out, const BatchSpec* batch, bool use_dedup, bool want_words = false,
+                    bool allow_direct = true) {
     t_pdl = ctx->pdl;
     const int group_mode = ctx->group_mode;
     const int nl = depth - 2;
@@ -1051,6 +1069,7 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
     const bool chunk_path = batch && ctx->batch_path == 1 && chunk_bin_bits(batch->chunk_depth) <= kChunkMaxBinBits;
     const bool direct_table = allow_direct && !batch && use_dedup && group_mode == 1 && direct_table_applies(n, depth);
     const bool direct = direct_table && direct_mark_applies(n, depth);
+    const bool words = want_words && use_dedup && nl > 0;
     const CreateLayout Lo(n, depth, batch ? batch->k : 0u, use_dedup, ctx->dedup_unique_limit,
                           group_mode != 0 && use_dedup && !chunk_path && !direct, chunk_path ? batch->chunk_depth : 0,
                           direct_table, direct);
@@ -1065,7 +1084,7 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
         if (st) return st;
     }
     if (direct_table && !reserve_direct(ctx, direct_entries(depth), s))
-        return create_pipeline(ctx, d_frag, n, depth, s, out, batch, use_dedup, false);
+        return create_pipeline(ctx, d_frag, n, depth, s, out, batch, use_dedup, want_words, false);
     char* b = static_cast<char*>(ctx->arena.base);
     auto P64 = [&](size_t o) { return reinterpret_cast<uint64_t*>(b + o); };
     auto P32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(b + o); };
@@ -1105,6 +1124,8 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
         cs.h = reinterpret_cast<CallHeader*>(b + Lo.o_hdr);
         cs.sv_next = P64(Lo.o_sv);
         cs.sv_end = P64(Lo.o_sv) + sv_total;
+        cs.hist_base = P32(Lo.o_hist);
+        cs.hist_count = Lo.sorts;
         SortBuffers sb{{P32(Lo.o_ss0), P32(Lo.o_ss1)}};
         DAGC_CUDA(ctx, cudaMemsetAsync(b, 0, zero_bytes, s));
         uint32_t* err = &cs.h->err;
@@ -1407,6 +1428,27 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
                 DAGC_LAUNCHED(ctx);
             }
             t_levels.stop();
+            if (words) {
+                // The words' positions with the call, from the counts on the
+                // device: once the host knows them, it allocates the exact
+                // words and only the write is left. The positions take the
+                // room of the nodes' arrays, which are no longer read.
+                StageTimer t(ctx, DAGC_STAGE_FINAL, s);
+                FinalArgs f{};
+                for (int l = 0; l < nl; ++l) f.lv_masks[l] = P8(Lo.o_pm[l]);
+                f.num_levels = nl;
+                f.d_level_n = cs.count(kCntUnique);
+                f.word_pos = P32(Lo.o_nh[0]);
+                f.d_total = cs.count(kCntWords);
+                f.status = P64(Lo.o_fsv);
+                f.tile_counter = cs.counter();
+                f.err = err;
+                f.grid_scan = grid_for(ctx->grid_scan / ctx->sms, ctx->sms, scan_tiles(Lo.node_bound));
+                launch_final_positions(f, s);
+                ++ctx->launches;
+                DAGC_LAUNCHED(ctx);
+                t.stop(1);  // the final layout's bytes are counted with its write
+            }
         } else {
             StageTimer t_dedup(ctx, DAGC_STAGE_LEAF_DEDUP, s);
             st = run_sort(ctx, cs, sb, P64(Lo.o_LM), P64(Lo.o_SK), P64(Lo.o_SKa), nullptr, P32(Lo.o_V), P32(Lo.o_Va), true, p0cap,
@@ -1530,7 +1572,7 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
     int st = run_enqueue(ctx, GraphKey{d_frag, n, depth, ctx->arena.base, batch ? batch->k : 0u,
                                        batch ? batch->chunk_depth : 0, chunk_path, use_dedup,
                                        use_dedup ? ctx->table : nullptr, use_dedup ? group_mode : 0,
-                                       direct_table ? ctx->direct : nullptr},
+                                       direct_table ? ctx->direct : nullptr, words},
                          s, enqueue);
     if (st) { ctx->table_dirty = true; ctx->direct_dirty = true; return st; }
     CallHeader* hdr = reinterpret_cast<CallHeader*>(b + Lo.o_hdr);
@@ -1606,6 +1648,10 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
     }
     out.leaves = P64(Lo.o_PL);
     out.num_leaves = counts[kCntLeaves];
+    if (words) {
+        out.word_pos = P32(Lo.o_nh[0]);
+        out.node_words = counts[kCntWords];
+    }
     return DAGC_OK;
 }
 
@@ -1669,6 +1715,8 @@ struct FinalSource {
     std::vector<uint64_t> off;              // num_levels + 1 node offsets
     const uint64_t* leaves = nullptr;
     uint64_t num_leaves = 0;
+    uint32_t* word_pos = nullptr;  // positions made already (CreatePools)
+    uint64_t node_words = 0;
 };
 
 // Bytes of arena scratch the final layout of nn nodes takes (from offset 0).
@@ -1697,8 +1745,10 @@ int final_words(dagc_context ctx, const FinalSource& src, cudaStream_t s, uint32
     const size_t o_pos = L.take<uint32_t>(nn + 1);
     char* b = static_cast<char*>(ctx->arena.base);
     CallHeader* h = reinterpret_cast<CallHeader*>(b + o_hdr);
-    uint32_t* pos = reinterpret_cast<uint32_t*>(b + o_pos);
-    DAGC_CUDA(ctx, cudaMemsetAsync(b, 0, zero_bytes, s));
+    // With positions made by the call, its header (at the same place, no error
+    // set) serves on.
+    uint32_t* pos = src.word_pos ? src.word_pos : reinterpret_cast<uint32_t*>(b + o_pos);
+    if (!src.word_pos) DAGC_CUDA(ctx, cudaMemsetAsync(b, 0, zero_bytes, s));
     FinalArgs a{};
     for (int l = 0; l < nlv; ++l) {
         a.lv_masks[l] = src.masks[l];
@@ -1720,11 +1770,14 @@ int final_words(dagc_context ctx, const FinalSource& src, cudaStream_t s, uint32
     // lets the positions and the write run back to back; the exact count
     // comes back with the error word in the call's one read-back.
     const uint64_t bound = 9 * nn + 2 * src.num_leaves;
-    const bool by_bound = bound < (1ull << 32);
-    uint64_t node_words = 0;
+    const bool by_bound = !src.word_pos && bound < (1ull << 32);
+    uint64_t node_words = src.node_words;
     void* w = nullptr;
     StageTimer t(ctx, DAGC_STAGE_FINAL, s);
-    if (nn) {
+    if (src.word_pos) {
+        if (node_words + 2 * src.num_leaves >= (1ull << 32))
+            return set_error(ctx, DAGC_ERR_TOO_LARGE, "final DAG exceeds 2^32 words");
+    } else if (nn) {
         launch_final_positions(a, s);
         ++ctx->launches;
         DAGC_LAUNCHED(ctx);
@@ -1750,7 +1803,7 @@ int final_words(dagc_context ctx, const FinalSource& src, cudaStream_t s, uint32
         ctx->pool.release(w);
         return set_error(ctx, cuda_status(le), std::string("final: ") + cudaGetErrorString(le));
     }
-    if (nn) node_words = ctx->h_stage[1];
+    if (nn && !src.word_pos) node_words = ctx->h_stage[1];
     const uint64_t total = node_words + 2 * src.num_leaves;
     set_pending_bytes(ctx, DAGC_STAGE_FINAL, nn * 2 + (41 * nn + 8 * src.num_leaves) + 4 * total);
     settle_profile(ctx);
@@ -1801,7 +1854,9 @@ int compress_from_pools(dagc_context ctx, const CreatePools& p, int nl, cudaStre
     }
     src.leaves = p.leaves;
     src.num_leaves = p.num_leaves;
-    if (final_scratch_bytes(src.off[nl]) > lowest) return DAGC_OK;  // would overlap a pool
+    src.word_pos = p.word_pos;
+    src.node_words = p.node_words;
+    if (!src.word_pos && final_scratch_bytes(src.off[nl]) > lowest) return DAGC_OK;  // would overlap a pool
     *done = true;
     return final_words(ctx, src, s, d_words, n_words);
 }
@@ -1831,6 +1886,7 @@ int union_radix(dagc_context ctx, dagc_dag* in, uint64_t k, cudaStream_t s, uint
     uint64_t sv_total = sv_words(total_leaves);
     for (int l = 0; l < nl; ++l) sv_total += sv_words(level_total[l]);
     const size_t o_sv = L.take<uint64_t>(sv_total);
+    const size_t o_hist = L.take<uint32_t>((uint64_t)(nl + 1) * kSortHistWords);
     const size_t zero_bytes = L.off;
     const size_t o_ss0 = L.take<uint32_t>(sort_status_words(capmax));
     const size_t o_ss1 = L.take<uint32_t>(sort_status_words(capmax));
@@ -1863,6 +1919,8 @@ int union_radix(dagc_context ctx, dagc_dag* in, uint64_t k, cudaStream_t s, uint
     cs.h = reinterpret_cast<CallHeader*>(b + o_hdr);
     cs.sv_next = P64(o_sv);
     cs.sv_end = P64(o_sv) + sv_total;
+    cs.hist_base = P32(o_hist);
+    cs.hist_count = nl + 1;
     SortBuffers sb{{P32(o_ss0), P32(o_ss1)}};
     DAGC_CUDA(ctx, cudaMemsetAsync(b, 0, zero_bytes, s));
     uint32_t* err = &cs.h->err;
@@ -2866,7 +2924,7 @@ int dagc_compress(dagc_context ctx, const uint64_t* d_fragments, uint64_t n, int
             DAGC_CUDA(ctx, cudaSetDevice(ctx->device));
             cudaStream_t s = static_cast<cudaStream_t>(stream);
             CreatePools p;
-            int st = create_pipeline(ctx, d_fragments, n, depth, s, p, nullptr, ctx->use_dedup);
+            int st = create_pipeline(ctx, d_fragments, n, depth, s, p, nullptr, ctx->use_dedup, true);
             if (st == kStatusFallback) {
                 ++ctx->fallbacks;
                 st = create_pipeline(ctx, d_fragments, n, depth, s, p, nullptr, false);
@@ -3222,6 +3280,7 @@ int enqueue_sort(dagc_context ctx, const uint64_t* d_keys_in, uint64_t* d_keys_o
     const bool with_values = d_vals_out != nullptr;
     Layout L;
     const size_t o_hdr = L.take<CallHeader>(1);
+    const size_t o_hist = L.take<uint32_t>(kSortHistWords);
     const size_t zero_bytes = L.off;
     const size_t o_ss0 = L.take<uint32_t>(sort_status_words(n));
     const size_t o_ss1 = L.take<uint32_t>(sort_status_words(n));
@@ -3232,6 +3291,8 @@ int enqueue_sort(dagc_context ctx, const uint64_t* d_keys_in, uint64_t* d_keys_o
     char* b = static_cast<char*>(ctx->arena.base);
     CallSlots cs;
     cs.h = reinterpret_cast<CallHeader*>(b + o_hdr);
+    cs.hist_base = reinterpret_cast<uint32_t*>(b + o_hist);
+    cs.hist_count = 1;
     SortBuffers sb{{reinterpret_cast<uint32_t*>(b + o_ss0), reinterpret_cast<uint32_t*>(b + o_ss1)}};
     DAGC_CUDA(ctx, cudaMemsetAsync(b, 0, zero_bytes, s));
     ctx->sort_err = &cs.h->err;

@@ -518,6 +518,9 @@ struct FinalArgs {
     uint64_t lv_off[kFinalMaxLevels + 1];
     int num_levels;
     uint64_t num_nodes;  // lv_off[num_levels]
+    // Positions before the host knows the counts: when non-null, the nodes per
+    // level on the device, and lv_off is not read.
+    const uint64_t* d_level_n;
     const uint64_t* leaves; uint64_t num_leaves;
     uint32_t* word_pos;  // num_nodes + 1
     uint64_t* d_total;   // exact 64-bit sum of node words
