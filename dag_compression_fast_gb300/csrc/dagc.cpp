@@ -3214,7 +3214,7 @@ int dagc_voxelize(dagc_context ctx, const double* d_vertices, uint64_t n_triangl
     DAGC_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // Scratch: total, tile counter, error word, look-back status per tile.
-    const uint64_t tiles = voxelize_tiles(n_triangles);
+    const uint64_t tiles = voxelize_tiles(n_triangles, mode);
     const size_t bytes = 64 + (tiles + 1) * 8;
     if (bytes > ctx->vox_scratch_bytes) {
         if (ctx->vox_scratch) cudaFree(ctx->vox_scratch);
@@ -3237,7 +3237,7 @@ int dagc_voxelize(dagc_context ctx, const double* d_vertices, uint64_t n_triangl
     a.tile_counter = reinterpret_cast<uint32_t*>(b + 8);
     a.err = reinterpret_cast<uint32_t*>(b + 16);
     a.status = reinterpret_cast<uint64_t*>(b + 64);
-    const int grid = (int)std::min<uint64_t>(tiles, (uint64_t)ctx->sms * 8);
+    const int grid = (int)std::min<uint64_t>(tiles, (uint64_t)ctx->sms * 12);
     launch_voxelize(a, grid, s);
     ++ctx->launches;
     DAGC_LAUNCHED(ctx);

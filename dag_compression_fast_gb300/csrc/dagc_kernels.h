@@ -477,6 +477,7 @@ struct VoxArgs {
     const double* vertices; uint64_t n_tri;  // 9 doubles per triangle
     double aabb[6];                          // box mapped onto the grid: min xyz, max xyz
     double scale[3];                         // 2^depth / extent (set by launch_voxelize)
+    int per;                                 // triangles per warp (set by launch_voxelize)
     int depth, mode;
     uint64_t* codes; uint64_t capacity;
     uint64_t* d_total;                       // fragments produced (may exceed capacity)
@@ -484,7 +485,7 @@ struct VoxArgs {
 };
 void voxelize_configure();
 void launch_voxelize(const VoxArgs& a, int grid, cudaStream_t s);
-uint64_t voxelize_tiles(uint64_t n_tri);
+uint64_t voxelize_tiles(uint64_t n_tri, int mode);
 
 // The radix form's top levels in one single-CTA launch: every level l <= first_level has at
 // most kTailCap nodes, so extract + hash + sort + unique run in shared memory.

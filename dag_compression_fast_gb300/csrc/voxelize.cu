@@ -15,23 +15,27 @@
 //           axis test (Akenine-Moller 2001); float64. The 26-connected
 //           surface used for the triangle-soup workload.
 //
-// Tiles of kVoxTile triangles: each triangle is set up by one thread (its
-// constants go to shared memory), then tested by one warp, lanes striding over
-// its bounding box (rows of pixels / voxel columns), so that large triangles
-// spread over 32 lanes. The hits found while counting are kept (packed local
-// positions, per warp) and only their codes are left to compute once the
-// per-tile counts have given the output offsets, through a single decoupled
+// Tiles of kVoxTile triangles, a run of them to each warp: its lanes set up one
+// triangle each (the constants go to shared memory), then the warp tests them
+// one by one, lanes striding over the bounding box (rows of pixels / voxel
+// columns), so that large triangles spread over 32 lanes. The hits found while
+// counting are kept (packed local positions, per warp) and only their codes are
+// left to compute, 32 at a time over all of the warp's triangles, once the
+// tiles' counts have given the output offsets through a single decoupled
 // look-back. The output order is fixed: triangles in input order, each
 // triangle's fragments in bounding-box order. A call without room for codes
 // only counts. This file is compiled with --fmad=false: every float operation
 // rounds once, as in the CPU checkers (but for the explicit fmaf of the SAT
 // filter, whose error bound covers it).
 //
-// Each form is bound by the arithmetic per candidate. A counting and a writing
-// call together: 500k triangles, depth 12, the GL rule, 2640 us when every lane
-// of the warp repeated the setup and a second pass repeated the tests, now 660;
-// 60k triangles, depth 11, the SAT rule, 57 ms when it ran in float64 throughout
-// (of which this part does 2 operations per SM and clock), now 0.89.
+// Each form is bound by the arithmetic per candidate (2.7 instructions per SM
+// and clock of 4). A counting and a writing call together, 500k triangles, depth
+// 12, the GL rule: 2640 us when every lane of the warp repeated the setup and a
+// second pass repeated the tests; 684 with one setup by 64 of 256 threads, a
+// third of whose time was barriers, and four integer divisions a lane to start
+// each box; now 515. 60k triangles, depth 11, the SAT rule: 57 ms in float64
+// throughout (of which this part does 2 operations per SM and clock), 0.90 ms
+// with the filter, now 0.72.
 
 #include "dagc_device.cuh"
 #include "dagc_kernels.h"
@@ -41,16 +45,29 @@
 namespace dagc {
 namespace {
 
-constexpr int kVoxThreads = 256;
+constexpr int kVoxThreads = 128;
 constexpr int kVoxWarps = kVoxThreads / 32;
-// Triangles per tile: small, so that a call of a few thousand triangles
-// spreads over the GPU.
+// Most triangles of a tile, and of a warp (consecutive ones): fewer when the
+// tiles would be too few for the GPU (voxelize_per).
 constexpr int kVoxTile = 64;
-// Hits kept per warp from the count to the emission, and the mark of a
-// triangle whose hits were not kept (it is tested again).
+constexpr int kVoxPer = kVoxTile / kVoxWarps;
+// Tiles below which a warp takes fewer triangles: 8 CTAs on each of 152 SMs
+// for the SAT rule (3000 triangles: 299 us for both calls against 748 with 16 a
+// warp), 4 for the GL rule, whose triangles are a tenth of the work.
+constexpr uint64_t kVoxMinTilesGl = 608, kVoxMinTilesSat = 1216;
+// Hits kept per warp from the count to the emission: the triangle in the
+// warp's run and the local position, packed.
 constexpr int kVoxKeep = 768;
-constexpr uint32_t kNotKept = 0xFFFFFFFFu;
+constexpr int kKeepShift = 28;
+static_assert(kVoxPer <= 32 && kVoxPer <= 1 << (32 - kKeepShift), "a lane and an id per triangle");
 
+__device__ __forceinline__ uint32_t spread10(uint32_t x) {
+    x &= 0x3FFu;
+    x = (x | x << 16) & 0x030000FFu;
+    x = (x | x << 8) & 0x0300F00Fu;
+    x = (x | x << 4) & 0x030C30C3u;
+    return (x | x << 2) & 0x09249249u;
+}
 // The low 11 bits of x, each moved to three times its place.
 __device__ __forceinline__ uint64_t spread11(uint32_t x) {
     x &= 0x7FFu;
@@ -62,9 +79,35 @@ __device__ __forceinline__ uint64_t spread11(uint32_t x) {
     return top | x;
 }
 __device__ __forceinline__ uint64_t spread21(uint32_t x) { return spread11(x & 0x3FFu) | spread11((x >> 10) & 0x7FFu) << 30; }
-__device__ __forceinline__ uint64_t morton3(uint32_t x, uint32_t y, uint32_t z) {
-    return spread21(x) << 2 | spread21(y) << 1 | spread21(z);
+// Ten bits of the three coordinates interleave in 32-bit words; G is the same
+// for all lanes.
+__device__ __forceinline__ uint64_t morton3(uint32_t x, uint32_t y, uint32_t z, int G) {
+    if (G > 1 << 20) return spread21(x) << 2 | spread21(y) << 1 | spread21(z);
+    const uint32_t lo = spread10(x) << 2 | spread10(y) << 1 | spread10(z);
+    if (G <= 1 << 10) return lo;
+    const uint32_t hi = spread10(x >> 10) << 2 | spread10(y >> 10) << 1 | spread10(z >> 10);
+    return (uint64_t)hi << 30 | lo;
 }
+
+// A box of candidates (nz fastest), walked by the lanes of a warp 32 at a time.
+// Set up once per triangle: how far 32 candidates on is, and the reciprocals
+// that give a lane's first position: (i + 0.5) / n is at least 0.5 / n from a
+// whole number, far more than its rounding for i < 32.
+struct Box {
+    uint32_t nx, ny, nz;
+    uint32_t dx, dy, dz;
+    float ry, rz;
+    __device__ void set(uint32_t x, uint32_t y, uint32_t z) {
+        nx = x; ny = y; nz = z;
+        if (x == 0 || y == 0 || z == 0) return;
+        dz = 32 % z;
+        const uint32_t rows = 32 / z;
+        dy = x == 1 ? rows : rows % y;  // one layer: the rows past its last end the walk
+        dx = rows / y;
+        ry = 1.0f / (float)y;
+        rz = 1.0f / (float)z;
+    }
+};
 
 // ---------------------------------------------------------------- GL rule --
 struct GlTri {
@@ -72,8 +115,8 @@ struct GlTri {
     float U[3], V[3], W[3];
     float dwdu, dwdv;
     float nx[3], ny[3], dk[3];
-    int i0, i1, j0, j1;
-    bool empty;
+    int i0, j0;
+    Box box;  // (1, rows, columns); no columns: empty
 };
 
 __device__ __forceinline__ int lo_cell(float m, float Gf) {
@@ -89,8 +132,7 @@ __device__ __forceinline__ int clamp_cell(float z, int G) {
     return k < 0 ? 0 : (k > G - 1 ? G - 1 : k);
 }
 
-__device__ GlTri gl_setup(const double* P, const double* aabb, int depth) {
-    GlTri t;
+__device__ void gl_setup(const double* P, const double* aabb, int depth, GlTri& t) {
     const int G = 1 << depth;
     const float Gf = (float)G;
     float p[3][3], mn[3], mx[3];
@@ -124,7 +166,7 @@ __device__ GlTri gl_setup(const double* P, const double* aabb, int depth) {
     const float e1u = t.U[1] - t.U[0], e1v = t.V[1] - t.V[0], e1w = t.W[1] - t.W[0];
     const float e2u = t.U[2] - t.U[0], e2v = t.V[2] - t.V[0], e2w = t.W[2] - t.W[0];
     const float det = e1u * e2v - e2u * e1v;
-    t.empty = !(det != 0.0f) || !isfinite(det);
+    bool empty = !(det != 0.0f) || !isfinite(det);
     t.dwdu = (e1w * e2v - e2w * e1v) / det;
     t.dwdv = (e2w * e1u - e1w * e2u) / det;
     const float sgn = det > 0.0f ? 1.0f : -1.0f;
@@ -136,11 +178,11 @@ __device__ GlTri gl_setup(const double* P, const double* aabb, int depth) {
         t.dk[k] = fmaxf(t.nx[k], 0.0f) + fmaxf(t.ny[k], 0.0f);
     }
     t.i0 = lo_cell(fminf(t.U[0], fminf(t.U[1], t.U[2])), Gf);
-    t.i1 = hi_cell(fmaxf(t.U[0], fmaxf(t.U[1], t.U[2])), Gf, G);
+    const int i1 = hi_cell(fmaxf(t.U[0], fmaxf(t.U[1], t.U[2])), Gf, G);
     t.j0 = lo_cell(fminf(t.V[0], fminf(t.V[1], t.V[2])), Gf);
-    t.j1 = hi_cell(fmaxf(t.V[0], fmaxf(t.V[1], t.V[2])), Gf, G);
-    if (t.i0 > t.i1 || t.j0 > t.j1) t.empty = true;
-    return t;
+    const int j1 = hi_cell(fmaxf(t.V[0], fmaxf(t.V[1], t.V[2])), Gf, G);
+    if (t.i0 > i1 || t.j0 > j1) empty = true;
+    t.box.set(1, (uint32_t)(j1 - t.j0 + 1), empty ? 0u : (uint32_t)(i1 - t.i0 + 1));
 }
 
 // Is pixel (i, j) covered?
@@ -160,8 +202,9 @@ __device__ __forceinline__ uint64_t gl_code(const GlTri& t, int i, int j, int G)
     const int s3 = clamp_cell(zc - hx + hy, G), s4 = clamp_cell(zc - hx - hy, G);
     const int k = min(min(min(s0, s1), min(s2, s3)), s4);
     // View axes back: X (u, v, w) = (z, y, x), Y (x, z, y), Z (y, x, z).
-    const uint64_t u = spread21((uint32_t)i), v = spread21((uint32_t)j), w = spread21((uint32_t)k);
-    return t.axis == 0 ? w << 2 | v << 1 | u : t.axis == 1 ? u << 2 | w << 1 | v : v << 2 | u << 1 | w;
+    const uint32_t u = (uint32_t)i, v = (uint32_t)j, w = (uint32_t)k;
+    return morton3(t.axis == 0 ? w : t.axis == 1 ? u : v, t.axis == 0 ? v : t.axis == 1 ? w : u,
+                   t.axis == 0 ? u : t.axis == 1 ? v : w, G);
 }
 
 // --------------------------------------------------------------- SAT rule --
@@ -231,7 +274,7 @@ struct SatTri {
     float mid[3][3], out[3][3], in[3][3];           // per box axis i and edge j
     float n[3], nmid, nout, nin;
     int x0, y0, z0;                                  // bounding box origin
-    int nx, ny, nz;                                  // and extents (0: empty)
+    Box box;                                         // and extents (0: empty)
     int ox, oy, oz;                                  // the filter's origin
     bool exact;
 };
@@ -250,17 +293,18 @@ __device__ void sat_setup(const VoxArgs& args, uint64_t tri, SatTri& t) {
     int64_t z0 = cell_floor(dmin(a.z, dmin(b.z, c.z)), G), z1 = cell_floor(dmax(a.z, dmax(b.z, c.z)), G);
     x0 = x0 < 0 ? 0 : x0; y0 = y0 < 0 ? 0 : y0; z0 = z0 < 0 ? 0 : z0;
     x1 = x1 > Gi - 1 ? Gi - 1 : x1; y1 = y1 > Gi - 1 ? Gi - 1 : y1; z1 = z1 > Gi - 1 ? Gi - 1 : z1;
-    t.nx = x1 >= x0 ? (int)(x1 - x0 + 1) : 0;
-    t.ny = y1 >= y0 ? (int)(y1 - y0 + 1) : 0;
-    t.nz = z1 >= z0 ? (int)(z1 - z0 + 1) : 0;
+    const int nx = x1 >= x0 ? (int)(x1 - x0 + 1) : 0;
+    const int ny = y1 >= y0 ? (int)(y1 - y0 + 1) : 0;
+    const int nz = z1 >= z0 ? (int)(z1 - z0 + 1) : 0;
+    t.box.set((uint32_t)nx, (uint32_t)ny, (uint32_t)nz);
     t.x0 = (int)x0; t.y0 = (int)y0; t.z0 = (int)z0;
     t.exact = true;
-    if (t.nx == 0 || t.ny == 0 || t.nz == 0) return;
-    t.ox = t.x0 + t.nx / 2;
-    t.oy = t.y0 + t.ny / 2;
-    t.oz = t.z0 + t.nz / 2;
+    if (nx == 0 || ny == 0 || nz == 0) return;
+    t.ox = t.x0 + nx / 2;
+    t.oy = t.y0 + ny / 2;
+    t.oz = t.z0 + nz / 2;
     float f[3][3];
-    float K = (float)(max(t.nx, max(t.ny, t.nz)) / 2 + 2);
+    float K = (float)(max(nx, max(ny, nz)) / 2 + 2);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         f[k][0] = (float)(v[k].x - (double)t.ox);
@@ -338,151 +382,137 @@ __device__ __forceinline__ bool sat_hit(const VoxArgs& a, uint64_t tri, const Sa
 template <int kMode>
 struct VoxSmem {
     typename std::conditional<kMode == kVoxGL, GlTri, SatTri>::type tri[kVoxTile];
-    uint64_t count[kVoxTile];             // fragments, then offsets inside the tile
-    uint32_t kept_at[kVoxTile];           // the triangle's hits in its warp's list, or kNotKept
-    uint32_t kept[kVoxWarps][kVoxKeep];
-    uint64_t scan[34];
-    uint32_t slot;
+    uint64_t warp_total[kVoxWarps];
     uint64_t base;
+    uint32_t kept[kVoxWarps][kVoxKeep];
+    uint32_t slot;
 };
 
-// A triangle's candidates, walked by the lanes of a warp 32 at a time in
-// bounding-box order (z, or the pixel column, fastest): the lane's position
-// moves on without a division.
-struct BoxWalk {
-    uint32_t nz, ny;     // the two inner extents
-    uint32_t dz, dy, dx; // 32 candidates on
-    uint32_t x, y, z;
-    __device__ BoxWalk(uint32_t ny_, uint32_t nz_, uint32_t lane) : nz(nz_), ny(ny_) {
-        dz = 32 % nz;
-        const uint32_t rows = 32 / nz;
-        dy = rows % ny;
-        dx = rows / ny;
-        z = lane % nz;
-        const uint32_t row = lane / nz;
-        y = row % ny;
-        x = row / ny;
-    }
-    __device__ __forceinline__ void next() {
-        z += dz;
-        y += dy;
-        x += dx;
-        if (z >= nz) { z -= nz; ++y; }
-        if (y >= ny) { y -= ny; ++x; }
-    }
-};
+// The code of candidate (x, y, z) of a triangle's box.
+template <int kMode, typename Tri>
+__device__ __forceinline__ uint64_t code_of(const Tri& t, uint32_t x, uint32_t y, uint32_t z, int G) {
+    if constexpr (kMode == kVoxGL) return gl_code(t, t.i0 + (int)z, t.j0 + (int)y, G);
+    else return morton3((uint32_t)t.x0 + x, (uint32_t)t.y0 + y, (uint32_t)t.z0 + z, G);
+}
 
-// The warp tests triangle k of the tile. kEmit: the hits' codes go out from
-// `pos` on. Otherwise they are counted and kept in the warp's list from
-// `at` on, where they fit and their local positions pack into a word. Every
-// lane runs the same trip count, so each ballot is made by all 32 lanes.
-template <int kMode, bool kEmit>
-__device__ uint64_t warp_triangle(const VoxArgs& a, VoxSmem<kMode>& S, uint64_t tri, uint32_t k, uint64_t pos, uint32_t at) {
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const auto& t = S.tri[k];
+// The warp tests a triangle, lanes striding over its box in order. kEmit: the
+// hits' codes go out from `pos` on. Otherwise they are counted and, where
+// `keep` is set, kept from `at` on with the triangle's id; *keep is cleared
+// once one does not fit. Every lane runs the same trip count, so each ballot
+// is made by all 32 lanes.
+template <int kMode, bool kEmit, typename Tri>
+__device__ __forceinline__ uint64_t warp_triangle(const VoxArgs& a, const Tri& tri_s, uint64_t tri, uint32_t id, uint64_t pos,
+                                                  uint32_t* kept, uint32_t at, bool* keep) {
+    const uint32_t lane = threadIdx.x & 31;
+    const Box box = tri_s.box;
+    const uint64_t area = (uint64_t)box.nx * box.ny * box.nz;
+    if (area == 0) return 0;
+    // What the GL tests read fits registers; the SAT's 45 words stay shared.
+    typename std::conditional<kMode == kVoxGL, const Tri, const Tri&>::type t = tri_s;
     const int G = 1 << a.depth;
-    uint64_t area;
-    uint32_t ny, nz;
-    bool packs;
-    if constexpr (kMode == kVoxGL) {
-        if (t.empty) return 0;
-        ny = (uint32_t)(t.j1 - t.j0 + 1);
-        nz = (uint32_t)(t.i1 - t.i0 + 1);
-        area = (uint64_t)ny * nz;
-        packs = ny <= 65536 && nz <= 65536;
-    } else {
-        ny = (uint32_t)t.ny;
-        nz = (uint32_t)t.nz;
-        area = (uint64_t)t.nx * ny * nz;
-        if (area == 0) return 0;
-        packs = t.nx <= 1024 && ny <= 1024 && nz <= 1024;
+    if (!kEmit && (kMode == kVoxGL ? (box.ny | box.nz) >> 14 : (box.nx | box.ny) >> 9 | box.nz >> 10)) *keep = false;
+    const bool keeps = !kEmit && *keep;
+    // The lane's position moves on without a division.
+    const uint32_t row = (uint32_t)(((float)lane + 0.5f) * box.rz);
+    uint32_t z = lane - row * box.nz, y = row, x = 0;
+    if constexpr (kMode != kVoxGL) {
+        x = (uint32_t)(((float)row + 0.5f) * box.ry);
+        y = row - x * box.ny;
     }
-    BoxWalk w(ny, nz, lane);
     uint64_t n = 0;
-    for (uint64_t b = 0; b < area; b += 32, w.next()) {
+    for (uint64_t b = 0; b < area; b += 32) {
         bool hit = b + lane < area;
-        if constexpr (kMode == kVoxGL) hit = hit && gl_covered(t, t.i0 + (int)w.z, t.j0 + (int)w.y);
-        else hit = hit && sat_hit(a, tri, t, t.x0 + (int)w.x, t.y0 + (int)w.y, t.z0 + (int)w.z);
+        if constexpr (kMode == kVoxGL) hit = hit && gl_covered(t, t.i0 + (int)z, t.j0 + (int)y);
+        else hit = hit && sat_hit(a, tri, t, t.x0 + (int)x, t.y0 + (int)y, t.z0 + (int)z);
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, hit);
         if (hit) {
             const uint64_t o = n + __popc(m & lanemask_lt());
             if constexpr (kEmit) {
-                uint64_t code;
-                if constexpr (kMode == kVoxGL) code = gl_code(t, t.i0 + (int)w.z, t.j0 + (int)w.y, G);
-                else code = morton3((uint32_t)t.x0 + w.x, (uint32_t)t.y0 + w.y, (uint32_t)t.z0 + w.z);
-                if (pos + o < a.capacity) a.codes[pos + o] = code;
-            } else if (packs && at + o < (uint64_t)kVoxKeep) {
-                S.kept[warp][at + o] = kMode == kVoxGL ? w.y << 16 | w.z : w.x << 20 | w.y << 10 | w.z;
+                if (pos + o < a.capacity) a.codes[pos + o] = code_of<kMode>(t, x, y, z, G);
+            } else if (keeps && at + o < (uint64_t)kVoxKeep) {
+                kept[at + o] = id << kKeepShift | (kMode == kVoxGL ? y << 14 | z : x << 19 | y << 10 | z);
             }
         }
         n += __popc(m);
+        z += box.dz;
+        y += box.dy;
+        x += box.dx;
+        if (z >= box.nz) { z -= box.nz; ++y; }
+        if constexpr (kMode != kVoxGL)
+            if (y >= box.ny) { y -= box.ny; ++x; }
     }
-    if constexpr (!kEmit) {
-        if (lane == 0) S.kept_at[k] = packs && at + n <= (uint64_t)kVoxKeep ? at : kNotKept;
-    }
+    if (!kEmit && at + n > (uint64_t)kVoxKeep) *keep = false;
     return n;
 }
 
 template <int kMode>
-__global__ void __launch_bounds__(kVoxThreads) voxelize(VoxArgs a) {
+__global__ void __launch_bounds__(kVoxThreads, 8) voxelize(VoxArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     VoxSmem<kMode>& S = *reinterpret_cast<VoxSmem<kMode>*>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int G = 1 << a.depth;
-    const uint64_t ntiles = (a.n_tri + kVoxTile - 1) / kVoxTile;
+    const uint32_t per = (uint32_t)a.per;
+    const uint64_t ntiles = (a.n_tri + per * kVoxWarps - 1) / (per * kVoxWarps);
+    auto* tris = S.tri + warp * kVoxPer;  // the warp's own: no barrier between setup, tests and emission
+    uint32_t* kept = S.kept[warp];
     while (true) {
         if (tid == 0) S.slot = atomicAdd(a.tile_counter, 1u);
         __syncthreads();
         const uint64_t tile = S.slot;
         if (tile >= ntiles) break;
-        const uint64_t t0 = tile * kVoxTile;
-        if (tid < kVoxTile && t0 + tid < a.n_tri) {
-            if constexpr (kMode == kVoxGL) S.tri[tid] = gl_setup(a.vertices + 9 * (t0 + tid), a.aabb, a.depth);
-            else sat_setup(a, t0 + tid, S.tri[tid]);
+        const uint64_t t0 = (tile * kVoxWarps + warp) * per;
+        const uint32_t mine = t0 >= a.n_tri ? 0u : (uint32_t)(a.n_tri - t0 < per ? a.n_tri - t0 : per);
+        if (lane < mine) {
+            if constexpr (kMode == kVoxGL) gl_setup(a.vertices + 9 * (t0 + lane), a.aabb, a.depth, tris[lane]);
+            else sat_setup(a, t0 + lane, tris[lane]);
         }
+        __syncwarp();
+        uint64_t count = 0;
+        bool keep = a.capacity != 0;
+        for (uint32_t k = 0; k < mine; ++k)
+            count += warp_triangle<kMode, false>(a, tris[k], t0 + k, k, 0, kept, keep ? (uint32_t)count : 0u, &keep);
+        if (lane == 0) S.warp_total[warp] = count;
         __syncthreads();
-        // Count: warp w takes triangles t0 + w, t0 + w + 8, ...
-        uint32_t at = 0;
-        for (uint32_t k = warp; k < kVoxTile; k += kVoxWarps) {
-            const uint64_t tri = t0 + k;
-            const uint64_t c = tri < a.n_tri ? warp_triangle<kMode, false>(a, S, tri, k, 0, at) : 0;
-            __syncwarp();
-            if (lane == 0) S.count[k] = c;
-            if (c && S.kept_at[k] != kNotKept) at += (uint32_t)c;
-        }
-        __syncthreads();
-        uint64_t total;
-        const uint64_t excl = block_exclusive_sum<uint64_t>(tid < kVoxTile ? S.count[tid] : 0, S.scan, &total);
-        if (tid < kVoxTile) S.count[tid] = excl;  // now the triangle's offset inside the tile
         if (warp == 0) {
+            uint64_t total = 0;
+#pragma unroll
+            for (int w = 0; w < kVoxWarps; ++w) total += S.warp_total[w];
             const uint64_t b = sv_lookback(a.status, (uint32_t)tile, total, a.err);
-            if (lane == 0) S.base = b;
-        }
-        __syncthreads();
-        const uint64_t base = S.base;
-        if (tid == 0 && tile == ntiles - 1) *a.d_total = base + total;
-        if (base < a.capacity) {
-            for (uint32_t k = warp; k < kVoxTile; k += kVoxWarps) {
-                const uint64_t tri = t0 + k;
-                const uint64_t o0 = S.count[k], o1 = k + 1 < (uint32_t)kVoxTile ? S.count[k + 1] : total;
-                if (o0 == o1) continue;  // also the triangles past the last
-                if (S.kept_at[k] == kNotKept) {
-                    warp_triangle<kMode, true>(a, S, tri, k, base + o0, 0);
-                    continue;
-                }
-                const auto& t = S.tri[k];
-                const uint32_t* kept = S.kept[warp] + S.kept_at[k];
-                for (uint64_t j = lane; j < o1 - o0; j += 32) {
-                    const uint32_t e = kept[j];
-                    uint64_t code;
-                    if constexpr (kMode == kVoxGL) code = gl_code(t, t.i0 + (int)(e & 0xFFFFu), t.j0 + (int)(e >> 16), G);
-                    else code = morton3((uint32_t)t.x0 + (e >> 20), (uint32_t)t.y0 + ((e >> 10) & 1023u), (uint32_t)t.z0 + (e & 1023u));
-                    if (base + o0 + j < a.capacity) a.codes[base + o0 + j] = code;
-                }
+            if (lane == 0) {
+                S.base = b;
+                if (tile == ntiles - 1) *a.d_total = b + total;
             }
         }
         __syncthreads();
+        uint64_t base = S.base;
+        for (uint32_t w = 0; w < warp; ++w) base += S.warp_total[w];
+        if (base >= a.capacity) continue;
+        if (keep) {
+            // Every hit was kept: all lanes take hits, of whichever triangle.
+            for (uint32_t j = lane; j < (uint32_t)count; j += 32) {
+                const uint32_t e = kept[j];
+                const auto& t = tris[e >> kKeepShift];
+                uint64_t code;
+                if constexpr (kMode == kVoxGL) code = code_of<kMode>(t, 0, (e >> 14) & 0x3FFFu, e & 0x3FFFu, G);
+                else code = code_of<kMode>(t, (e >> 19) & 0x1FFu, (e >> 10) & 0x1FFu, e & 0x3FFu, G);
+                if (base + j < a.capacity) a.codes[base + j] = code;
+            }
+            __syncwarp();
+        } else {
+            for (uint32_t k = 0; k < mine; ++k) {
+                bool unused = false;
+                base += warp_triangle<kMode, true>(a, tris[k], t0 + k, k, base, kept, 0u, &unused);
+            }
+        }
     }
+}
+
+// Triangles per warp.
+int voxelize_per(uint64_t n_tri, int mode) {
+    const uint64_t tiles = mode == kVoxGL ? kVoxMinTilesGl : kVoxMinTilesSat;
+    int per = kVoxPer;
+    while (per > 1 && n_tri < tiles * kVoxWarps * per) per >>= 1;
+    return per;
 }
 
 }  // namespace
@@ -494,11 +524,15 @@ void voxelize_configure() {
 
 void launch_voxelize(const VoxArgs& args, int grid, cudaStream_t s) {
     VoxArgs a = args;
+    a.per = voxelize_per(a.n_tri, a.mode);
     for (int k = 0; k < 3; ++k) a.scale[k] = (double)((int64_t)1 << a.depth) / (a.aabb[3 + k] - a.aabb[k]);
     if (a.mode == kVoxGL) voxelize<kVoxGL><<<grid, kVoxThreads, sizeof(VoxSmem<kVoxGL>), s>>>(a);
     else voxelize<kVoxSAT><<<grid, kVoxThreads, sizeof(VoxSmem<kVoxSAT>), s>>>(a);
 }
 
-uint64_t voxelize_tiles(uint64_t n_tri) { return (n_tri + kVoxTile - 1) / kVoxTile; }
+uint64_t voxelize_tiles(uint64_t n_tri, int mode) {
+    const uint64_t tile = (uint64_t)voxelize_per(n_tri, mode) * kVoxWarps;
+    return (n_tri + tile - 1) / tile;
+}
 
 }  // namespace dagc
