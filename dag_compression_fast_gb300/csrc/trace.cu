@@ -31,27 +31,35 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 namespace dagc {
 namespace {
 
 constexpr uint32_t kTraceMaxSteps = 1u << 22;
+constexpr int kTraceThreads = 128;
 constexpr int kTraceMaxDepth = 21;  // the deepest DAG the library builds
 
-__device__ __forceinline__ float max_ref(float a, float b) { return a > b ? a : b; }
-__device__ __forceinline__ float min_ref(float a, float b) { return a < b ? a : b; }
+// The reference's maximum and minimum; kTame: no operand is NaN, and the
+// machine's own differ at most in the sign of a zero, which no later
+// operation tells apart.
+template <bool kTame>
+__device__ __forceinline__ float max_ref(float a, float b) { return kTame ? fmaxf(a, b) : a > b ? a : b; }
+template <bool kTame>
+__device__ __forceinline__ float min_ref(float a, float b) { return kTame ? fminf(a, b) : a < b ? a : b; }
 
-// Children of the node around `path` at `level` that the ray crosses.
-__device__ uint32_t crossed_children(bool root, int depth, int level, const uint32_t path[3], float3 org,
-                                     float3 dir, float3 inv) {
-    const uint32_t shift = (uint32_t)(depth - level);
-    const float radius = float(1u << (shift - 1));
-    const float3 cr = make_float3(radius + float(path[0] << shift) - org.x, radius + float(path[1] << shift) - org.y,
-                                  radius + float(path[2] << shift) - org.z);
+// Children of the node at `pos` (its corner, in voxels), half its edge
+// `radius`, that the ray crosses.
+template <bool kTame>
+__device__ __forceinline__ uint32_t crossed_children(bool root, uint32_t half_edge, const uint32_t pos[3], float3 org,
+                                                     float3 dir, float3 inv) {
+    const float radius = float(half_edge);
+    const float3 cr = make_float3(radius + float(pos[0]) - org.x, radius + float(pos[1]) - org.y,
+                                  radius + float(pos[2]) - org.z);
     const float3 tmid = make_float3(cr.x * inv.x, cr.y * inv.y, cr.z * inv.z);
     const float3 slab = make_float3(radius * fabsf(inv.x), radius * fabsf(inv.y), radius * fabsf(inv.z));
-    const float tmin = max_ref(max_ref(tmid.x - slab.x, max_ref(tmid.y - slab.y, tmid.z - slab.z)), 0.0f);
-    const float tmax = min_ref(tmid.x + slab.x, min_ref(tmid.y + slab.y, tmid.z + slab.z));
+    const float tmin = max_ref<kTame>(max_ref<kTame>(tmid.x - slab.x, max_ref<kTame>(tmid.y - slab.y, tmid.z - slab.z)), 0.0f);
+    const float tmax = min_ref<kTame>(tmid.x + slab.x, min_ref<kTame>(tmid.y + slab.y, tmid.z + slab.z));
     if (root && tmin >= tmax) return 0;
     // The child holding the midpoint of the ray's span inside the node...
     const float half = 0.5f * (tmin + tmax);
@@ -160,54 +168,63 @@ __device__ __forceinline__ float3 ray_direction(const TraceArgs& a, uint32_t px,
     return make_float3(out[0], out[1], out[2]);
 }
 
-__global__ void __launch_bounds__(128) trace_rays(TraceArgs a) {
-    const uint32_t px = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t py = blockIdx.y * blockDim.y + threadIdx.y;
-    if (px >= a.width || py >= a.height) return;
+// The child bytes of a leaf half that are not zero, one bit each: the sum
+// carries into a byte's top bit unless its low seven are zero, and the product
+// moves the four top bits together.
+__device__ __forceinline__ uint32_t nonzero_bytes(uint32_t x) {
+    const uint32_t t = (((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) & 0x80808080u;
+    return ((t >> 7) * 0x01020408u) >> 24;
+}
+
+struct Ray {
+    uint32_t pos[3];       // the voxel hit
+    uint32_t debug_index;
+    bool hit, ok;
+};
+
+// One ray. kNarrow: the words' indices fit 32 bits. kTame: no infinity or NaN
+// comes up (trace_rays).
+template <bool kNarrow, bool kTame>
+__device__ __forceinline__ Ray walk(const TraceArgs& a, float3 org, float3 dir, float3 inv) {
+    using Index = typename std::conditional<kNarrow, uint32_t, uint64_t>::type;
     const int depth = a.depth, leaf_level = depth - 2;
     const uint32_t* w = a.words;
-    const uint64_t nw = a.n_words;
+    const Index nw = (Index)a.n_words;
     bool ok = true;
-    auto word = [&](uint64_t i) -> uint32_t {
+    auto word = [&](Index i) -> uint32_t {
         if (i >= nw) { ok = false; return 0; }
         return __ldg(w + i);
     };
-
-    const float3 org = make_float3(float(a.camera[0]), float(a.camera[1]), float(a.camera[2]));
-    const float3 dir = ray_direction(a, px, py);
-    // 1 / double(dir), rounded to float: the float32 quotient is the same (a
-    // double holds more than twice a float's bits, and no quotient of a
-    // component below 2 is subnormal).
-    const float3 inv = make_float3(__frcp_rn(dir.x), __frcp_rn(dir.y), __frcp_rn(dir.z));
     const uint32_t order = (dir.x < 0.f ? 4u : 0u) + (dir.y < 0.f ? 2u : 0u) + (dir.z < 0.f ? 1u : 0u);
+    const uint32_t debug_at = (uint32_t)(depth - 2) - a.debug_level;  // level entered when the index is noted
 
+    // The levels above that have children left (their bits in `live`), for
+    // the ascent in one step.
     uint64_t stack[kTraceMaxDepth];
-    uint32_t path[3] = {0, 0, 0};
+    uint32_t live = 0;
+    uint32_t pos[3] = {0, 0, 0};
     uint32_t debug_index = 0, leaf_lo = 0, leaf_hi = 0;
     int level = 0;
+    uint32_t edge = 1u << depth;  // of a node at `level`
     uint32_t index = 0;
     uint32_t cm = word(0) & 0xFFu;
-    uint32_t vm = cm & crossed_children(true, depth, 0, path, org, dir, inv);
+    uint32_t vm = cm & crossed_children<kTame>(true, edge >> 1, pos, org, dir, inv);
     bool hit = false;
     for (uint32_t step = 0;; ++step) {
         if (step >= kTraceMaxSteps) { ok = false; break; }
-        // Ascend to the deepest level with a child left.
-        int nl = level;
-        while (nl > 0 && !vm) {
-            --nl;
-            const uint64_t e = stack[nl];
+        if (!vm) {
+            // Ascend to the deepest level with a child left.
+            if (!live) { pos[0] = pos[1] = pos[2] = 0; break; }
+            level = 31 - __clz(live);
+            const uint64_t e = stack[level];
             index = (uint32_t)e;
             cm = (uint32_t)(e >> 32) & 0xFFu;
             vm = (uint32_t)(e >> 40) & 0xFFu;
+            edge = 1u << (depth - level);
+            pos[0] &= 0u - edge;
+            pos[1] &= 0u - edge;
+            pos[2] &= 0u - edge;
         }
-        if (nl == 0 && !vm) {
-            path[0] = path[1] = path[2] = 0;
-            break;
-        }
-        path[0] >>= (level - nl);
-        path[1] >>= (level - nl);
-        path[2] >>= (level - nl);
-        level = nl;
         // Next child in the ray's order: the first set bit of vm after
         // relabelling the children by child ^ order.
         uint32_t seen = vm;
@@ -216,35 +233,60 @@ __global__ void __launch_bounds__(128) trace_rays(TraceArgs a) {
         if (order & 4u) seen = ((seen & 0x0Fu) << 4) | (seen >> 4);
         const uint32_t child = (uint32_t)(__ffs(seen) - 1) ^ order;
         vm &= ~(1u << child);
-        path[0] = (path[0] << 1) | ((child >> 2) & 1u);
-        path[1] = (path[1] << 1) | ((child >> 1) & 1u);
-        path[2] = (path[2] << 1) | (child & 1u);
-        stack[level] = pack(index, cm, vm);
+        edge >>= 1;
+        if (child & 4u) pos[0] |= edge;
+        if (child & 2u) pos[1] |= edge;
+        if (child & 1u) pos[2] |= edge;
+        const uint32_t bit = 1u << level;
+        live &= ~bit;
+        if (vm) {
+            stack[level] = pack(index, cm, vm);
+            live |= bit;
+        }
         ++level;
-        if ((uint32_t)(depth - 2 - level) == a.debug_level) debug_index = index;
+        if ((uint32_t)level == debug_at) debug_index = index;
         if (level == depth) { hit = true; break; }
         if (level <= leaf_level) {
-            const uint32_t ptr = word((uint64_t)index + __popc(cm & ((1u << child) - 1u)) + 1);
+            const uint32_t ptr = word((Index)index + (Index)(__popc(cm & ((1u << child) - 1u)) + 1));
             if (level < leaf_level) {
                 index = ptr;
                 cm = word(index) & 0xFFu;
             } else {
                 leaf_lo = word(ptr);
-                leaf_hi = word((uint64_t)ptr + 1);
+                leaf_hi = word((Index)ptr + 1);
                 // Sub-block b of the leaf is byte b of the 64-bit mask.
-                cm = 0;
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    cm |= ((leaf_lo >> (8 * b)) & 0xFFu) ? 1u << b : 0u;
-                    cm |= ((leaf_hi >> (8 * b)) & 0xFFu) ? 1u << (4 + b) : 0u;
-                }
+                cm = nonzero_bytes(leaf_lo) | nonzero_bytes(leaf_hi) << 4;
             }
         } else {
             cm = (((child & 4u) ? leaf_hi : leaf_lo) >> ((child & 3u) * 8)) & 0xFFu;
         }
-        vm = cm & crossed_children(false, depth, level, path, org, dir, inv);
+        vm = cm & crossed_children<kTame>(false, edge >> 1, pos, org, dir, inv);
         if (!ok) break;
     }
+    return {{pos[0], pos[1], pos[2]}, debug_index, hit, ok};
+}
+
+template <bool kNarrow>
+__global__ void __launch_bounds__(kTraceThreads) trace_rays(TraceArgs a) {
+    const uint32_t px = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t py = blockIdx.y * blockDim.y + threadIdx.y;
+    if (px >= a.width || py >= a.height) return;
+    const int depth = a.depth;
+    const float3 org = make_float3(float(a.camera[0]), float(a.camera[1]), float(a.camera[2]));
+    const float3 dir = ray_direction(a, px, py);
+    // 1 / double(dir), rounded to float: the float32 quotient is the same (a
+    // double holds more than twice a float's bits, and no quotient of a
+    // component below 2 is subnormal).
+    const float3 inv = make_float3(__frcp_rn(dir.x), __frcp_rn(dir.y), __frcp_rn(dir.z));
+    // With a camera below 1e15 and no component below 1e-10, no product of the
+    // walk exceeds 1e26.
+    const bool tame = fminf(fabsf(dir.x), fminf(fabsf(dir.y), fabsf(dir.z))) > 1e-10f &&
+                      fabsf(org.x) < 1e15f && fabsf(org.y) < 1e15f && fabsf(org.z) < 1e15f &&
+                      fabsf(dir.x) + fabsf(dir.y) + fabsf(dir.z) < 4.0f;
+    const Ray ray = tame ? walk<kNarrow, true>(a, org, dir, inv) : walk<kNarrow, false>(a, org, dir, inv);
+    const uint32_t* path = ray.pos;
+    const uint32_t debug_index = ray.debug_index;
+    const bool hit = ray.hit, ok = ray.ok;
     const uint64_t pix = (uint64_t)py * a.width + px;
     a.colors[pix] = a.debug_level == 0xFFFFFFFFu ? channel(path[0]) | channel(path[1]) << 8 | channel(path[2]) << 16
                                                  : murmur32(debug_index);
@@ -283,9 +325,10 @@ void launch_trace(const TraceArgs& args, cudaStream_t s) {
     a.magnitude = finite && most > 1e-6 && most < 1e15 && a.width < (1u << 24) && a.height < (1u << 24)
                       ? (float)(most * 1.0001)
                       : 0.0f;
-    const dim3 block(8, 16);
+    const dim3 block(8, kTraceThreads / 8);
     const dim3 grid((a.width + block.x - 1) / block.x, (a.height + block.y - 1) / block.y);
-    trace_rays<<<grid, block, 0, s>>>(a);
+    if (a.n_words <= 0xFFFFFFF0ull) trace_rays<true><<<grid, block, 0, s>>>(a);
+    else trace_rays<false><<<grid, block, 0, s>>>(a);
 }
 
 }  // namespace dagc
