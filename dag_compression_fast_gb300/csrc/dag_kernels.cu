@@ -808,6 +808,15 @@ __global__ void __launch_bounds__(kT) final_write(FinalArgs a) {
 // ---------------------------------------------------------------------------
 // Small helpers.
 // ---------------------------------------------------------------------------
+// A call's error word and counts to the context's pinned host words: the last
+// kernel of the call, in place of a copy, which the copy engine starts only
+// after a hand-over from the compute engine (the whole call, 2^5 sphere: 112 us
+// with the copies, 102 without).
+__global__ void publish(const uint64_t* __restrict__ in, uint64_t* __restrict__ host, uint32_t n) {
+    pdl_prologue();
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) host[i] = in[i];
+}
+
 __global__ void remap_children(const uint32_t* __restrict__ in, const uint32_t* __restrict__ map,
                                uint32_t* __restrict__ out, uint64_t n_words) {
     pdl_prologue();
@@ -932,6 +941,9 @@ void launch_final_positions(const FinalArgs& a, cudaStream_t s) {
 }
 void launch_final_write(const FinalArgs& a, cudaStream_t s) {
     launch_pdl(final_write, dim3(a.grid_write), dim3(kT), 0, s, a);
+}
+void launch_publish(const uint64_t* in, uint64_t* host, uint32_t n, cudaStream_t s) {
+    launch_pdl(publish, dim3(1), dim3(128), 0, s, in, host, n);
 }
 void launch_remap_children(const uint32_t* in, const uint32_t* map, uint32_t* out, uint64_t n_nodes,
                            cudaStream_t s) {

@@ -62,6 +62,8 @@ struct CallHeader {
     LeafOrder leaf;                     // ordering of the distinct leaf masks
 };
 static_assert(kCntSlots <= kCntWords, "count slots");
+constexpr uint32_t kPublishWords = 1 + 64;  // error word and counts
+static_assert(offsetof(CallHeader, counts) == 8 && sizeof(CallHeader::counts) == 8 * 64, "header");
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -1567,6 +1569,10 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
             t_levels.stop();
         }
         if (cs.sv_next > cs.sv_end) return set_error(ctx, DAGC_ERR_CUDA, "look-back status regions miscounted");
+        // 5. Every count and the error word to the host.
+        launch_publish(reinterpret_cast<const uint64_t*>(cs.h), ctx->h_stage, kPublishWords, s);
+        ++ctx->launches;
+        DAGC_LAUNCHED(ctx);
     return DAGC_OK;
     };
     int st = run_enqueue(ctx, GraphKey{d_frag, n, depth, ctx->arena.base, batch ? batch->k : 0u,
@@ -1576,9 +1582,6 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
                          s, enqueue);
     if (st) { ctx->table_dirty = true; ctx->direct_dirty = true; return st; }
     CallHeader* hdr = reinterpret_cast<CallHeader*>(b + Lo.o_hdr);
-    // 5. One read-back of every count and the error word.
-    static_assert(sizeof(CallHeader) >= 8 * 65, "header");
-    DAGC_CUDA(ctx, cudaMemcpyAsync(ctx->h_stage, hdr, 8 + 8 * 64, cudaMemcpyDeviceToHost, s));
     DAGC_CUDA(ctx, cudaStreamSynchronize(s));
     const uint32_t e32 = (uint32_t)(ctx->h_stage[0] & 0xFFFFFFFFu);
     const uint64_t* counts = ctx->h_stage + 1;
@@ -1745,8 +1748,6 @@ int final_words(dagc_context ctx, const FinalSource& src, cudaStream_t s, uint32
     const size_t o_pos = L.take<uint32_t>(nn + 1);
     char* b = static_cast<char*>(ctx->arena.base);
     CallHeader* h = reinterpret_cast<CallHeader*>(b + o_hdr);
-    // With positions made by the call, its header (at the same place, no error
-    // set) serves on.
     uint32_t* pos = src.word_pos ? src.word_pos : reinterpret_cast<uint32_t*>(b + o_pos);
     if (!src.word_pos) DAGC_CUDA(ctx, cudaMemsetAsync(b, 0, zero_bytes, s));
     FinalArgs a{};
@@ -1763,7 +1764,10 @@ int final_words(dagc_context ctx, const FinalSource& src, cudaStream_t s, uint32
     a.d_total = &h->counts[0];
     a.status = reinterpret_cast<uint64_t*>(b + o_sv);
     a.tile_counter = &h->tile_counters[0];
-    a.err = &h->err;
+    // After a call that made the positions only the write's own finding is
+    // left to learn: it goes to the pinned host word itself.
+    a.err = src.word_pos ? reinterpret_cast<uint32_t*>(ctx->h_stage) : &h->err;
+    if (src.word_pos) ctx->h_stage[0] = 0;
     a.grid_scan = grid_for(ctx->grid_scan / ctx->sms, ctx->sms, scan_tiles(nn));
     a.grid_write = grid_for(ctx->grid_write / ctx->sms, ctx->sms, (nn + src.num_leaves + 255) / 256);
     // Words: at most 1 + 8 per node and 2 per leaf. Allocating that bound
@@ -1797,7 +1801,8 @@ int final_words(dagc_context ctx, const FinalSource& src, cudaStream_t s, uint32
     ++ctx->launches;
     t.stop();
     cudaError_t le = cudaGetLastError();
-    if (le == cudaSuccess) le = cudaMemcpyAsync(ctx->h_stage, h, 16, cudaMemcpyDeviceToHost, s);  // err, counts[0]
+    if (le == cudaSuccess && !src.word_pos)
+        le = cudaMemcpyAsync(ctx->h_stage, h, 16, cudaMemcpyDeviceToHost, s);  // err, counts[0]
     if (le == cudaSuccess) le = cudaStreamSynchronize(s);
     if (le != cudaSuccess) {
         ctx->pool.release(w);

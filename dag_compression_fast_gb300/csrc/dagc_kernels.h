@@ -555,6 +555,8 @@ struct CopyTable {
     int lit_count;
 };
 void launch_copy_segments(const CopyTable& t, cudaStream_t s);
+// n words to pinned host memory (a call's counts).
+void launch_publish(const uint64_t* in, uint64_t* host, uint32_t n, cudaStream_t s);
 
 void kernels_configure();
 
