@@ -63,6 +63,9 @@ struct CallHeader {
 };
 static_assert(kCntSlots <= kCntWords, "count slots");
 constexpr uint32_t kPublishWords = 1 + 64;  // error word and counts
+constexpr uint32_t kStagedRoots = 256;      // roots of a merge, after them
+constexpr size_t kStageBytes = 4096;        // a context's pinned words
+static_assert(8 * kPublishWords + 12 * kStagedRoots <= kStageBytes, "pinned words");
 static_assert(offsetof(CallHeader, counts) == 8 && sizeof(CallHeader::counts) == 8 * 64, "header");
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -372,7 +375,6 @@ struct dagc_context_t {
     uint64_t direct_cap = 0;
     bool direct_dirty = true;
     uint64_t fallbacks = 0;  // calls rerun with the radix form
-    uint32_t* trace_err = nullptr;  // tracer error word
     void* vox_scratch = nullptr;    // voxelizer counters and look-back status
     size_t vox_scratch_bytes = 0;
     std::string last_error;
@@ -1801,8 +1803,11 @@ int final_words(dagc_context ctx, const FinalSource& src, cudaStream_t s, uint32
     ++ctx->launches;
     t.stop();
     cudaError_t le = cudaGetLastError();
-    if (le == cudaSuccess && !src.word_pos)
-        le = cudaMemcpyAsync(ctx->h_stage, h, 16, cudaMemcpyDeviceToHost, s);  // err, counts[0]
+    if (le == cudaSuccess && !src.word_pos) {
+        launch_publish(reinterpret_cast<const uint64_t*>(h), ctx->h_stage, 2, s);  // err, counts[0]
+        ++ctx->launches;
+        le = cudaGetLastError();
+    }
     if (le == cudaSuccess) le = cudaStreamSynchronize(s);
     if (le != cudaSuccess) {
         ctx->pool.release(w);
@@ -2178,19 +2183,33 @@ int union_hash(dagc_context ctx, dagc_dag* in, uint64_t k_all, cudaStream_t s, u
         ga.err = &h->err;
         ctx->launches += launch_group_dedup(ga, items, s);
     }
+    // The roots of up to kStagedRoots inputs go to the pinned words themselves.
+    const bool staged = k <= kStagedRoots;
+    if (staged) {
+        m.root_hash = ctx->h_stage + kPublishWords;
+        m.root_uid = reinterpret_cast<uint32_t*>(m.root_hash + k);
+    }
     launch_merge_roots(m, s);
     ++ctx->launches;
     t_merge.stop();
     cudaError_t e = cudaGetLastError();
     std::vector<uint64_t> stage_hash(k, 0);
     std::vector<uint32_t> stage_uid(k, 0);
-    if (!e) e = cudaMemcpyAsync(stage_hash.data(), m.root_hash, k * 8ull, cudaMemcpyDeviceToHost, s);
-    if (!e) e = cudaMemcpyAsync(stage_uid.data(), m.root_uid, k * 4ull, cudaMemcpyDeviceToHost, s);
-    if (!e) e = cudaMemcpyAsync(ctx->h_stage, h, 8 + 8 * 64, cudaMemcpyDeviceToHost, s);
+    if (!e && !staged) e = cudaMemcpyAsync(stage_hash.data(), m.root_hash, k * 8ull, cudaMemcpyDeviceToHost, s);
+    if (!e && !staged) e = cudaMemcpyAsync(stage_uid.data(), m.root_uid, k * 4ull, cudaMemcpyDeviceToHost, s);
+    if (!e) {
+        launch_publish(reinterpret_cast<const uint64_t*>(h), ctx->h_stage, kPublishWords, s);
+        ++ctx->launches;
+        e = cudaGetLastError();
+    }
     const cudaError_t es = cudaStreamSynchronize(s);  // also before the host vectors go
     if (!e) e = es;
     if (e != cudaSuccess) ctx->table_dirty = true;
     DAGC_CUDA(ctx, e);
+    if (staged) {
+        std::memcpy(stage_hash.data(), m.root_hash, k * 8ull);
+        std::memcpy(stage_uid.data(), m.root_uid, k * 4ull);
+    }
     settle_profile(ctx);
     const uint32_t e32 = (uint32_t)(ctx->h_stage[0] & 0xFFFFFFFFu);
     if (e32) ctx->table_dirty = true;
@@ -2507,7 +2526,7 @@ int dagc_context_create(int device, dagc_context* out) {
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
     sort_configure();
     kernels_configure();
-    e = cudaMallocHost(&c->h_stage, 4096);
+    e = cudaMallocHost(&c->h_stage, kStageBytes);
     if (e != cudaSuccess) { cudaGetLastError(); return cuda_status(e); }
     if (cudaStreamCreateWithFlags(&c->capture_stream, cudaStreamNonBlocking) != cudaSuccess) {
         cudaGetLastError();
@@ -2595,7 +2614,6 @@ void dagc_context_destroy(dagc_context ctx) {
     if (ctx->table) cudaFree(ctx->table);
     if (ctx->gtable) cudaFree(ctx->gtable);
     release_direct(ctx);
-    if (ctx->trace_err) cudaFree(ctx->trace_err);
     if (ctx->vox_scratch) cudaFree(ctx->vox_scratch);
     ctx->pool.trim();
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
@@ -3175,8 +3193,7 @@ int dagc_trace(dagc_context ctx, const uint32_t* d_words, uint64_t n_words, int 
         return set_error(ctx, DAGC_ERR_INVALID_ARGUMENT, "image too large");
     DAGC_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (!ctx->trace_err) DAGC_CUDA(ctx, cudaMalloc(&ctx->trace_err, 256));
-    DAGC_CUDA(ctx, cudaMemsetAsync(ctx->trace_err, 0, 4, s));
+    ctx->h_stage[0] = 0;  // the rays' error word, in pinned memory
     TraceArgs a{};
     a.words = d_words;
     a.n_words = n_words;
@@ -3192,14 +3209,12 @@ int dagc_trace(dagc_context ctx, const uint32_t* d_words, uint64_t n_words, int 
     }
     a.colors = d_colors;
     a.hits = d_hits;
-    a.err = ctx->trace_err;
+    a.err = reinterpret_cast<uint32_t*>(ctx->h_stage);
     launch_trace(a, s);
     ++ctx->launches;
     DAGC_LAUNCHED(ctx);
-    uint32_t err = 0;
-    DAGC_CUDA(ctx, cudaMemcpyAsync(&err, ctx->trace_err, 4, cudaMemcpyDeviceToHost, s));
     DAGC_CUDA(ctx, cudaStreamSynchronize(s));
-    if (err) return set_error(ctx, DAGC_ERR_BAD_INPUT, "the word array is not a valid final DAG of this depth");
+    if (ctx->h_stage[0]) return set_error(ctx, DAGC_ERR_BAD_INPUT, "the word array is not a valid final DAG of this depth");
     return DAGC_OK;
 }
 
@@ -3246,9 +3261,12 @@ int dagc_voxelize(dagc_context ctx, const double* d_vertices, uint64_t n_triangl
     launch_voxelize(a, grid, s);
     ++ctx->launches;
     DAGC_LAUNCHED(ctx);
-    uint64_t h[3] = {0, 0, 0};
-    DAGC_CUDA(ctx, cudaMemcpyAsync(h, b, 24, cudaMemcpyDeviceToHost, s));
+    t_pdl = ctx->pdl;
+    launch_publish(reinterpret_cast<const uint64_t*>(b), ctx->h_stage, 3, s);
+    ++ctx->launches;
+    DAGC_LAUNCHED(ctx);
     DAGC_CUDA(ctx, cudaStreamSynchronize(s));
+    const uint64_t* h = ctx->h_stage;
     if ((uint32_t)h[2]) return set_error(ctx, DAGC_ERR_DEVICE_TIMEOUT, "a bounded device wait ran out");
     *n_codes = h[0];
     if (h[0] > capacity) return set_error(ctx, DAGC_ERR_TOO_LARGE, "fragment buffer too small (see n_codes)");
