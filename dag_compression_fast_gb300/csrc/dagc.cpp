@@ -2689,7 +2689,7 @@ int dagc_create_batched(dagc_context ctx, const uint64_t* d_fragments, const uin
 
 uint64_t dagc_create_footprint(uint64_t n, int depth) {
     if (depth < 2 || depth > kMaxDepth || n == 0) return 0;
-    const CreateLayout L(n, depth, 0, true, kDedupMaxUnique, true);
+    const CreateLayout L(n, depth, 0, true, kDedupMaxUnique, true, 0, direct_table_applies(n, depth));
     return L.total + L.table_slots * 16 + kGroupScratchBytes + (direct_table_applies(n, depth) ? direct_entries(depth) * 8 : 0);
 }
 

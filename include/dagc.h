@@ -248,14 +248,14 @@ int dagc_dedup_fallbacks(dagc_context ctx, uint64_t* count);
  * accumulate per stage until dagc_profile_reset. The fragment-sort digit passes
  * are bracketed one launch at a time. */
 #define DAGC_STAGE_FRAGMENT_HIST 0  /* histogram + key-range check of the fragment sort */
-#define DAGC_STAGE_FRAGMENT_PASS 1  /* one 8-bit digit pass of the fragment sort */
-#define DAGC_STAGE_LEAF_BUILD 2     /* fused unique + 4x4x4 leaf build */
-#define DAGC_STAGE_LEAF_DEDUP 3     /* leaf sort + unique */
-#define DAGC_STAGE_LEVELS 4         /* every inner level: extract, hash, sort, unique */
+#define DAGC_STAGE_FRAGMENT_PASS 1  /* one digit pass of the fragment sort */
+#define DAGC_STAGE_LEAF_BUILD 2     /* fused unique + 4x4x4 leaf build; the direct-mapped table's marking and compaction */
+#define DAGC_STAGE_LEAF_DEDUP 3     /* distinct leaf masks found and ordered */
+#define DAGC_STAGE_LEVELS 4         /* every inner level: extracted, hashed, deduplicated */
 #define DAGC_STAGE_MATERIALISE 5    /* copy of the level outputs into the DAG */
 #define DAGC_STAGE_FINAL 6          /* final word layout */
 #define DAGC_STAGE_MERGE 7          /* MergeDAGs */
-#define DAGC_STAGE_GROUP 8             /* fragment grouping by hash: brick sort, gather */
+#define DAGC_STAGE_GROUP 8             /* fragment grouping by hash: the bricks in order */
 #define DAGC_STAGE_GROUP_SKETCH 9      /* its probe (a sampled sketch of the distinct bricks) and the path choice */
 #define DAGC_STAGE_GROUP_AGGREGATE 10  /* its per-partition tables (one read of the partitioned fragments) */
 #define DAGC_STAGE_GROUP_SCATTER 11    /* its partitioning (one read and one write of the fragments) */
