@@ -29,7 +29,7 @@
 // part can run beside it. When each level was deduplicated before the next was
 // extracted (four launches per level, and the tail's sorts one after another),
 // the levels of a 512^3 terrain took 107 us, now 68 (and half of that beside the
-// leaves: the call 217 -> 143); of the 8192^3 soup 2.36 ms, now 1.64.
+// leaves: the call 217 -> 143 by that step); of the 8192^3 soup 2.36 ms, now 1.64.
 
 #include "dagc_device.cuh"
 #include "dagc_kernels.h"
