@@ -25,7 +25,7 @@
 // look-back. The output order is fixed: triangles in input order, each
 // triangle's fragments in bounding-box order. A call without room for codes
 // only counts. This file is compiled with --fmad=false: every float operation
-// rounds once, as in the CPU checkers (but for the explicit fmaf of the SAT
+// rounds once, as in the CPU oracle (but for the explicit fmaf of the SAT
 // filter, whose error bound covers it).
 //
 // Each form is bound by the arithmetic per candidate (2.7 instructions per SM
@@ -247,7 +247,7 @@ __device__ bool tri_box(D3 c, double h, D3 a, D3 b, D3 d) {
 __device__ __forceinline__ D3 sat_vertex(const double* P, const double* aabb, const double* scale, int k) {
     return {(P[3 * k + 0] - aabb[0]) * scale[0], (P[3 * k + 1] - aabb[1]) * scale[1], (P[3 * k + 2] - aabb[2]) * scale[2]};
 }
-// The rule itself, for one voxel: float64, in the checkers' order.
+// The rule itself, for one voxel: float64, in the oracle's order.
 __device__ __noinline__ bool sat_exact(const VoxArgs& a, uint64_t tri, int64_t x, int64_t y, int64_t z) {
     const double* P = a.vertices + 9 * tri;
     const D3 c{(double)x + 0.5, (double)y + 0.5, (double)z + 0.5};
