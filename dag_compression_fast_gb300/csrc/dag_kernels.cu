@@ -715,6 +715,15 @@ __device__ __forceinline__ int level_of(const FinalLevels& L, int num_levels, ui
     return l;
 }
 
+// The same, searching down from the last level, which with the one above holds
+// most of the nodes (both kernels are half ALU-bound: 14.4M nodes in 11 levels
+// 250 -> 233 us).
+__device__ __forceinline__ int level_of(const FinalLevels& L, int num_levels, uint64_t i) {
+    int l = num_levels - 1;
+    while (l > 0 && i < L.off[l]) --l;
+    return l;
+}
+
 // word_pos[i] = sum over nodes j < i of (popc(mask_j) + 1); word_pos[n] = total.
 __global__ void __launch_bounds__(kT) final_positions(FinalArgs a) {
     pdl_prologue();
@@ -731,7 +740,7 @@ __global__ void __launch_bounds__(kT) final_positions(FinalArgs a) {
         const uint64_t i0 = (uint64_t)tile * kTile + (uint64_t)tid * kI;
         uint32_t w[kI];
         uint32_t sum = 0;
-        int l = level_of(LV, a.num_levels, i0, 0);
+        int l = level_of(LV, a.num_levels, i0);
 #pragma unroll
         for (int j = 0; j < kI; ++j) {
             w[j] = 0;
@@ -779,7 +788,7 @@ __global__ void __launch_bounds__(kT) final_write(FinalArgs a) {
             a.words[leaf_start + 2 * j + 1] = (uint32_t)(leaf >> 32);
             continue;
         }
-        const int l = level_of(LV, a.num_levels, i, 0);
+        const int l = level_of(LV, a.num_levels, i);
         const bool last = l + 1 == a.num_levels;
         const uint64_t li = i - s_off[l];
         const uint32_t mask = LV.masks[l][li];
