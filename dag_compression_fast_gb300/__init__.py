@@ -39,6 +39,7 @@ OPT_TEST_SPIN_LIMIT = 9
 OPT_TEST_STALL_LOOKBACK = 10
 OPT_TEST_FAIL_ALLOCS = 11
 OPT_BATCH_PATH = 12
+OPT_TEST_FAIL_BESIDE = 13
 VOXELIZE_GL = 0
 VOXELIZE_SAT = 1
 NUM_KEY_SHAPES = 9

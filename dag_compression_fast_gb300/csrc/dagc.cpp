@@ -356,6 +356,7 @@ struct dagc_context_t {
     Arena arena;
     uint32_t test_spin_limit = 0;  // DAGC_OPT_TEST_SPIN_LIMIT (0: kSpinLimit)
     int test_stall = 0;            // DAGC_OPT_TEST_STALL_LOOKBACK
+    bool test_fail_beside = false;  // DAGC_OPT_TEST_FAIL_BESIDE
     // Dedup table: keys (0 = empty), then aux words; every level leaves its
     // keys zero; after a call that stopped early it is cleared. Grouping
     // scratch (kGroupScratchBytes): the brick masks.
@@ -484,6 +485,33 @@ struct StageTimer {
         cudaEventRecord(b, s);
         ctx->pending.push_back({stage, a, b, ctx->launches - launches0, bytes});
         a = nullptr;
+    }
+};
+
+// Work on the context's side stream beside a call's stream, from fork to join. A
+// call that returns in between joins it all the same: the next call writes the
+// same arena, and a recording must not end with a branch left open.
+struct SideWork {
+    dagc_context ctx;
+    cudaStream_t s;
+    bool open = false;
+    SideWork(dagc_context c, cudaStream_t stream) : ctx(c), s(stream) {}
+    cudaError_t fork() {
+        const cudaError_t e = cudaEventRecord(ctx->side_fork, s);
+        if (e != cudaSuccess) return e;
+        open = true;
+        return cudaStreamWaitEvent(ctx->side_stream, ctx->side_fork, 0);
+    }
+    // The end of the side work; work queued on `s` after join() follows it.
+    cudaError_t done() { return cudaEventRecord(ctx->side_join, ctx->side_stream); }
+    cudaError_t join() {
+        open = false;
+        return cudaStreamWaitEvent(s, ctx->side_join, 0);
+    }
+    ~SideWork() {
+        if (!open) return;
+        if (done() != cudaSuccess || join() != cudaSuccess) cudaStreamSynchronize(ctx->side_stream);
+        cudaGetLastError();
     }
 };
 
@@ -1358,12 +1386,13 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
                 }
             };
             const bool beside = ctx->side_stream && !ctx->profiling && !ctx->pdl && nl > 0;
+            SideWork side(ctx, s);
             if (beside) {
-                DAGC_CUDA(ctx, cudaEventRecord(ctx->side_fork, s));
-                DAGC_CUDA(ctx, cudaStreamWaitEvent(ctx->side_stream, ctx->side_fork, 0));
+                DAGC_CUDA(ctx, side.fork());
                 extract_all(ctx->side_stream);
-                DAGC_CUDA(ctx, cudaEventRecord(ctx->side_join, ctx->side_stream));
+                DAGC_CUDA(ctx, side.done());
                 DAGC_LAUNCHED(ctx);
+                if (ctx->test_fail_beside) return set_error(ctx, DAGC_ERR_CUDA, "failed on request (test hook)");
             } else {
                 StageTimer t(ctx, DAGC_STAGE_LEVELS, s);
                 extract_all(s);
@@ -1401,7 +1430,7 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
             ctx->launches += 2;
             DAGC_LAUNCHED(ctx);
             t_dedup.stop();
-            if (beside) DAGC_CUDA(ctx, cudaStreamWaitEvent(s, ctx->side_join, 0));
+            if (beside) DAGC_CUDA(ctx, side.join());
             // The node levels' dedup, a group of levels at a time, bottom up.
             StageTimer t_levels(ctx, DAGC_STAGE_LEVELS, s);
             uint32_t* maps[2] = {P32(Lo.o_M0), P32(Lo.o_M1)};
@@ -1582,9 +1611,18 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
                                        use_dedup ? ctx->table : nullptr, use_dedup ? group_mode : 0,
                                        direct_table ? ctx->direct : nullptr, words},
                          s, enqueue);
-    if (st) { ctx->table_dirty = true; ctx->direct_dirty = true; return st; }
+    if (st) {
+        // What was queued before the error still writes the arena and the tables.
+        cudaStreamSynchronize(s);
+        cudaGetLastError();
+        ctx->table_dirty = true;
+        ctx->direct_dirty = true;
+        return st;
+    }
     CallHeader* hdr = reinterpret_cast<CallHeader*>(b + Lo.o_hdr);
-    DAGC_CUDA(ctx, cudaStreamSynchronize(s));
+    const cudaError_t es = cudaStreamSynchronize(s);
+    if (es != cudaSuccess) ctx->table_dirty = ctx->direct_dirty = true;
+    DAGC_CUDA(ctx, es);
     const uint32_t e32 = (uint32_t)(ctx->h_stage[0] & 0xFFFFFFFFu);
     const uint64_t* counts = ctx->h_stage + 1;
     ctx->last_counts.assign(3 + nl, 0);
@@ -3054,6 +3092,9 @@ int dagc_set_option(dagc_context ctx, int option, int value) {
         case DAGC_OPT_TEST_STALL_LOOKBACK:
             ctx->test_stall = value != 0;
             ++ctx->tune_version;
+            return DAGC_OK;
+        case DAGC_OPT_TEST_FAIL_BESIDE:
+            ctx->test_fail_beside = value != 0;
             return DAGC_OK;
         case DAGC_OPT_TEST_FAIL_ALLOCS:
             if (value < 0) return set_error(ctx, DAGC_ERR_INVALID_ARGUMENT, "count must be >= 0");

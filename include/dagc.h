@@ -233,10 +233,13 @@ int dagc_last_counts(dagc_context ctx, uint64_t* out, int cap);
  * first digit pass of every sort leave its tile 0 unpublished, so the waits of
  * the tiles after it run out and the call returns DAGC_ERR_DEVICE_TIMEOUT (the
  * context stays usable). TEST_FAIL_ALLOCS: the context's next `value` device
- * allocations fail as on a full device (dagc_memory_events counts them). */
+ * allocations fail as on a full device (dagc_memory_events counts them).
+ * TEST_FAIL_BESIDE: 1 makes every CreateDAG call that queues work beside its
+ * stream return DAGC_ERR_CUDA while that work runs. */
 #define DAGC_OPT_TEST_SPIN_LIMIT 9
 #define DAGC_OPT_TEST_STALL_LOOKBACK 10
 #define DAGC_OPT_TEST_FAIL_ALLOCS 11
+#define DAGC_OPT_TEST_FAIL_BESIDE 13
 int dagc_set_option(dagc_context ctx, int option, int value);
 /* Calls of this context rerun in the radix form so far. */
 int dagc_dedup_fallbacks(dagc_context ctx, uint64_t* count);
