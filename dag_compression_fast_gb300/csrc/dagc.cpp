@@ -2143,10 +2143,14 @@ int union_hash(dagc_context ctx, dagc_dag* in, uint64_t k_all, cudaStream_t s, u
         o_pm[l] = L.take<uint8_t>(level_total[l]);
     }
     const size_t o_root_hash = L.take<uint64_t>(k), o_root_uid = L.take<uint32_t>(k);
-    DAGC_CUDA(ctx, ctx->arena.reserve(L.off));
+    // The table and the buckets (up to 16 KB per 128 nodes) are more than the
+    // sorts take: without room for them the union goes by sorts.
+    const cudaError_t room = ctx->arena.reserve(L.off);
+    if (room == cudaErrorMemoryAllocation) return kStatusFallback;
+    DAGC_CUDA(ctx, room);
     arena_wait(ctx, s);
     int st = reserve_table(ctx, std::max(leaf_slots_upto(total_leaves), G.table_slots), s, false);
-    if (st) return st;
+    if (st) return st == DAGC_ERR_OUT_OF_MEMORY ? kStatusFallback : st;
     for (uint32_t j = 0; j < k; ++j) dag_ready_wait(in[live[j]], s);
     char* b = static_cast<char*>(ctx->arena.base);
     auto P64 = [&](size_t o) { return reinterpret_cast<uint64_t*>(b + o); };
