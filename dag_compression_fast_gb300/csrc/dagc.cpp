@@ -12,6 +12,7 @@
 
 #include "../../include/dagc.h"
 #include "dagc_hash.h"
+#include "dagc_internal.h"
 #include "dagc_kernels.h"
 #include "dagc_launch.h"
 
@@ -70,7 +71,7 @@ static_assert(offsetof(CallHeader, counts) == 8 && sizeof(CallHeader::counts) ==
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-// Device allocations of a context go through here: a test hook can make the
+// All device allocations of a context go through here: a test hook can make the
 // next `inject` of them fail as cudaMalloc does when the device is full
 // (cudaErrorMemoryAllocation), without touching the device.
 struct AllocStats {
@@ -1017,6 +1018,45 @@ void release_direct(dagc_context ctx) {
     ctx->direct_dirty = true;
 }
 
+// Every context of the process. A brick table is only kept to save its next
+// allocation: when an allocation of any context fails, the tables of the
+// others on its device that are between calls go too.
+struct Contexts {
+    std::mutex mu;
+    std::vector<dagc_context> all;
+};
+Contexts& contexts() {
+    static Contexts* c = new Contexts;  // contexts may outlive the static objects
+    return *c;
+}
+
+// With ctx->mu held.
+void give_back_tables(dagc_context ctx) {
+    release_direct(ctx);
+    Contexts& all = contexts();
+    std::lock_guard<std::mutex> lock(all.mu);
+    for (dagc_context c : all.all) {
+        if (c == ctx || c->device != ctx->device || !c->mu.try_lock()) continue;
+        release_direct(c);
+        c->mu.unlock();
+    }
+}
+
+// A device allocation outside the pool and the arena, retried like theirs once
+// the pool's cache and the brick tables are given back.
+cudaError_t ctx_malloc(dagc_context ctx, void** p, size_t bytes) {
+    cudaError_t e = dev_malloc(p, bytes, &ctx->alloc_stats);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        ctx->pool.trim();
+        give_back_tables(ctx);
+        e = dev_malloc(p, bytes, &ctx->alloc_stats);
+        if (e == cudaSuccess) ++ctx->alloc_stats.retries_ok;
+    }
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
+}
+
 // Grows the context's dedup table to `slots` (zeroed); clears it after a call
 // that may have stopped between an insert and its map.
 int reserve_table(dagc_context ctx, uint64_t slots, cudaStream_t s, bool grouping) {
@@ -1024,14 +1064,7 @@ int reserve_table(dagc_context ctx, uint64_t slots, cudaStream_t s, bool groupin
         if (ctx->table) cudaFree(ctx->table);
         ctx->table = nullptr;
         ctx->table_cap = 0;
-        cudaError_t e = cudaMalloc(&ctx->table, slots * 16);  // per slot: key u64, aux u64
-        if (e == cudaErrorMemoryAllocation && ctx->direct) {
-            cudaGetLastError();
-            release_direct(ctx);
-            e = cudaMalloc(&ctx->table, slots * 16);
-        }
-        if (e != cudaSuccess) ctx->table = nullptr;
-        DAGC_CUDA(ctx, e);
+        DAGC_CUDA(ctx, ctx_malloc(ctx, &ctx->table, slots * 16));  // per slot: key u64, aux u64
         ctx->table_cap = slots;
         ctx->table_dirty = true;
     }
@@ -1039,7 +1072,7 @@ int reserve_table(dagc_context ctx, uint64_t slots, cudaStream_t s, bool groupin
         DAGC_CUDA(ctx, cudaMemsetAsync(ctx->table, 0, ctx->table_cap * 16, s));
         ctx->table_dirty = false;
     }
-    if (!ctx->gtable && grouping) DAGC_CUDA(ctx, cudaMalloc(&ctx->gtable, kGroupScratchBytes));
+    if (!ctx->gtable && grouping) DAGC_CUDA(ctx, ctx_malloc(ctx, &ctx->gtable, kGroupScratchBytes));
     return DAGC_OK;
 }
 
@@ -1071,7 +1104,7 @@ bool reserve_direct(dagc_context ctx, uint64_t entries, cudaStream_t s) {
     if (entries > ctx->direct_cap) {
         void* p = nullptr;
         release_direct(ctx);
-        if (cudaMalloc(&p, entries * 8) != cudaSuccess) { cudaGetLastError(); return false; }
+        if (dev_malloc(&p, entries * 8, &ctx->alloc_stats) != cudaSuccess) { cudaGetLastError(); return false; }
         ctx->direct = p;
         ctx->direct_cap = entries;
         ctx->direct_dirty = true;
@@ -2534,6 +2567,11 @@ bool valid_ctx(dagc_context ctx) { return ctx != nullptr; }
 
 }  // namespace
 
+cudaError_t dagc::context_malloc(dagc_context ctx, void** p, size_t bytes) {
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    return ctx_malloc(ctx, p, bytes);
+}
+
 // ===================================================================== C ABI
 extern "C" {
 
@@ -2564,7 +2602,7 @@ int dagc_context_create(int device, dagc_context* out) {
     c->device = device;
     c->pool.stats = &c->alloc_stats;
     c->arena.stats = &c->alloc_stats;
-    c->pool.on_oom = c->arena.on_oom = [p = c.get()] { release_direct(p); };
+    c->pool.on_oom = c->arena.on_oom = [p = c.get()] { give_back_tables(p); };
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
     sort_configure();
     kernels_configure();
@@ -2635,12 +2673,21 @@ int dagc_context_create(int device, dagc_context* out) {
     levels_configure(c->sms);
     chunk_configure(c->sms);
     voxelize_configure();
+    {
+        std::lock_guard<std::mutex> lock(contexts().mu);
+        contexts().all.push_back(c.get());
+    }
     *out = c.release();
     return DAGC_OK;
 }
 
 void dagc_context_destroy(dagc_context ctx) {
     if (!ctx) return;
+    {
+        std::lock_guard<std::mutex> lock(contexts().mu);
+        std::vector<dagc_context>& all = contexts().all;
+        all.erase(std::remove(all.begin(), all.end(), ctx), all.end());
+    }
     cudaSetDevice(ctx->device);
     cudaDeviceSynchronize();
     settle_profile(ctx);
@@ -3285,7 +3332,7 @@ int dagc_voxelize(dagc_context ctx, const double* d_vertices, uint64_t n_triangl
         if (ctx->vox_scratch) cudaFree(ctx->vox_scratch);
         ctx->vox_scratch = nullptr;
         ctx->vox_scratch_bytes = 0;
-        DAGC_CUDA(ctx, cudaMalloc(&ctx->vox_scratch, bytes));
+        DAGC_CUDA(ctx, ctx_malloc(ctx, &ctx->vox_scratch, bytes));
         ctx->vox_scratch_bytes = bytes;
     }
     char* b = static_cast<char*>(ctx->vox_scratch);

@@ -18,6 +18,7 @@
 // the server was created, so overlap of jobs on the device can be read off.
 
 #include "../../include/dagc.h"
+#include "dagc_internal.h"
 
 #include <algorithm>
 #include <chrono>
@@ -135,7 +136,7 @@ void worker_loop(dagc_server_t* sv, int slot) {
                 if (stage) cudaFree(stage);
                 stage = nullptr;
                 stage_cap = 0;
-                if (cudaMalloc(&stage, r->n * 8) != cudaSuccess) { cudaGetLastError(); st = DAGC_ERR_OUT_OF_MEMORY; }
+                if (dagc::context_malloc(ctx, &stage, r->n * 8) != cudaSuccess) { cudaGetLastError(); st = DAGC_ERR_OUT_OF_MEMORY; }
                 else stage_cap = r->n;
             }
             if (!st && r->n && cudaMemcpyAsync(stage, r->h_fragments, r->n * 8, cudaMemcpyHostToDevice, stream) != cudaSuccess) {

@@ -25,3 +25,89 @@ def test_a_union_without_room_for_the_hash_set_goes_by_sorts():
         assert_dag_equal(c.lift_dag(body, roots).to_host(), O.create_dag(codes, 9))
         assert_dag_equal(c.merge_dags(dags).to_host(), O.create_dag(codes, 9))  # by hash set again
         assert c.dedup_fallbacks() == before + 1
+
+
+def test_a_union_without_room_for_the_table_goes_by_sorts():
+    parts = [random_codes(10, 60_000, 60 + i) for i in range(4)]
+    with D.Context(0) as c, D.Context(0) as other:
+        dags = [other.create_dag(p, 10) for p in parts]
+        ref = other.union_dags(dags)[0].to_host()
+        # A context with a large arena and a small table: many fragments of few bricks, through the radix sort.
+        c.set_option(D.OPT_GROUP, 0)
+        c.create_dag(random_codes(4, 20_000_000, 64), 4).free()
+        before, fell = c.memory_events(), c.dedup_fallbacks()
+        c.set_option(D.OPT_TEST_FAIL_ALLOCS, 2)  # the table's allocation and its retry
+        got = c.union_dags(dags)[0].to_host()
+        assert c.memory_events()["alloc_failures"] == before["alloc_failures"] + 2
+        assert c.dedup_fallbacks() == fell + 1
+        assert_dag_equal(got, ref)
+
+
+def has_brick_table(c):
+    return "brick table" in c.memory_report()
+
+
+def test_idle_brick_tables_are_given_back_to_any_allocation():
+    """The voxelizer's scratch in one context takes the idle tables of both; each is taken again and exact."""
+    codes = random_codes(10, 30_000, 71)
+    ref = O.final_dag(O.create_dag(codes, 10))
+    tri = np.random.default_rng(72).uniform(0, 64, (5_000, 9))
+    with D.Context(0) as a, D.Context(0) as b:
+        for c in (a, b):
+            assert np.array_equal(c.compress(codes, 10).to_numpy(), ref)
+            assert has_brick_table(c)
+        before = a.memory_events()
+        a.set_option(D.OPT_TEST_FAIL_ALLOCS, 1)
+        a.voxelize(tri, (0, 0, 0, 64, 64, 64), 6)
+        after = a.memory_events()
+        assert (after["alloc_failures"], after["retries_ok"]) == (before["alloc_failures"] + 1, before["retries_ok"] + 1)
+        assert not has_brick_table(a) and not has_brick_table(b)
+        for c in (a, b):
+            for _ in range(3):
+                assert np.array_equal(c.compress(codes, 10).to_numpy(), ref)
+            assert has_brick_table(c)
+
+
+@pytest.mark.parametrize("graphs", [0, 1])
+def test_a_call_without_room_for_the_brick_table(graphs):
+    """Only the table's allocation fails: the call does without it, the next one takes it."""
+    import torch
+    big = random_codes(9, 1_500_000, 81)
+    codes = torch.from_numpy(random_codes(10, 20_000, 82).view(np.int64)).cuda()
+    ref = O.final_dag(O.create_dag(codes.cpu().numpy().view(np.uint64), 10))
+    with D.Context(0) as c:
+        c.set_option(D.OPT_GRAPHS, graphs)
+        c.set_option(D.OPT_GROUP, 2)
+        c.compress(big, 9).free()  # scratch and tables larger than the next call's, but for the brick table
+        c.set_option(D.OPT_GROUP, 1)
+        for turn in range(2):
+            before = c.memory_events()
+            c.set_option(D.OPT_TEST_FAIL_ALLOCS, 1)
+            assert np.array_equal(c.compress(codes, 10).to_numpy(), ref)
+            after = c.memory_events()
+            assert (after["alloc_failures"], after["retries_ok"]) == (before["alloc_failures"] + 1, before["retries_ok"])
+            assert not has_brick_table(c)
+            for _ in range(3):
+                assert np.array_equal(c.compress(codes, 10).to_numpy(), ref)
+            assert has_brick_table(c)
+            if turn == 0:
+                c.voxelize(np.zeros((1, 9)), (0, 0, 0, 1, 1, 1), 1)
+                c.set_option(D.OPT_TEST_FAIL_ALLOCS, 1)  # takes the table back for the second turn
+                c.voxelize(np.zeros((90_000, 9)), (0, 0, 0, 1, 1, 1), 1)
+                c.set_option(D.OPT_TEST_FAIL_ALLOCS, 0)
+
+
+def test_a_server_jobs_staging_buffer():
+    small, many = random_codes(9, 300_000, 91), random_codes(5, 2_000_000, 92)
+    ref = O.final_dag(O.create_dag(many, 5))
+    srv = D.Server(0, slots=1, hbm_budget_bytes=64 << 30)
+    try:
+        srv.wait(srv.submit(small, 9))
+        srv.set_option(D.OPT_TEST_FAIL_ALLOCS, 2)  # of the next job only its staging buffer has to grow
+        with pytest.raises(D.DagcError) as e:
+            srv.wait(srv.submit(many, 5))
+        assert e.value.status == D.ERR_OUT_OF_MEMORY
+        srv.set_option(D.OPT_TEST_FAIL_ALLOCS, 1)
+        assert np.array_equal(srv.wait(srv.submit(many, 5))[0], ref)
+    finally:
+        srv.close()
