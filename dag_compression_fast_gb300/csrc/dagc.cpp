@@ -852,7 +852,7 @@ struct LevelGroups {
                 --lo;
                 sum += items[lo];
                 slots += node_slots_upto(items[lo]);
-                buckets += node_buckets_upto(items[lo]);
+                buckets += node_buckets(items[lo]);
                 places += group_slot_items(items[lo]);
             }
             groups.push_back({hi, lo});
@@ -884,9 +884,10 @@ struct CreateLayout {
     uint64_t item_cap = 0, uniq_cap = 0, leaf_area = 0, bucket_area = 0, table_slots = 0;
     size_t o_islot = 0, o_ukey = 0, o_uslot = 0;
     size_t o_bcnt = 0, o_bent = 0;
-    // Its node levels: per level the nodes' hashes, child masks and first
-    // children; groups of levels deduplicated together, (last, first) bottom up.
-    std::vector<size_t> o_nh, o_nm, o_nf;
+    // Its node levels: per level the nodes' hashes (where the distinct ones go
+    // once all are in the table: o_ph), child masks and first children; groups
+    // of levels deduplicated together, (last, first) bottom up.
+    std::vector<size_t> o_nm, o_nf;
     std::vector<std::pair<int, int>> groups;
     uint64_t slot_cap = 0, bucket_cap = 0;
     // Nodes of a level that the dedup can hold.
@@ -939,12 +940,9 @@ struct CreateLayout {
         if (direct_table) o_dlist = L.take<uint2>(direct_blocks(depth));
         o_ss0 = L.take<uint32_t>(sorts ? sort_status_words(n) : 0);
         o_ss1 = L.take<uint32_t>(sorts ? sort_status_words(n) : 0);
-        o_A = L.take<uint64_t>(direct ? 0 : n);
-        o_B = L.take<uint64_t>(direct ? 0 : n);
-        if (grouping) {
-            group_shape(n, &group_slab_total, &group_probe_max);
-            o_slab = L.take<uint64_t>(group_slab_total);
-            o_over = L.take<uint64_t>(n);
+        if (!use_dedup) {
+            o_A = L.take<uint64_t>(n);
+            o_B = L.take<uint64_t>(n);
         }
         o_P = L.take<uint64_t>(p0cap);
         o_LM = L.take<uint64_t>(p0cap);
@@ -966,14 +964,7 @@ struct CreateLayout {
         o_M1 = L.take<uint32_t>(p0cap);
         o_NC0 = L.take<uint64_t>(capmax);
         o_NC1 = L.take<uint64_t>(capmax);
-        if (dedup) {
-            o_nh.resize(nl); o_nm.resize(nl); o_nf.resize(nl);
-            for (int l = 0; l < nl; ++l) {
-                o_nh[l] = L.take<uint64_t>(cap[l]);
-                o_nf[l] = L.take<uint32_t>(cap[l]);
-                o_nm[l] = L.take<uint8_t>(cap[l]);
-            }
-        } else {
+        if (!dedup) {
             o_NM = L.take<uint8_t>(capmax);
             o_NCH = L.take<uint32_t>(std::max<uint64_t>(capmax, kTailCap) * 8);
             o_NH = L.take<uint64_t>(capmax);
@@ -1006,6 +997,25 @@ struct CreateLayout {
             o_ck_gd = L.take<uint32_t>((uint64_t)k_batch * ck_groups);
         }
         total = L.off;
+        if (dedup) {
+            // The fragments' buffers are done with once the leaves are built; the
+            // nodes' first children and masks are only made then, in their room.
+            // The first children of all levels follow one another: the word
+            // positions of the final layout (one more than nodes) take theirs.
+            Layout F = L;
+            o_A = F.take<uint64_t>(direct ? 0 : n);
+            o_B = F.take<uint64_t>(direct ? 0 : n);
+            if (grouping) {
+                group_shape(n, &group_slab_total, &group_probe_max);
+                o_slab = F.take<uint64_t>(group_slab_total);
+                o_over = F.take<uint64_t>(n);
+            }
+            o_nf.resize(nl);
+            o_nm.resize(nl);
+            for (int l = 0; l < nl; ++l) o_nf[l] = L.take<uint32_t>(cap[l] + (l + 1 == nl ? 1 : 0));
+            for (int l = 0; l < nl; ++l) o_nm[l] = L.take<uint8_t>(cap[l]);
+            total = std::max(F.off, L.off);
+        }
     }
 };
 
@@ -1379,7 +1389,7 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
             // stages are timed one after the other, and programmatic launches,
             // which follow one stream).
             auto nodes_of = [&](int l) {
-                return NodeArrays{P64(Lo.o_nh[l]), P8(Lo.o_nm[l]), P32(Lo.o_nf[l]), nullptr};
+                return NodeArrays{P64(Lo.o_ph[l]), P8(Lo.o_nm[l]), P32(Lo.o_nf[l]), nullptr};
             };
             auto extract_all = [&](cudaStream_t s) {
                 TailNodesArgs ta{};
@@ -1391,7 +1401,7 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
                     const uint64_t bound = bottom ? p0cap : cap[l + 1];
                     NodesArgs e{};
                     e.child_codes = bottom ? P64(Lo.o_P) : node_codes[(it & 1) ^ 1];
-                    e.child_hashes = bottom ? P64(Lo.o_LM) : P64(Lo.o_nh[l + 1]);
+                    e.child_hashes = bottom ? P64(Lo.o_LM) : P64(Lo.o_ph[l + 1]);
                     e.d_n = bottom ? cs.count(kCntBricks) : cs.count(kCntNodes + l + 1);
                     TailNodesLevel& t = ta.lv[l];
                     t.child_codes = e.child_codes;
@@ -1498,13 +1508,13 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
                 // The words' positions with the call, from the counts on the
                 // device: once the host knows them, it allocates the exact
                 // words and only the write is left. The positions take the
-                // room of the nodes' arrays, which are no longer read.
+                // room of the nodes' first children, which are no longer read.
                 StageTimer t(ctx, DAGC_STAGE_FINAL, s);
                 FinalArgs f{};
                 for (int l = 0; l < nl; ++l) f.lv_masks[l] = P8(Lo.o_pm[l]);
                 f.num_levels = nl;
                 f.d_level_n = cs.count(kCntUnique);
-                f.word_pos = P32(Lo.o_nh[0]);
+                f.word_pos = P32(Lo.o_nf[0]);
                 f.d_total = cs.count(kCntWords);
                 f.status = P64(Lo.o_fsv);
                 f.tile_counter = cs.counter();
@@ -1725,7 +1735,7 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
     out.leaves = P64(Lo.o_PL);
     out.num_leaves = counts[kCntLeaves];
     if (words) {
-        out.word_pos = P32(Lo.o_nh[0]);
+        out.word_pos = P32(Lo.o_nf[0]);
         out.node_words = counts[kCntWords];
     }
     return DAGC_OK;

@@ -40,13 +40,10 @@ __device__ __forceinline__ uint64_t home_slot(uint64_t k, uint64_t S) { return _
 __device__ __forceinline__ uint64_t next_slot(uint64_t s, uint64_t S) { return s + 1 == S ? 0 : s + 1; }
 __device__ __forceinline__ uint32_t next_slot(uint32_t s, uint32_t S) { return s + 1 == S ? 0u : s + 1; }
 
-// Buckets of the top-bit form: a power of two with ~kDedupPerBucket keys each
-// for u keys; a key's bucket is key >> *shift.
+// The buckets of a node level of u items (node_buckets): a key's bucket is key >> *shift.
 __device__ __forceinline__ uint32_t topbit_buckets(uint64_t u, int* shift) {
-    uint32_t nb = 1;
-    int lg = 0;
-    while ((uint64_t)nb * kDedupPerBucket < u && nb < kDedupMaxBuckets) { nb <<= 1; ++lg; }
-    *shift = 64 - lg;
+    const uint32_t nb = node_buckets(u);
+    *shift = 64 - (31 - __clz(nb));
     return nb;
 }
 

@@ -295,10 +295,11 @@ DAGC_HD uint64_t dedup_bucket_area(uint64_t uniq_cap) {
     const uint64_t most = (uint64_t)kDedupMaxBuckets * kDedupTopBitCap;
     return a < most ? a : most;
 }
-// The same for one node level of up to n items: its buckets' room.
-DAGC_HD uint64_t node_buckets_upto(uint64_t n) {
-    const uint64_t b = n / (kDedupPerBucket / 2) + 1;
-    return b < kDedupMaxBuckets ? b : kDedupMaxBuckets;
+// Buckets of a node level of n items (they only grow with n): a power of two.
+DAGC_HD uint32_t node_buckets(uint64_t n) {
+    uint32_t b = 1;
+    while ((uint64_t)b * kDedupPerBucket < n && b < kDedupMaxBuckets) b <<= 1;
+    return b;
 }
 // Table slots for n items. Leaf masks repeat (about one distinct mask per ten
 // bricks): 1.25 n slots, at most 0.8 full even when every mask is distinct,
