@@ -1144,10 +1144,10 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
     const bool chunk_path = batch && ctx->batch_path == 1 && chunk_bin_bits(batch->chunk_depth) <= kChunkMaxBinBits;
     const bool direct_table = allow_direct && !batch && use_dedup && group_mode == 1 && direct_table_applies(n, depth);
     const bool direct = direct_table && direct_mark_applies(n, depth);
+    const bool grouping = group_mode != 0 && use_dedup && !chunk_path && !direct;
     const bool words = want_words && use_dedup && nl > 0;
-    const CreateLayout Lo(n, depth, batch ? batch->k : 0u, use_dedup, ctx->dedup_unique_limit,
-                          group_mode != 0 && use_dedup && !chunk_path && !direct, chunk_path ? batch->chunk_depth : 0,
-                          direct_table, direct);
+    const CreateLayout Lo(n, depth, batch ? batch->k : 0u, use_dedup, ctx->dedup_unique_limit, grouping,
+                          chunk_path ? batch->chunk_depth : 0, direct_table, direct);
     const std::vector<uint64_t>& cap = Lo.cap;
     const uint64_t capmax = Lo.capmax, p0cap = Lo.p0cap, sv_total = Lo.sv_total;
     const size_t zero_bytes = Lo.zero_bytes;
@@ -1155,7 +1155,8 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
     DAGC_CUDA(ctx, ctx->arena.reserve(Lo.total));
     arena_wait(ctx, s);
     if (use_dedup) {
-        const int st = reserve_table(ctx, Lo.table_slots, s, group_mode != 0);
+        // (The grouping's brick masks go to the brick table where there is one.)
+        const int st = reserve_table(ctx, Lo.table_slots, s, grouping && !direct_table);
         if (st) return st;
     }
     if (direct_table && !reserve_direct(ctx, direct_entries(depth), s))
@@ -1276,7 +1277,7 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
             DAGC_LAUNCHED(ctx);
             t.stop();
         }
-        if (!chunk_path && !direct && group_mode != 0 && use_dedup && ctx->gtable) {
+        if (grouping) {
             GroupArgs g{};
             g.frags = d_frag;
             g.n = n;
@@ -1699,7 +1700,7 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
         }
         set_pending_bytes(ctx, DAGC_STAGE_LEVELS, lb);
         // The kernels of the path the device did not take returned at once.
-        if (!direct && group_mode != 0 && use_dedup && ctx->gtable) {
+        if (grouping) {
             uint32_t path = 0;
             DAGC_CUDA(ctx, cudaMemcpy(&path, &hdr->path[0], 4, cudaMemcpyDeviceToHost));
             if (path == 1) {

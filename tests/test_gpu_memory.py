@@ -111,3 +111,17 @@ def test_a_server_jobs_staging_buffer():
         assert np.array_equal(srv.wait(srv.submit(many, 5))[0], ref)
     finally:
         srv.close()
+
+
+def test_grouping_scratch_only_for_calls_that_group():
+    """Marked straight into the brick table, or chunk by chunk: no grouping scratch; deeper volumes take it."""
+    with D.Context(0) as c:
+        codes = random_codes(9, 20_000, 101)
+        assert np.array_equal(c.compress(codes, 9).to_numpy(), O.final_dag(O.create_dag(codes, 9)))
+        chunks, sub = chunks_of(codes, 9, 1)
+        batched = c.create_dag_batched(np.concatenate(chunks), [x.size for x in chunks], list(range(8)), sub, 1)
+        assert_dag_equal(batched.to_host(), O.create_dag(codes, 9))
+        assert "grouping table" not in c.memory_report()
+        deep = random_codes(12, 20_000, 102, cluster=True)
+        assert np.array_equal(c.compress(deep, 12).to_numpy(), O.final_dag(O.create_dag(deep, 12)))
+        assert "grouping table" in c.memory_report()
