@@ -45,6 +45,7 @@ enum : int {
     kCntNodes = 3,                 // + level
     kCntUnique = 3 + kMaxDepth,    // + level
     kCntSlots = 3 + 2 * kMaxDepth + 1,
+    kCntGrouped = 60,              // 1: the fragments were grouped by hash
     kCntWords = 61,                // words of all nodes (final layout)
     kCntDirectBlocks = 62,         // occupied blocks of the direct-mapped brick table
     kCntOverflow = 63,             // fragments the grouping spilled past their partition's slab
@@ -62,7 +63,7 @@ struct CallHeader {
     uint32_t path[4];                   // [0] 1: fragments grouped by hash, 0: sorted; [1], [2] its shape
     LeafOrder leaf;                     // ordering of the distinct leaf masks
 };
-static_assert(kCntSlots <= kCntWords, "count slots");
+static_assert(kCntSlots <= kCntGrouped, "count slots");
 constexpr uint32_t kPublishWords = 1 + 64;  // error word and counts
 constexpr uint32_t kStagedRoots = 256;      // roots of a merge, after them
 constexpr size_t kStageBytes = 4096;        // a context's pinned words
@@ -376,6 +377,7 @@ struct dagc_context_t {
     void* direct = nullptr;
     uint64_t direct_cap = 0;
     bool direct_dirty = true;
+    bool deep_table = false;  // a call at kDirectMaxDepth was grouped: the next ones take the table there
     uint64_t fallbacks = 0;  // calls rerun with the radix form
     void* vox_scratch = nullptr;    // voxelizer counters and look-back status
     size_t vox_scratch_bytes = 0;
@@ -1086,11 +1088,16 @@ int reserve_table(dagc_context ctx, uint64_t slots, cudaStream_t s, bool groupin
     return DAGC_OK;
 }
 
-// Whether an unbatched call uses the direct-mapped brick table (direct.cu). It
+// Whether an unbatched call can use the direct-mapped brick table (direct.cu). It
 // has 8 bytes per brick of the volume whatever the fragments, so the line is
 // its size: up to depth 10 (134 MB, about the L2) always, at depth 11 (1 GB)
 // from 2^21 fragments on, where the call's own scratch (about 400 bytes per
-// fragment) is of that order.
+// fragment) is of that order. At depth 11 it only orders grouped bricks, and
+// whether fragments are grouped or sorted is decided on the device: a context
+// takes that table once one of its calls was grouped (the call that finds out
+// sorts its bricks: 2048^3 terrain, 31M fragments, 738 us against 543 with the
+// table), never for inputs that are sorted (4.2M scattered fragments: a context's
+// first call 1682 us when it took the table, now 1414).
 bool direct_table_applies(uint64_t n, int depth) {
     return depth < kDirectMaxDepth || (depth == kDirectMaxDepth && n >= (1u << 21));
 }
@@ -1142,7 +1149,8 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
     // Batched calls take the persistent per-chunk leaf build (chunks.cu) when
     // the chunk's bins fit its limits; otherwise the composite-key path.
     const bool chunk_path = batch && ctx->batch_path == 1 && chunk_bin_bits(batch->chunk_depth) <= kChunkMaxBinBits;
-    const bool direct_table = allow_direct && !batch && use_dedup && group_mode == 1 && direct_table_applies(n, depth);
+    const bool table_fits = !batch && use_dedup && group_mode == 1 && direct_table_applies(n, depth);
+    const bool direct_table = allow_direct && table_fits && (depth < kDirectMaxDepth || ctx->deep_table);
     const bool direct = direct_table && direct_mark_applies(n, depth);
     const bool grouping = group_mode != 0 && use_dedup && !chunk_path && !direct;
     const bool words = want_words && use_dedup && nl > 0;
@@ -1303,6 +1311,7 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
             g.masks = static_cast<uint64_t*>(ctx->gtable);
             g.cap = std::min<uint64_t>(p0cap, kGroupMaxBricks);
             g.d_count = cs.count(kCntBricks);
+            g.d_grouped = cs.count(kCntGrouped);
             g.sorted_bricks = P64(Lo.o_P);
             g.sorted_idx = P32(Lo.o_M1);
             g.parents = P64(Lo.o_P);
@@ -1715,6 +1724,7 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
         }
         settle_profile(ctx);
     }
+    if (table_fits && counts[kCntGrouped]) ctx->deep_table = true;
     if (e32) ctx->table_dirty = ctx->direct_dirty = true;  // a kernel may have stopped before clearing its slots
     if ((e32 & kErrFallback) && !(e32 & (kErrBadInput | kErrTimeout))) return kStatusFallback;
     std::string msg;

@@ -176,6 +176,7 @@ struct GroupArgs {
     float probe_max_distinct;  // grouping when the probe's sample shows at most this many distinct bricks
     uint64_t* cursor;          // kGroupMaxParts: partition p's next free position in its slab
     uint32_t* path;            // [0] 1 grouping, 0 sort path; [1] log2 partitions; [2] log2 table slots; [3] slab size
+    uint64_t* d_grouped;       // path[0] among the call's counts
     uint64_t* parts;           // partition slabs (group_shape's slab_total fragment keys)
     uint64_t* overflow; uint64_t overflow_cap;  // fragments past their slab's end, any partition
     uint64_t* overflow_count;  // zero on entry

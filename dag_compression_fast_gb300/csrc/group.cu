@@ -257,6 +257,7 @@ __global__ void __launch_bounds__(kPlanThreads) group_plan(GroupArgs a) {
         shape[0] = (uint32_t)lp;
         shape[1] = (uint32_t)(mean + mean / 4 + 1024);
         a.path[0] = group ? 1u : 0u;
+        *a.d_grouped = group ? 1u : 0u;
         a.path[1] = (uint32_t)lp;
         a.path[2] = (uint32_t)kGroupPartSlotsLog;
         a.path[3] = shape[1];

@@ -125,3 +125,26 @@ def test_grouping_scratch_only_for_calls_that_group():
         deep = random_codes(12, 20_000, 102, cluster=True)
         assert np.array_equal(c.compress(deep, 12).to_numpy(), O.final_dag(O.create_dag(deep, 12)))
         assert "grouping table" in c.memory_report()
+
+
+def test_the_depth_11_table_only_once_fragments_are_grouped():
+    """1 GB, and of use only to grouped fragments: not for sorted ones, and from the second grouped call on (launched,
+    recorded, replayed)."""
+    sparse = random_codes(11, 2**21, 111)
+    rng = np.random.default_rng(112)
+    bricks = rng.integers(0, 8**9, 30_000, dtype=np.uint64)
+    crowded = (bricks[rng.integers(0, bricks.size, 2**21 + 77)] << np.uint64(6)) | rng.integers(0, 64, 2**21 + 77, dtype=np.uint64)
+    refs = [O.final_dag(O.create_dag(x, 11, threads=8)) for x in (sparse, crowded)]
+    with D.Context(0) as c:
+        import torch
+        sparse, crowded = (torch.from_numpy(x.view(np.int64)).cuda() for x in (sparse, crowded))
+        for _ in range(3):
+            assert np.array_equal(c.compress(sparse, 11).to_numpy(), refs[0])
+        assert np.array_equal(c.compress(crowded, 11).to_numpy(), refs[1])
+        assert not has_brick_table(c)
+        for _ in range(4):
+            assert np.array_equal(c.compress(crowded, 11).to_numpy(), refs[1])
+            assert has_brick_table(c)
+        assert np.array_equal(c.compress(sparse, 11).to_numpy(), refs[0])
+        c.free_all()
+        assert np.array_equal(c.compress(crowded, 11).to_numpy(), refs[1])
