@@ -40,6 +40,7 @@ OPT_TEST_STALL_LOOKBACK = 10
 OPT_TEST_FAIL_ALLOCS = 11
 OPT_BATCH_PATH = 12
 OPT_TEST_FAIL_BESIDE = 13
+OPT_BRICK_TABLE = 14
 VOXELIZE_GL = 0
 VOXELIZE_SAT = 1
 NUM_KEY_SHAPES = 9

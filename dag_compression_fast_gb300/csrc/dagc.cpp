@@ -377,6 +377,7 @@ struct dagc_context_t {
     void* direct = nullptr;
     uint64_t direct_cap = 0;
     bool direct_dirty = true;
+    bool use_direct = true;   // DAGC_OPT_BRICK_TABLE
     bool deep_table = false;  // a call at kDirectMaxDepth was grouped: the next ones take the table there
     uint64_t fallbacks = 0;  // calls rerun with the radix form
     void* vox_scratch = nullptr;    // voxelizer counters and look-back status
@@ -1149,7 +1150,7 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
     // Batched calls take the persistent per-chunk leaf build (chunks.cu) when
     // the chunk's bins fit its limits; otherwise the composite-key path.
     const bool chunk_path = batch && ctx->batch_path == 1 && chunk_bin_bits(batch->chunk_depth) <= kChunkMaxBinBits;
-    const bool table_fits = !batch && use_dedup && group_mode == 1 && direct_table_applies(n, depth);
+    const bool table_fits = ctx->use_direct && !batch && use_dedup && group_mode == 1 && direct_table_applies(n, depth);
     const bool direct_table = allow_direct && table_fits && (depth < kDirectMaxDepth || ctx->deep_table);
     const bool direct = direct_table && direct_mark_applies(n, depth);
     const bool grouping = group_mode != 0 && use_dedup && !chunk_path && !direct;
@@ -2593,6 +2594,17 @@ cudaError_t dagc::context_malloc(dagc_context ctx, void** p, size_t bytes) {
     return ctx_malloc(ctx, p, bytes);
 }
 
+// The table's entries, and its block counters and lists in the call's scratch.
+uint64_t dagc::brick_table_bytes(uint64_t n, int depth) {
+    if (!n || !direct_table_applies(n, depth)) return 0;
+    return direct_entries(depth) * 8 + direct_blocks(depth) * 12;
+}
+
+uint64_t dagc::brick_table_held(dagc_context ctx) {
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    return ctx->direct_cap * 8 + (ctx->direct_cap >> kDirectBlockLog) * 12;
+}
+
 // ===================================================================== C ABI
 extern "C" {
 
@@ -2799,8 +2811,8 @@ int dagc_create_batched(dagc_context ctx, const uint64_t* d_fragments, const uin
 
 uint64_t dagc_create_footprint(uint64_t n, int depth) {
     if (depth < 2 || depth > kMaxDepth || n == 0) return 0;
-    const CreateLayout L(n, depth, 0, true, kDedupMaxUnique, true, 0, direct_table_applies(n, depth));
-    return L.total + L.table_slots * 16 + kGroupScratchBytes + (direct_table_applies(n, depth) ? direct_entries(depth) * 8 : 0);
+    const CreateLayout L(n, depth, 0, true, kDedupMaxUnique, true);
+    return L.total + L.table_slots * 16 + kGroupScratchBytes;
 }
 
 int dagc_dag_num_levels(dagc_dag d, int* num_levels) {
@@ -3151,6 +3163,14 @@ int dagc_set_option(dagc_context ctx, int option, int value) {
         case DAGC_OPT_GROUP:
             if (value < 0 || value > 2) return set_error(ctx, DAGC_ERR_INVALID_ARGUMENT, "group mode must be 0, 1 or 2");
             ctx->group_mode = value;
+            return DAGC_OK;
+        case DAGC_OPT_BRICK_TABLE:
+            if (value < 0 || value > 1) return set_error(ctx, DAGC_ERR_INVALID_ARGUMENT, "brick table must be 0 or 1");
+            ctx->use_direct = value != 0;
+            if (!ctx->use_direct && ctx->direct) {
+                DAGC_CUDA(ctx, cudaSetDevice(ctx->device));
+                release_direct(ctx);
+            }
             return DAGC_OK;
         case DAGC_OPT_BATCH_PATH:
             if (value < 0 || value > 1) return set_error(ctx, DAGC_ERR_INVALID_ARGUMENT, "batch path must be 0 or 1");

@@ -62,6 +62,11 @@ struct Request {
 struct dagc_server_t {
     int device = 0;
     uint64_t budget = 0, in_use = 0, peak_in_use = 0;
+    // Bytes of the brick table of each slot's context, which it keeps between
+    // jobs, and whether the slot is running one.
+    std::vector<uint64_t> tables;
+    std::vector<char> busy;
+    bool use_tables = true;  // DAGC_OPT_BRICK_TABLE
     std::mutex mu;
     std::condition_variable cv_work, cv_done;
     std::deque<std::shared_ptr<Request>> queue;
@@ -94,6 +99,43 @@ struct dagc_server_t {
 
 namespace {
 
+// Bytes of the brick tables of the running slots; of all slots but one. With sv->mu held.
+uint64_t busy_tables(const dagc_server_t* sv) {
+    uint64_t sum = 0;
+    for (size_t j = 0; j < sv->tables.size(); ++j) sum += sv->busy[j] ? sv->tables[j] : 0;
+    return sum;
+}
+uint64_t other_tables(const dagc_server_t* sv, int except) {
+    uint64_t sum = 0;
+    for (size_t j = 0; j < sv->tables.size(); ++j) sum += (int)j != except ? sv->tables[j] : 0;
+    return sum;
+}
+
+// Admits `r` to a free slot. Its footprint counts as its need; a brick table
+// only saves time, so it is the tables that give way: those of idle slots go
+// where the job needs their room, and the job takes (or keeps) one only while
+// all of them together are at most an eighth of the budget and fit in it.
+// Returns whether the job may. With sv->mu held.
+bool admit(dagc_server_t* sv, int slot, const Request& r) {
+    if (sv->in_use + r.footprint + other_tables(sv, slot) > sv->budget) {
+        for (size_t j = 0; j < sv->tables.size(); ++j) {
+            if ((int)j == slot || sv->busy[j] || !sv->tables[j]) continue;
+            dagc_set_option(sv->contexts[j], DAGC_OPT_BRICK_TABLE, 0);
+            sv->tables[j] = 0;
+        }
+    }
+    const uint64_t want = std::max(dagc::brick_table_bytes(r.n, r.depth), sv->tables[slot]);
+    const uint64_t all = other_tables(sv, slot) + want;
+    const bool table = sv->use_tables && all <= sv->budget / 8 && sv->in_use + r.footprint + all <= sv->budget;
+    sv->tables[slot] = table ? want : 0;
+    sv->busy[slot] = 1;
+    sv->in_use += r.footprint;
+    sv->peak_in_use = std::max(sv->peak_in_use, sv->in_use + other_tables(sv, -1));
+    ++sv->running;
+    sv->max_running = std::max(sv->max_running, sv->running);
+    return table;
+}
+
 void worker_loop(dagc_server_t* sv, int slot) {
     cudaSetDevice(sv->device);
     dagc_context ctx = sv->contexts[slot];
@@ -108,6 +150,7 @@ void worker_loop(dagc_server_t* sv, int slot) {
     cudaEventCreate(&ev1);
     for (;;) {
         std::shared_ptr<Request> r;
+        bool table = false;
         {
             std::unique_lock<std::mutex> lock(sv->mu);
             // FIFO admission: the head of the queue starts when a slot (this
@@ -115,24 +158,21 @@ void worker_loop(dagc_server_t* sv, int slot) {
             sv->cv_work.wait(lock, [&] {
                 return sv->stop ||
                        (!sv->queue.empty() &&
-                        (sv->in_use + sv->queue.front()->footprint <= sv->budget || sv->in_use == 0));
+                        (sv->in_use + busy_tables(sv) + sv->queue.front()->footprint <= sv->budget || sv->in_use == 0));
             });
             if (sv->stop && sv->queue.empty()) break;
             r = sv->queue.front();
             sv->queue.pop_front();
-            sv->in_use += r->footprint;
-            sv->peak_in_use = std::max(sv->peak_in_use, sv->in_use);
-            ++sv->running;
-            sv->max_running = std::max(sv->max_running, sv->running);
+            table = admit(sv, slot, *r);
             r->started = Clock::now();
         }
-        int st = DAGC_OK;
+        int st = dagc_set_option(ctx, DAGC_OPT_BRICK_TABLE, table);
         std::string err;
         std::vector<uint32_t> words;
         dagc_dag keep = nullptr;
         {
             // Host fragments in, host words out, on this slot's stream.
-            if (r->n > stage_cap) {
+            if (!st && r->n > stage_cap) {
                 if (stage) cudaFree(stage);
                 stage = nullptr;
                 stage_cap = 0;
@@ -185,6 +225,7 @@ void worker_loop(dagc_server_t* sv, int slot) {
                 cudaGetLastError();
             }
         }
+        const uint64_t held = dagc::brick_table_held(ctx);
         {
             std::lock_guard<std::mutex> lock(sv->mu);
             r->status = st;
@@ -193,6 +234,8 @@ void worker_loop(dagc_server_t* sv, int slot) {
             r->finished = Clock::now();
             r->done = true;
             sv->in_use -= r->footprint;
+            sv->tables[slot] = held;
+            sv->busy[slot] = 0;
             --sv->running;
             ++sv->completed;
             sv->fragments_done += r->n;
@@ -295,6 +338,8 @@ int dagc_server_create(int device, int slots, uint64_t hbm_budget_bytes, dagc_se
         if (i < slots) sv->contexts.push_back(c);
         else sv->merge_ctx = c;
     }
+    sv->tables.assign(slots, 0);
+    sv->busy.assign(slots, 0);
     cudaSetDevice(device);
     if (cudaEventCreate(&sv->origin) == cudaSuccess) {
         cudaEventRecord(sv->origin, nullptr);
@@ -407,6 +452,10 @@ int dagc_server_set_option(dagc_server sv, int option, int value) {
     for (dagc_context c : sv->contexts) {
         const int st = dagc_set_option(c, option, value);
         if (st) return st;
+    }
+    if (option == DAGC_OPT_BRICK_TABLE) {  // set again for each job (admit)
+        std::lock_guard<std::mutex> lock(sv->mu);
+        sv->use_tables = value != 0;
     }
     return DAGC_OK;
 }

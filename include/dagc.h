@@ -102,7 +102,9 @@ int dagc_dag_upload(dagc_context ctx, int num_levels, const uint64_t* level_size
 int dagc_dag_copy(dagc_context ctx, dagc_dag src, void* stream, dagc_dag* out);
 void dagc_dag_free(dagc_dag dag);
 /* Bytes of device scratch one dagc_create call of n fragments at this depth
- * lays out (its arena; the DAG itself comes on top). 0 for n == 0. */
+ * needs (its arena and tables; the DAG itself comes on top, and the brick table
+ * that a context keeps where there is room, see DAGC_OPT_BRICK_TABLE). 0 for
+ * n == 0. */
 uint64_t dagc_create_footprint(uint64_t n, int depth);
 
 /* ------------------------------------------------------------ MergeDAGs ---- */
@@ -206,7 +208,7 @@ int dagc_last_counts(dagc_context ctx, uint64_t* out, int cap);
 #define DAGC_OPT_DEDUP_UNIQUE_LIMIT 5
 /* How fragments are grouped into bricks (SortKeys + SelectUnique +
  * ReduceByKey): 1 (default) up to depth 10 through a direct-mapped table of
- * the volume's bricks (8 bytes each, kept by the context; not for calls of
+ * the volume's bricks (DAGC_OPT_BRICK_TABLE; not for calls of
  * more than 2^25 fragments with more than 4 per brick of the volume); beyond,
  * choose on the device per call, from a sketch of
  * the distinct bricks in a sample of the fragments: hash partitions and
@@ -227,6 +229,14 @@ int dagc_last_counts(dagc_context ctx, uint64_t* out, int cap);
  * shared memory); 0 the composite-key path (chunk rank above the local code,
  * one sort or grouping over all chunks). Results are identical. */
 #define DAGC_OPT_BATCH_PATH 12
+/* 1 (default): calls with DAGC_OPT_GROUP 1 may take a direct-mapped table of the
+ * volume's bricks, 8 bytes each (up to 134 MB to depth 10; 1 GB at depth 11, only
+ * from 2^21 fragments on and once the context has had such a call grouped). The
+ * context keeps it until dagc_free_all, until an allocation of any context on the
+ * device would fail otherwise, or until this option is set to 0: it is then given
+ * back at once and calls do without. A call whose table does not fit does without
+ * too. Results are identical. */
+#define DAGC_OPT_BRICK_TABLE 14
 /* Failure-path test hooks (off by default; no counterpart in the reference).
  * TEST_SPIN_LIMIT: polls before a bounded device wait of the sorts gives up
  * (0: the production limit, about a second). TEST_STALL_LOOKBACK: 1 makes the
@@ -384,7 +394,9 @@ int dagc_voxelize(dagc_context ctx, const double* d_vertices, uint64_t n_triangl
 /* -------------------------------------------------------------- serving ---- */
 /* A request loop: compression jobs are admitted in arrival order as soon as
  * one of `slots` worker slots is free and their device-memory footprint fits
- * in hbm_budget_bytes (a job larger than the budget runs alone); admitted jobs
+ * in hbm_budget_bytes (a job larger than the budget runs alone). The brick tables
+ * of the slots count against the budget too and take at most an eighth of it: a
+ * job whose table would be more runs without (DAGC_OPT_BRICK_TABLE). Admitted jobs
  * run concurrently, each slot with its own context and stream, so their work
  * overlaps on the GPU. Each job: host fragments in, final words out. The
  * reference has no counterpart (it compresses one subvolume after another). */

@@ -148,3 +148,39 @@ def test_the_depth_11_table_only_once_fragments_are_grouped():
         assert np.array_equal(c.compress(sparse, 11).to_numpy(), refs[0])
         c.free_all()
         assert np.array_equal(c.compress(crowded, 11).to_numpy(), refs[1])
+
+
+def test_brick_table_option_gives_it_back():
+    codes = random_codes(10, 40_000, 121)
+    ref = O.final_dag(O.create_dag(codes, 10))
+    with D.Context(0) as c:
+        for on in (1, 0, 1):
+            c.set_option(D.OPT_BRICK_TABLE, on)
+            assert not has_brick_table(c) or on
+            for _ in range(3):
+                assert np.array_equal(c.compress(codes, 10).to_numpy(), ref)
+            assert has_brick_table(c) == bool(on)
+
+
+@pytest.mark.parametrize("room", ["tight", "roomy"])
+def test_server_budget_holds_the_brick_tables(room):
+    """Tight: as many jobs side by side as their scratch allows, without tables, inside the budget. Roomy: tables, and
+    they count."""
+    jobs = [random_codes(10, 2_000 + i, 130 + i) for i in range(12)]
+    table = 8 * 8**8
+    need = max(D.create_footprint(x.size, 10) + 24 * x.size for x in jobs)
+    assert need < table
+    budget = 4 * need if room == "tight" else 16 << 30
+    srv = D.Server(0, slots=4, hbm_budget_bytes=budget)
+    try:
+        for _ in range(2):
+            tickets = [srv.submit(x, 10) for x in jobs]
+            for x, t in zip(jobs, tickets):
+                assert np.array_equal(srv.wait(t)[0], O.final_dag(O.create_dag(x, 10)))
+        s = srv.stats()
+        assert s["max_concurrent"] >= 2
+        assert s["peak_footprint"] <= budget
+        if room == "roomy":
+            assert s["peak_footprint"] > table
+    finally:
+        srv.close()
