@@ -214,6 +214,7 @@ DAGC_HD uint64_t direct_plan_tiles(int depth) { return direct_blocks(depth) / kD
 struct DirectArgs {
     const uint64_t* frags; uint64_t n;
     int code_bits;          // 3 * depth: codes are below 2^code_bits
+    uint32_t mark_rows;     // rows of 32 fragments that a warp marks at a time (launch_direct_mark)
     uint64_t* table;        // a leaf mask per brick (direct_entries), zero on entry and exit
     uint32_t blocks;
     uint32_t* block_count;  // bricks per block, zero on entry
