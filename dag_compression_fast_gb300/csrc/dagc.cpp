@@ -492,6 +492,16 @@ struct StageTimer {
     }
 };
 
+// Whether the caller is recording `s` (the call is then refused at its first
+// wait): what follows a recorded event would be drawn into that recording, and
+// the side stream be lost to the context's other streams until it ends.
+bool caller_records(cudaStream_t s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 // Work on the context's side stream beside a call's stream, from fork to join. A
 // call that returns in between joins it all the same: the next call writes the
 // same arena, and a recording must not end with a branch left open.
@@ -1439,7 +1449,8 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
                     ++ctx->launches;
                 }
             };
-            const bool beside = ctx->side_stream && !ctx->profiling && !ctx->pdl && nl > 0;
+            const bool beside = ctx->side_stream && !ctx->profiling && !ctx->pdl && nl > 0 &&
+                                (s == ctx->capture_stream || !caller_records(s));
             SideWork side(ctx, s);
             if (beside) {
                 DAGC_CUDA(ctx, side.fork());
@@ -1674,9 +1685,9 @@ int create_pipeline(dagc_context ctx, const uint64_t* d_frag, uint64_t n, int de
         return st;
     }
     CallHeader* hdr = reinterpret_cast<CallHeader*>(b + Lo.o_hdr);
-    const cudaError_t es = cudaStreamSynchronize(s);
-    if (es != cudaSuccess) ctx->table_dirty = ctx->direct_dirty = true;
-    DAGC_CUDA(ctx, es);
+    const cudaError_t synchronized = cudaStreamSynchronize(s);
+    if (synchronized != cudaSuccess) ctx->table_dirty = ctx->direct_dirty = true;
+    DAGC_CUDA(ctx, synchronized);
     const uint32_t e32 = (uint32_t)(ctx->h_stage[0] & 0xFFFFFFFFu);
     const uint64_t* counts = ctx->h_stage + 1;
     ctx->last_counts.assign(3 + nl, 0);
