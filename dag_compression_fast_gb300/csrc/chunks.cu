@@ -30,10 +30,11 @@
 //
 // What bounds it: the chain of barriers and round trips of each tile and bin, at
 // 24 bytes of traffic per fragment (read for COUNT, read and 4 bytes written by
-// SCATTER, 4 read by LEAVES). 318M fragments, 256 chunks of 1024^3: 2.86 ms;
-// 6.39 when every fragment left its SCATTER tile as a scattered 8-byte store
-// and every voxel was ORed with an atomic, set or not; 3.47 without the loads
-// ahead and with a block scan per bin.
+// SCATTER, 4 read by LEAVES). 256 chunks of 1024^3, 338M fragments, with the
+// scan and the pack: 2.96 ms; 6.70 when every fragment left its SCATTER tile as
+// a scattered 8-byte store and every voxel was ORed with an atomic, set or not.
+// 318M, the persistent launch alone: 2.86 ms; 3.47 without the loads ahead and
+// with a block scan per bin.
 
 #include "dagc_device.cuh"
 #include "dagc_kernels.h"
@@ -49,7 +50,7 @@ constexpr int kPerThread = kChunkTile / kT;
 static_assert(kChunkTile % kT == 0 && kDirect % kT == 0 && kMaxBins % kT == 0, "chunk shapes");
 
 constexpr int kBitmapWords = kDirect / 32;
-static_assert(kBitmapWords <= kT, "one bitmap word per thread");
+static_assert(2 * kBitmapWords <= kT, "a thread per word of both bitmaps");
 
 struct ChunkSmem {
     union {

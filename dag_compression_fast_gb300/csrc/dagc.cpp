@@ -1118,9 +1118,12 @@ bool direct_table_applies(uint64_t n, int depth) {
 // (leaf stages, us, before / with the table: triangle soup of 0.65M fragments,
 // depth 10, 115 / 32; 61M, 1500 / 1140; terrain of 7.9M, depth 10, 200 / 93;
 // sphere shell in 32^3, 52 / 16) but at 20-50 G/s over the 1 GB of depth 11
-// (terrain, 31M: 400 grouped, 617 straight in). Crowded bricks go through the
-// grouping's shared-memory tables faster: depth 9, 61M fragments, 29 per
-// brick, 700 grouped, 792 straight in.
+// (terrain, 31M: 400 grouped, 617 straight in). Crowded volumes up to 2^25
+// fragments, the whole call, us, grouped / straight in: 33.5M over 32^3 2660 /
+// 243, 64^3 434 / 186, 256^3 684 / 448, 1000 voxels of 512^3 5990 / 188; in a
+// slab of 512^3 589 / 388, sorted 869 / 288. Beyond, the line was drawn when
+// each fragment made its own access (depth 9, 61M, 29 per brick: 700 grouped,
+// 792 straight in).
 bool direct_mark_applies(uint64_t n, int depth) {
     return depth < kDirectMaxDepth && (n <= (1u << 25) || n <= 4 * direct_entries(depth));
 }

@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(256, 4) dedup_insert(DedupArgs a) {
             const uint64_t i = base + k * 32 + lane;
             if (i < n) {
                 const bool placed = live[k] && (won[k] || found[k]);
-                if (live[k] && !placed) full = true;  // cannot happen below half load; rerun rather than guess
+                if (live[k] && !placed) full = true;  // cannot happen: tables are at most 0.8 full; rerun rather than guess
                 a.item_slot[i] = placed ? s[k] : 0xFFFFFFFFu;
             }
         }
